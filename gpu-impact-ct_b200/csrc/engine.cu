@@ -2516,213 +2516,319 @@ __global__ void __launch_bounds__(MNT, 1) k_lv_multi(const LevelJob<T>* __restri
 // Chebyshev polynomial of degree cheb on the interval, bounded by 1 on [0, 2], so the smooth
 // modes that damped Jacobi removes in O(n^2) sweeps fall in O(n) steps, and the preconditioner
 // stays a fixed linear operator.  Such a tail may be the coarsest level alone.
+//
+// What bounds it: one SM, so the instructions and latencies of about 50 passes over at most 17 k
+// cells.  A thread owns one column segment (i, j, k0 .. k0+nk-1) of a level for all the passes of
+// a smoothing phase: its coefficients, omega / diag and neighbour offsets stay in registers,
+// z neighbours slide through them.  The level descriptions come ready from the host and the
+// tables of all levels are staged in shared memory with one copy, so that no pass waits for
+// global memory, and only the warps that own cells of a level meet at its barriers.  Against one
+// block whose threads take single cells strided by the block (coefficients from global memory,
+// omega / diag and index divisions per cell), V-cycle times in us: 32x32x64 FP32 106 -> 64 (its
+// tail 79 -> 36), FP64 89 -> 78, 128x128x256 FP32 233 -> 192, 104x104x208 with 32 Chebyshev steps
+// FP32 224 -> 189, FP64 295 -> 255.  Slower here: 256 and 1024 threads, z-fastest storage with
+// 16-byte accesses (more instructions per pass on the small levels), one run-time choice of the
+// pass in place of the four instances, loads of two or four planes ahead.
 constexpr int TNT = 512;
-constexpr size_t TAIL_BYTES = 200 * 1024;
+constexpr size_t TAIL_BYTES = 200 * 1024;     // the levels' fields
+constexpr size_t TAIL_TAB_BYTES = 22 * 1024;  // their tables (longer ones are read from global memory)
+
+// one level inside the tail: extents, thread mapping, shared-memory offsets (elements)
+struct TailLevel {
+  int n1, n2, n3, zuni;
+  int ncol, len, ncs;    // columns, planes per segment, column segments
+  int nthr;              // threads of the warps that own segments
+  int rf[3], rc[3];      // coarsening factors from the next finer level and to the next coarser one
+  int oA, oX[2];         // fields (compact, i fastest)
+  int tcd[3], tcI[3];    // cdg and interpolation tables, offsets from TailJob::tab
+};
 template <typename T>
 struct TailJob {
-  int nl;                          // levels in the tail (>= 2; >= 1 with cheb)
-  int cheb;                        // Chebyshev steps on the coarsest level (0: Jacobi sweeps)
-  T cgam, csig2;                   // their g and s^2
-  LevelJob<T> lv[MG_MAX_LEVELS];   // their level jobs; lv[0].A / lv[0].B are the global fields
+  int nl;            // levels in the tail (>= 2; >= 1 with cheb)
+  int cheb;          // Chebyshev steps on the coarsest level (0: Jacobi sweeps)
+  int ntab;          // elements of the tables staged in shared memory; 0: read from tab
+  T cgam, csig2;     // g and s^2 of the Chebyshev steps
+  const T* tab;      // the levels' tables, one run of global memory
+  Geom g;            // the first level's grid and its global right-hand side and iterate
+  const T* A;
+  T* B;
+  const SolverScalars* sc;
+  TailLevel lv[MG_MAX_LEVELS];
 };
 
-// the cells idx = tid, tid + TNT, ... of an n1 x n2 x n3 level with their 1-based (i, j, k),
-// advanced by carries instead of one division per cell
-template <typename F>
-__device__ __forceinline__ void tail_cells(const Geom& g, F&& f) {
-  const int m = g.n1 * g.n2 * g.n3;
-  int idx = threadIdx.x;
-  int i = idx % g.n1, r = idx / g.n1, j = r % g.n2, k = r / g.n2;
-  const int di = TNT % g.n1, r2 = TNT / g.n1, dj = r2 % g.n2, dk = r2 / g.n2;
-  for (; idx < m; idx += TNT) {
-    f(idx, i + 1, j + 1, k + 1);
-    i += di;
-    const int ci = i >= g.n1;
-    if (ci) i -= g.n1;
-    j += dj + ci;
-    const int cj = j >= g.n2;
-    if (cj) j -= g.n2;
-    k += dk + cj;
+// the column segment of a thread: coefficients and neighbour offsets
+template <typename T>
+struct TailCol {
+  int i, j, k0, nk;      // 1-based column, 0-based first plane, planes (0: none)
+  int p;                 // index of (i, j, k0) in the level's compact layout
+  int dW, dE, dS, dN;
+  T a0, a2, b0, b2, s1;  // lateral weights, sum of the x and y diagonal parts
+  T inv;                 // uniform z: omega / diag
+};
+template <typename T>
+__device__ __forceinline__ TailCol<T> tail_col(const TailLevel& L, const T* __restrict__ tb, int c, T omega) {
+  TailCol<T> C;
+  const bool own = c < L.ncs;
+  const int seg = own ? c / L.ncol : 0, col = own ? c - seg * L.ncol : 0;
+  const int j = col / L.n1, i = col - j * L.n1;
+  C.i = i + 1;
+  C.j = j + 1;
+  C.k0 = seg * L.len;
+  C.nk = own ? min(L.len, L.n3 - C.k0) : 0;
+  C.p = col + C.k0 * L.ncol;
+  C.dW = i == 0 ? L.n1 - 1 : -1;
+  C.dE = i == L.n1 - 1 ? 1 - L.n1 : 1;
+  C.dS = j == 0 ? (L.n2 - 1) * L.n1 : -L.n1;
+  C.dN = j == L.n2 - 1 ? -(L.n2 - 1) * L.n1 : L.n1;
+  const T* cx = tb + L.tcd[0] + 3 * i;
+  const T* cy = tb + L.tcd[1] + 3 * j;
+  C.a0 = cx[0];
+  C.a2 = cx[2];
+  C.b0 = cy[0];
+  C.b2 = cy[2];
+  C.s1 = cx[1] + cy[1];
+  C.inv = L.zuni ? omega / (C.s1 + tb[L.tcd[2] + 1]) : T(0);
+  return C;
+}
+
+// One pass over a column segment.  OP 0: dst = init(A); 1: dst = sweep(A, src);
+// 2: dst = A - cdg(src); 3: a Chebyshev step, dst = xm + w (x + g z - xm) with xm = dst's old
+// value (x itself on the first step).  oS, oD: shared-memory offsets of src and dst.
+template <typename T, int OP>
+__device__ __forceinline__ void tail_seg(const TailLevel& L, const TailCol<T>& C, T* sm, const T* __restrict__ tb,
+                                         T omega, int oS, int oD, T w, T gam, bool first) {
+  const bool zu = L.zuni != 0;
+  const T* __restrict__ cz = tb + L.tcd[2];
+  const T zm0 = cz[0], zc0 = cz[1], zp0 = cz[2];
+  const int sz = L.ncol, n3 = L.n3;
+  const int wz = (n3 - 1) * sz;
+  const T* A = sm + L.oA + C.p;
+  const T* s = sm + oS + C.p;
+  T* d = sm + oD + C.p;
+  T xm = T(0), xc = T(0);
+  if (OP != 0 && C.nk > 0) {
+    xm = s[C.k0 == 0 ? wz : -sz];
+    xc = s[0];
+  }
+  for (int k = 0; k < C.nk; ++k) {
+    T cm = zm0, cc = zc0, cp = zp0;
+    if (!zu) {
+      cm = cz[3 * (C.k0 + k)];
+      cc = cz[3 * (C.k0 + k) + 1];
+      cp = cz[3 * (C.k0 + k) + 2];
+    }
+    const T diag = C.s1 + cc;
+    T o;
+    if (OP == 0) {
+      o = jinit(A[0], omega, zu, C.inv, diag);
+    } else {
+      const T zn = s[C.k0 + k + 1 == n3 ? -wz : sz];
+      if (OP == 1) {
+        const T r = jres(A[0], C.a0, s[C.dW], C.a2, s[C.dE], C.b0, s[C.dS], C.b2, s[C.dN], cm, xm, cp, zn);
+        o = jsweep(r, xc, omega, zu, C.inv, diag);
+      } else {
+        o = jresid(A[0], C.a0, s[C.dW], C.a2, s[C.dE], C.b0, s[C.dS], C.b2, s[C.dN], cm, xm, cp, zn, diag, xc);
+        if (OP == 3) {
+          const T old = first ? xc : d[0];
+          o = old + w * (xc + gam * o / diag - old);
+        }
+      }
+      xm = xc;
+      xc = zn;
+    }
+    d[0] = o;
+    A += sz;
+    s += sz;
+    d += sz;
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict__ jobs, const int* __restrict__ ts,
-                                                    int nj, int ntiles, T omega, int n_down, int n_up, int n_bottom) {
+__global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict__ jobs,
+                                                               const int* __restrict__ ts, int nj, int ntiles, T omega,
+                                                               int n_down, int n_up, int n_bottom) {
+  constexpr int NT = TNT;
   extern __shared__ __align__(16) unsigned char tl_raw[];
+  __shared__ TailLevel lev[MG_MAX_LEVELS];
   T* const sm = reinterpret_cast<T*>(tl_raw);
+  T* const stab = sm + TAIL_BYTES / sizeof(T);
+  const int tid = threadIdx.x;
   for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
-    const int q0 = find_job(ts, nj, b);
-    const TailJob<T>& TJ = jobs[q0];
-    if (e_halted(TJ.lv[0].sc)) continue;
+    const TailJob<T>& TJ = jobs[find_job(ts, nj, b)];
+    if (e_halted(TJ.sc)) continue;
     const int nl = TJ.nl;
-    // shared-memory arrays of level q: A, X0, X1 (compact, i fastest)
-    T* Aq[MG_MAX_LEVELS];
-    T* X0[MG_MAX_LEVELS];
-    T* X1[MG_MAX_LEVELS];
-    int cur[MG_MAX_LEVELS];  // which of X0 / X1 holds the level's iterate
-    {
-      size_t o = 0;
-      for (int q = 0; q < nl; ++q) {
-        const Geom& g = TJ.lv[q].g;
-        const size_t m = (size_t)g.n1 * g.n2 * g.n3;
-        Aq[q] = sm + o;
-        X0[q] = sm + o + m;
-        X1[q] = sm + o + 2 * m;
-        o += 3 * m;
-        cur[q] = 0;
-      }
-    }
-    auto X = [&](int q, int which) { return which ? X1[q] : X0[q]; };
-    // right-hand side of the first level from global memory
-    {
-      const Geom& g = TJ.lv[0].g;
-      T* a0 = Aq[0];
-      const T* src = TJ.lv[0].A;
-      tail_cells(g, [&](int idx, int i, int j, int k) { a0[idx] = src[off(g, i, j, k)]; });
-    }
+    const T* __restrict__ gt = TJ.tab;
+    for (int t = tid; t < nl * (int)(sizeof(TailLevel) / 4); t += NT)
+      reinterpret_cast<int*>(lev)[t] = reinterpret_cast<const int*>(TJ.lv)[t];
+    for (int t = tid; t < TJ.ntab; t += NT) stab[t] = gt[t];
+    const T* const tb = TJ.ntab > 0 ? stab : gt;
     __syncthreads();
-    // OP 0: dst = init(A); 1: dst = sweep(A, src); 2: dst = A - cdg(src)
-    auto relax = [&](int q, int op, const T* src, T* dst) {
-      const LevelJob<T>& J = TJ.lv[q];
-      const Geom& g = J.g;
-      const bool zu = J.zuni != 0;
-      const T* __restrict__ cz = J.cdg[2];
-      const T* a = Aq[q];
-      tail_cells(g, [&](int idx, int i, int j, int k) {
-        const T a0 = J.cdg[0][3 * (i - 1)], a1 = J.cdg[0][3 * (i - 1) + 1], a2 = J.cdg[0][3 * (i - 1) + 2];
-        const T b0 = J.cdg[1][3 * (j - 1)], b1 = J.cdg[1][3 * (j - 1) + 1], b2 = J.cdg[1][3 * (j - 1) + 2];
-        const T cm = zu ? cz[0] : cz[3 * (k - 1)], cc = zu ? cz[1] : cz[3 * (k - 1) + 1],
-                cp = zu ? cz[2] : cz[3 * (k - 1) + 2];
-        const T inv = zu ? omega / (a1 + b1 + cz[1]) : T(0);
-        const T diag = a1 + b1 + cc;
-        if (op == 0) {
-          dst[idx] = jinit(a[idx], omega, zu, inv, diag);
-          return;
+    // this thread's segment of a level; a level of more segments than threads walks its further
+    // ones from `each`
+    TailCol<T> C;
+    auto take = [&](const TailLevel& L) { C = tail_col(L, tb, tid, omega); };
+    auto each = [&](const TailLevel& L, auto&& f) {
+      f();
+      if (L.ncs > NT) {
+        for (int c = tid + NT; c < L.ncs; c += NT) {
+          C = tail_col(L, tb, c, omega);
+          f();
         }
-        const int im = i == 1 ? idx + g.n1 - 1 : idx - 1, ip = i == g.n1 ? idx - g.n1 + 1 : idx + 1;
-        const int sy = g.n1, sz = g.n1 * g.n2;
-        const int jm = j == 1 ? idx + (g.n2 - 1) * sy : idx - sy, jp = j == g.n2 ? idx - (g.n2 - 1) * sy : idx + sy;
-        const int km = k == 1 ? idx + (g.n3 - 1) * sz : idx - sz, kp = k == g.n3 ? idx - (g.n3 - 1) * sz : idx + sz;
-        const T zc = src[idx];
-        if (op == 1) {
-          const T rr = jres(a[idx], a0, src[im], a2, src[ip], b0, src[jm], b2, src[jp], cm, src[km], cp, src[kp]);
-          dst[idx] = jsweep(rr, zc, omega, zu, inv, diag);
-        } else {
-          dst[idx] = jresid(a[idx], a0, src[im], a2, src[ip], b0, src[jm], b2, src[jp], cm, src[km], cp, src[kp], diag, zc);
-        }
-      });
-      __syncthreads();
-    };
-    // n sweeps of level q (after an init sweep when init): the iterate moves between X0 and X1
-    auto smooth = [&](int q, int init, int n) {
-      for (int w = 0; w < n; ++w) {
-        if (init && w == 0) {
-          relax(q, 0, nullptr, X(q, cur[q]));
-        } else {
-          relax(q, 1, X(q, cur[q]), X(q, cur[q] ^ 1));
-          cur[q] ^= 1;
-        }
+        C = tail_col(L, tb, tid, omega);
       }
     };
-    // the residual of level q (in its spare buffer) restricted into the right-hand side of q + 1
-    auto restrict_down = [&](int q) {
-      const LevelJob<T>& C = TJ.lv[q + 1];
-      const Geom& gf = TJ.lv[q].g;
-      const Geom& g = C.g;
-      const T* d = X(q, cur[q] ^ 1);
-      T* aq = Aq[q + 1];
-      tail_cells(g, [&](int idx, int i, int j, int k) {
-        const int fi = C.rf[0] * (i - 1) + 1, fj = C.rf[1] * (j - 1) + 1, fk = C.rf[2] * (k - 1) + 1;
-        auto at = [&](int a, int bq, int c) { return d[(a - 1) + gf.n1 * ((bq - 1) + gf.n2 * (c - 1))]; };
-        aq[idx] = restrict7(at(fi, fj, fk), at(wrapi(fi - 1, gf.n1), fj, fk), at(wrapi(fi + 1, gf.n1), fj, fk),
-                            at(fi, wrapi(fj - 1, gf.n2), fk), at(fi, wrapi(fj + 1, gf.n2), fk),
-                            at(fi, fj, wrapi(fk - 1, gf.n3)), at(fi, fj, wrapi(fk + 1, gf.n3)));
-      });
-      __syncthreads();
+    auto pass = [&](const TailLevel& L, auto op, int oS, int oD, T w, T gam, bool first) {
+      each(L, [&]() { tail_seg<T, decltype(op)::value>(L, C, sm, tb, omega, oS, oD, w, gam, first); });
     };
-    // spare buffer of level q = its iterate + P (iterate of q + 1); then it holds the iterate
-    auto prolong_up = [&](int q) {
-      const LevelJob<T>& J = TJ.lv[q];
-      const Geom& g = J.g;
-      const Geom& gc = TJ.lv[q + 1].g;
-      const T* xf = X(q, cur[q]);
-      const T* xc = X(q + 1, cur[q + 1]);
-      T* out = X(q, cur[q] ^ 1);
-      tail_cells(g, [&](int idx, int i, int j, int k) {
-        int xl, xh, yl, yh, zl, zh;
-        bool mx, my, mz;
-        bracket(i, J.rc[0], gc.n1, xl, xh, mx);
-        bracket(j, J.rc[1], gc.n2, yl, yh, my);
-        bracket(k, J.rc[2], gc.n3, zl, zh, mz);
-        auto P = [&](int a, int bq, int c) { return xc[(a - 1) + gc.n1 * ((bq - 1) + gc.n2 * (c - 1))]; };
-        const T wz0 = J.cI[2][2 * k], wz1 = J.cI[2][2 * k + 1];
-        const T wy0 = J.cI[1][2 * j], wy1 = J.cI[1][2 * j + 1];
-        const T wx0 = J.cI[0][2 * i], wx1 = J.cI[0][2 * i + 1];
-        const T Z0 = pmix(mz, wz0, P(xl, yl, zl), wz1, P(xl, yl, zh));
-        const T Z1 = pmix(mz, wz0, P(xl, yh, zl), wz1, P(xl, yh, zh));
-        const T Z2 = pmix(mz, wz0, P(xh, yl, zl), wz1, P(xh, yl, zh));
-        const T Z3 = pmix(mz, wz0, P(xh, yh, zl), wz1, P(xh, yh, zh));
-        const T Yl = pmix(my, wy0, Z0, wy1, Z1);
-        const T Yh = pmix(my, wy0, Z2, wy1, Z3);
-        out[idx] = xf[idx] + pmix(mx, wx0, Yl, wx1, Yh);
-      });
-      cur[q] ^= 1;
-      __syncthreads();
-    };
-    for (int q = 0; q + 1 < nl; ++q) {  // relax_restrict
-      smooth(q, 1, n_down);
-      relax(q, 2, X(q, cur[q]), X(q, cur[q] ^ 1));
-      restrict_down(q);
-    }
-    if (TJ.cheb > 0) {  // Chebyshev semi-iteration on the coarsest level, from x = 0
-      const int q = nl - 1;
-      const LevelJob<T>& J = TJ.lv[q];
-      const Geom& g = J.g;
-      const bool zu = J.zuni != 0;
-      const T* __restrict__ cz = J.cdg[2];
-      const T* a = Aq[q];
-      T* x0 = X0[q];
-      T* x1 = X1[q];
-      tail_cells(g, [&](int idx, int, int, int) { x0[idx] = T(0); x1[idx] = T(0); });
-      __syncthreads();
-      const T gam = TJ.cgam, s2 = TJ.csig2;
-      T w = T(1);
-      for (int it = 0; it < TJ.cheb; ++it) {
-        w = it == 0 ? T(1) : (it == 1 ? T(2) / (T(2) - s2) : T(1) / (T(1) - s2 * w / T(4)));
-        const T* src = X(q, cur[q]);
-        T* dst = X(q, cur[q] ^ 1);  // holds x_{k-1} (x_0 = 0 on the first step)
-        tail_cells(g, [&](int idx, int i, int j, int k) {
-          const T a0 = J.cdg[0][3 * (i - 1)], a1 = J.cdg[0][3 * (i - 1) + 1], a2 = J.cdg[0][3 * (i - 1) + 2];
-          const T b0 = J.cdg[1][3 * (j - 1)], b1 = J.cdg[1][3 * (j - 1) + 1], b2 = J.cdg[1][3 * (j - 1) + 2];
-          const T cm = zu ? cz[0] : cz[3 * (k - 1)], cc = zu ? cz[1] : cz[3 * (k - 1) + 1],
-                  cp = zu ? cz[2] : cz[3 * (k - 1) + 2];
-          const T diag = a1 + b1 + cc;
-          const int im = i == 1 ? idx + g.n1 - 1 : idx - 1, ip = i == g.n1 ? idx - g.n1 + 1 : idx + 1;
-          const int sy = g.n1, sz = g.n1 * g.n2;
-          const int jm = j == 1 ? idx + (g.n2 - 1) * sy : idx - sy, jp = j == g.n2 ? idx - (g.n2 - 1) * sy : idx + sy;
-          const int km = k == 1 ? idx + (g.n3 - 1) * sz : idx - sz, kp = k == g.n3 ? idx - (g.n3 - 1) * sz : idx + sz;
-          const T xk = src[idx];
-          const T r = jresid(a[idx], a0, src[im], a2, src[ip], b0, src[jm], b2, src[jp], cm, src[km], cp, src[kp], diag, xk);
-          const T xm = it == 0 ? xk : dst[idx];
-          dst[idx] = xm + w * (xk + gam * r / diag - xm);
-        });
-        cur[q] ^= 1;
+    // barrier of the warps that own cells of level L (the others do not come here)
+    auto level_sync = [&](const TailLevel& L) {
+      if (L.nthr == NT)
         __syncthreads();
+      else
+        asm volatile("bar.sync 1, %0;\n" ::"r"(L.nthr) : "memory");
+    };
+    // n sweeps of a level (after an init sweep when init) from its field oX[cur]; a barrier of the
+    // level after every pass but the last
+    auto smooth = [&](const TailLevel& L, unsigned& cur, int init, int n) {
+      for (int w = 0; w < n; ++w) {
+        if (w > 0) level_sync(L);
+        if (init && w == 0) {
+          pass(L, std::integral_constant<int, 0>{}, 0, L.oX[cur], T(0), T(0), false);
+        } else {
+          pass(L, std::integral_constant<int, 1>{}, L.oX[cur], L.oX[cur ^ 1], T(0), T(0), false);
+          cur ^= 1;
+        }
       }
-    } else {
-      smooth(nl - 1, 1, n_bottom);  // relax_bottom
-      smooth(nl - 1, 0, n_bottom);
+    };
+    unsigned curs = 0;  // bit q: which of the two fields holds the iterate of level q
+    auto get = [&](int q) { return (curs >> q) & 1u; };
+    auto put = [&](int q, unsigned c) { curs = (curs & ~(1u << q)) | (c << q); };
+    // the residual of level q (in its spare field) restricted into the right-hand side of q + 1:
+    // every thread forms the cells it owns there
+    auto restrict_down = [&](const TailLevel& F, const TailLevel& L, int oD) {
+      each(L, [&]() {
+        const int fi = L.rf[0] * (C.i - 1), fj = L.rf[1] * (C.j - 1);  // 0-based fine column
+        const int xm = fi == 0 ? F.n1 - 1 : -1, xp = fi == F.n1 - 1 ? 1 - F.n1 : 1;
+        const int ym = fj == 0 ? (F.n2 - 1) * F.n1 : -F.n1, yp = fj == F.n2 - 1 ? -(F.n2 - 1) * F.n1 : F.n1;
+        const int wz = (F.n3 - 1) * F.ncol;
+        const T* d0 = sm + oD + fi + F.n1 * fj;
+        T* a = sm + L.oA + C.p;
+        for (int k = 0; k < C.nk; ++k) {
+          const int fk = L.rf[2] * (C.k0 + k);
+          const T* d = d0 + F.ncol * fk;
+          a[k * L.ncol] = restrict7(d[0], d[xm], d[xp], d[ym], d[yp], d[fk == 0 ? wz : -F.ncol],
+                                    d[fk == F.n3 - 1 ? -wz : F.ncol]);
+        }
+      });
+    };
+    // spare field of level L = its iterate + P (iterate of the next coarser level G)
+    auto prolong_up = [&](const TailLevel& L, const TailLevel& G, int oF, int oO, int oC) {
+      each(L, [&]() {
+        int xl, xh, yl, yh;
+        bool mx, my;
+        bracket(C.i, L.rc[0], G.n1, xl, xh, mx);
+        bracket(C.j, L.rc[1], G.n2, yl, yh, my);
+        const T wx0 = tb[L.tcI[0] + 2 * C.i], wx1 = tb[L.tcI[0] + 2 * C.i + 1];
+        const T wy0 = tb[L.tcI[1] + 2 * C.j], wy1 = tb[L.tcI[1] + 2 * C.j + 1];
+        const T* cI3 = tb + L.tcI[2];
+        const int o0 = (xl - 1) + G.n1 * (yl - 1), o1 = (xl - 1) + G.n1 * (yh - 1);
+        const int o2 = (xh - 1) + G.n1 * (yl - 1), o3 = (xh - 1) + G.n1 * (yh - 1);
+        const T* xc = sm + oC;
+        const T* xf = sm + oF + C.p;
+        T* out = sm + oO + C.p;
+        for (int k = 0; k < C.nk; ++k) {
+          const int kk = C.k0 + k + 1;
+          int zl, zh;
+          bool mz;
+          bracket(kk, L.rc[2], G.n3, zl, zh, mz);
+          const T wz0 = cI3[2 * kk], wz1 = cI3[2 * kk + 1];
+          const T* pl = xc + (zl - 1) * G.ncol;
+          const T* ph = xc + (zh - 1) * G.ncol;
+          const T Z0 = pmix(mz, wz0, pl[o0], wz1, ph[o0]);
+          const T Z1 = pmix(mz, wz0, pl[o1], wz1, ph[o1]);
+          const T Z2 = pmix(mz, wz0, pl[o2], wz1, ph[o2]);
+          const T Z3 = pmix(mz, wz0, pl[o3], wz1, ph[o3]);
+          const T Yl = pmix(my, wy0, Z0, wy1, Z1);
+          const T Yh = pmix(my, wy0, Z2, wy1, Z3);
+          out[k * L.ncol] = xf[k * L.ncol] + pmix(mx, wx0, Yl, wx1, Yh);
+        }
+      });
+    };
+    {  // right-hand side of the first level from global memory: every thread its own cells
+      const TailLevel& L = lev[0];
+      take(L);
+      const Geom g = TJ.g;
+      const T* __restrict__ src = TJ.A;
+      each(L, [&]() {
+        const T* s = src + off(g, C.i, C.j, C.k0 + 1);
+        for (int k = 0; k < C.nk; ++k) cp_async1(sm + L.oA + C.p + k * L.ncol, s + k * g.nxy);
+      });
+    }
+    cp_commit();
+    cp_wait<0>();
+    for (int q = 0; q + 1 < nl; ++q) {  // relax_restrict
+      const TailLevel& L = lev[q];
+      unsigned cur = 0;
+      if (tid < L.nthr) {
+        smooth(L, cur, 1, n_down);
+        level_sync(L);
+        pass(L, std::integral_constant<int, 2>{}, L.oX[cur], L.oX[cur ^ 1], T(0), T(0), false);
+      }
+      cur = (n_down - 1) & 1;  // the same in the warps without cells
+      put(q, cur);
+      __syncthreads();
+      take(lev[q + 1]);
+      restrict_down(L, lev[q + 1], L.oX[cur ^ 1]);
+    }
+    {
+      const TailLevel& L = lev[nl - 1];
+      unsigned cur = 0;
+      if (TJ.cheb > 0) {  // Chebyshev semi-iteration on the coarsest level, from x = 0
+        const int steps = TJ.cheb;
+        if (tid < L.nthr) {
+          each(L, [&]() {
+            for (int k = 0; k < C.nk; ++k) sm[L.oX[0] + C.p + k * L.ncol] = sm[L.oX[1] + C.p + k * L.ncol] = T(0);
+          });
+          const T gam = TJ.cgam, s2 = TJ.csig2;
+          T w = T(1);
+          for (int it = 0; it < steps; ++it) {
+            level_sync(L);
+            w = it == 0 ? T(1) : (it == 1 ? T(2) / (T(2) - s2) : T(1) / (T(1) - s2 * w / T(4)));
+            pass(L, std::integral_constant<int, 3>{}, L.oX[cur], L.oX[cur ^ 1], w, gam, it == 0);
+            cur ^= 1;
+          }
+        }
+        cur = steps & 1;
+      } else {  // relax_bottom: n_bottom sweeps from an init sweep, n_bottom more
+        if (tid < L.nthr) smooth(L, cur, 1, 2 * n_bottom);
+        cur = (2 * n_bottom - 1) & 1;
+      }
+      put(nl - 1, cur);
     }
     for (int q = nl - 2; q >= 0; --q) {  // interpolate_relax
-      prolong_up(q);
-      smooth(q, 0, n_up);
+      const TailLevel& L = lev[q];
+      __syncthreads();  // level q + 1's iterate is complete
+      unsigned cur = get(q);
+      take(L);
+      prolong_up(L, lev[q + 1], L.oX[cur], L.oX[cur ^ 1], lev[q + 1].oX[get(q + 1)]);
+      cur ^= 1;
+      if (tid < L.nthr && n_up > 0) {
+        level_sync(L);
+        unsigned c = cur;
+        smooth(L, c, 0, n_up);
+      }
+      put(q, cur ^ (n_up & 1));
     }
-    {
-      const Geom& g = TJ.lv[0].g;
-      const T* x0 = X(0, cur[0]);
-      T* dst = TJ.lv[0].B;
-      tail_cells(g, [&](int idx, int i, int j, int k) { dst[off(g, i, j, k)] = x0[idx]; });
+    {  // every thread stores its own cells
+      const TailLevel& L = lev[0];
+      const Geom g = TJ.g;
+      T* __restrict__ dst = TJ.B;
+      const int o = L.oX[get(0)];
+      each(L, [&]() {
+        T* d = dst + off(g, C.i, C.j, C.k0 + 1);
+#pragma unroll 4
+        for (int k = 0; k < C.nk; ++k) d[k * g.nxy] = sm[o + C.p + k * L.ncol];
+      });
     }
     __syncthreads();  // shared memory is rewritten by the next case
   }
@@ -2788,8 +2894,8 @@ void ax_attributes() {
                                occ(k_kr_ax32v<2>, AXV_NT, axv_smem_bytes())});
   g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<1>, AXD_NT, axd_smem_bytes()),
                                occ(k_kr_ax64v<2>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<3>, AXD_NT, axd_smem_bytes())});
-  cudaFuncSetAttribute(k_lv_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_BYTES);
-  cudaFuncSetAttribute(k_lv_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_BYTES);
+  cudaFuncSetAttribute(k_lv_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
+  cudaFuncSetAttribute(k_lv_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
 #define IMPACT_MULTI_ATTR(T, N, I, R)                                                                           \
   cudaFuncSetAttribute(k_lv_multi<T, N, I, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
                        (int)multi_smem_bytes<T, N, I, R>());                                                    \
@@ -3173,6 +3279,47 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       if (first >= 0 && (nlev[c] - first >= 2 || p_.bottom_cheb > 0)) lt[c] = first;
     }
   }
+  // the tail of case c from level lt on: level descriptions and the run of tables that holds theirs
+  auto tail_job = [&](int c, int lt0, int nlv, int variant) {
+    TailJob<T> job{};
+    const MGData<T>& mg = *cs[c].mg;
+    const LevelJob<T> first = lvjob(c, lt0, variant);
+    job.nl = nlv - lt0;
+    job.g = first.g;
+    job.A = first.A;
+    job.B = first.B;
+    job.sc = first.sc;
+    job.tab = mg.lv[lt0].cdg[0];
+    const Geom& gl = mg.lv[nlv - 1].g;
+    const long long ntab = (mg.lv[nlv - 1].cI[2] + 2 * (gl.n3 + 2)) - job.tab;
+    job.ntab = ntab > 0 && ntab * (long long)sizeof(T) <= (long long)TAIL_TAB_BYTES ? (int)ntab : 0;
+    int o = 0;
+    for (int q = 0; q < job.nl; ++q) {
+      const MGLevel<T>& M = mg.lv[lt0 + q];
+      TailLevel& L = job.lv[q];
+      const int m = M.g.n1 * M.g.n2 * M.g.n3;
+      L.n1 = M.g.n1;
+      L.n2 = M.g.n2;
+      L.n3 = M.g.n3;
+      L.zuni = M.zuni;
+      L.ncol = L.n1 * L.n2;
+      const int segs = std::max(1, std::min(L.n3, TNT / L.ncol));
+      L.len = (L.n3 + segs - 1) / segs;
+      L.ncs = L.ncol * ((L.n3 + L.len - 1) / L.len);
+      L.nthr = std::min(TNT, (L.ncs + 31) / 32 * 32);
+      L.oA = o;
+      L.oX[0] = o + m;
+      L.oX[1] = o + 2 * m;
+      o += 3 * m;
+      for (int a = 0; a < 3; ++a) {
+        L.rf[a] = lt0 + q > 0 ? mg.lv[lt0 + q - 1].ratio[a] : 1;
+        L.rc[a] = M.ratio[a];
+        L.tcd[a] = (int)(M.cdg[a] - job.tab);
+        L.tcI[a] = (int)(M.cI[a] - job.tab);
+      }
+    }
+    return job;
+  };
   auto in_lists = [&](int c, int g) { return lt[c] < 0 || g < lt[c]; };
   if (use_mg) {
     // fused smoothing phases for the sweep counts that have kernels
@@ -3203,9 +3350,7 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
         if (lt[c] < 0) {
           bot.push_back({c, nlev[c] - 1});
         } else {
-          TailJob<T> job{};
-          job.nl = nlev[c] - lt[c];
-          for (int q = 0; q < job.nl; ++q) job.lv[q] = lvjob(c, lt[c] + q, v);
+          TailJob<T> job = tail_job(c, lt[c], nlev[c], v);
           if (p_.bottom_cheb > 0) {
             const double lo = std::max(1e-6, std::min(1.0, cs[c].mg->lv[nlev[c] - 1].lmin));
             const double sg = (2.0 - lo) / (2.0 + lo);
@@ -3350,7 +3495,7 @@ void Engine<T>::enqueue_phase(const Phase& ph) {
       break;
     case PH_TAIL:  // one block per case; bytes: read the first level's right-hand side, write its iterate
       IMPACT_PROF(prof::K_MG_TAIL, 2 * sz * c, s,
-                  (k_lv_tail<T><<<L.ntiles, TNT, TAIL_BYTES, s>>>(static_cast<const TailJob<T>*>(L.jobs), L.ts, L.njobs,
+                  (k_lv_tail<T><<<L.ntiles, TNT, TAIL_BYTES + TAIL_TAB_BYTES, s>>>(static_cast<const TailJob<T>*>(L.jobs), L.ts, L.njobs,
                                                                   L.ntiles, om, p_.mg_down, p_.mg_up, p_.mg_bottom)));
       break;
     default:

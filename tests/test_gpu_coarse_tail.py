@@ -1,0 +1,33 @@
+"""The one-block coarse tail of the V-cycle (k_lv_tail) at the edges of its thread mapping and of
+its shared memory: levels with more columns than threads, one plane or a partial segment per
+thread, two-point axes, and tables too long to be staged.  Like every fused phase it must give the
+iterate of the one-launch-per-phase schedule (which has no tail) bit for bit."""
+import numpy as np
+import pytest
+
+import impact_b200 as I
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [((33, 33, 9), (1.0, 1.0, 0.25), (0, 0, 0)),      # first tail level 32 x 32 x 8: 1024 columns
+         ((49, 25, 13), (1.0, 0.5, 0.25), (1, 0, 1)),     # 48 x 24 x 12, z rows differ
+         ((9, 9, 1201), (0.1, 0.1, 15.0), (0, 0, 0)),     # 4 x 4 x 600 and coarser: tables of 6000 values
+         ((21, 13, 37), (1.0, 0.6, 1.8), (0, 0, 0)),      # 20 x 12 x 36 -> 5 x 3 x 9
+         ((9, 9, 9), (1.0, 1.0, 1.0), (0, 0, 0))]         # 8 x 8 x 8 -> 2 x 2 x 2
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("gi", range(len(GRIDS)), ids=["32x32x8", "48x24x12-xz", "8x8x1200", "20x12x36", "8x8x8"])
+@pytest.mark.parametrize("sw", [(1, 1, 1), (2, 3, 1), (3, 2, 3)], ids=lambda s: "%d%d%d" % s)
+def test_coarse_tail_equals_one_launch_per_phase(gi, sw, precision):
+    g = I.Grid(*GRIDS[gi])
+    case = I.Case(g, precision=precision)
+    case.upload("res", np.random.default_rng(31).uniform(-1.0, 1.0, g.shape))
+    out = []
+    for unfused in (1, 0):
+        case.precond("res", "pre", I.solver_params(precond=1, mg_down=sw[0], mg_up=sw[1], mg_bottom=sw[2],
+                                                   smooth_unfused=unfused))
+        out.append(g.interior(case.download("pre")).copy())
+    assert np.isfinite(out[0]).all()
+    assert np.array_equal(out[0], out[1])
+    case.close()

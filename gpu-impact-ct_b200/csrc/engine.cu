@@ -2861,6 +2861,7 @@ __global__ void __launch_bounds__(ENT) k_mx_apply(const MixJob* __restrict__ job
 // grids of the vector operator kernels: the blocks resident at once on the device (a grid-stride
 // kernel given more would leave its last blocks to run after the others, one tile step behind)
 int g_axv_grid = 0, g_axd_grid = 0;
+int g_axs32_grid = 0, g_axs64_grid = 0;  // the same of the staged operator kernels
 // the operator kernels use more than 48 KB of dynamic shared memory: opt in once per process
 // and device
 void ax_attributes() {
@@ -2894,6 +2895,8 @@ void ax_attributes() {
                                occ(k_kr_ax32v<2>, AXV_NT, axv_smem_bytes())});
   g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<1>, AXD_NT, axd_smem_bytes()),
                                occ(k_kr_ax64v<2>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<3>, AXD_NT, axd_smem_bytes())});
+  g_axs32_grid = nsm * occ(k_kr_ax32<1>, AXNT, axa_smem_bytes());
+  g_axs64_grid = nsm * occ(k_kr_ax<double, 1>, AXNT, ax_smem_bytes<double>());
   cudaFuncSetAttribute(k_lv_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
   cudaFuncSetAttribute(k_lv_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
 #define IMPACT_MULTI_ATTR(T, N, I, R)                                                                           \
@@ -2914,14 +2917,17 @@ void ax_attributes() {
 }
 
 int g_sms = 0;
-inline int grid_for(int ntiles) {
+inline int device_sms() {
   if (g_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
     if (g_sms <= 0) g_sms = 148;
   }
-  const int cap = g_sms * 8;
+  return g_sms;
+}
+inline int grid_for(int ntiles) {
+  const int cap = device_sms() * 8;
   return ntiles < cap ? ntiles : cap;
 }
 const dim3 kBlock(ETX, ETY);
@@ -2945,6 +2951,48 @@ void launch_ax(int grid, const KrylovJob<T>* J, const int* ts, int n, int ntiles
 }
 // the fused smoothing kernel runs one block per tile (one block per SM at a time)
 inline int grid_multi(int ntiles) { return ntiles; }
+
+// Tile depth of one grid in a Krylov list, at most kc (the solver parameter tile_kc or its
+// default).  A tile is a serial chain of planes after a prologue of about 8 planes' time (the
+// job's scalars; in the operator the z window and the first staged group), so the depth minimises
+// waves of tiles over the kernel's resident blocks x (depth + 8), among kc, the multiples of 8
+// below it (the vector updates walk blocks of 8 planes) and 4.  Grids of many waves keep kc; on
+// 32 x 32 x 64 the 4 tiles of 64 planes become 64 of 4 (FP32 operator 26.6 -> 6.2 us, x update
+// 14.4 -> 4.3 us).  It depends on the grid alone, so a case's partial sums do not depend on its
+// batch.
+constexpr int kVecBlocksPerSm = 4;  // resident blocks of the vector updates
+template <typename TilesXY>
+inline int depth_for(TilesXY&& tiles, int n3, int kc, int slots) {
+  int best = kc;
+  long long cost = -1;
+  auto consider = [&](int d) {
+    const long long c = (tiles(d) + slots - 1) / slots * (std::min(d, n3) + 8);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = d;
+    }
+  };
+  consider(kc);
+  for (int d = (kc - 1) / 8 * 8; d >= 8; d -= 8) consider(d);
+  if (kc > 4) consider(4);
+  return best;
+}
+inline int krylov_depth(const Geom& g, int kc, int slots) {
+  return depth_for([&](int d) { return (long long)tiles_of(g, d); }, g.n3, kc, slots);
+}
+// the depth of a list without partial sums: the same rule over all its grids together (the small
+// grids of a batch need no shallow tiles of their own to fill the GPU)
+inline int list_depth(const std::vector<Geom>& gs, int kc, int slots) {
+  int n3 = 0;
+  for (const Geom& g : gs) n3 = std::max(n3, g.n3);
+  return depth_for(
+      [&](int d) {
+        long long t = 0;
+        for (const Geom& g : gs) t += tiles_of(g, d);
+        return t;
+      },
+      n3, kc, slots);
+}
 
 }  // namespace
 
@@ -3085,9 +3133,6 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
   const int kc = p_.kc;
   cudaError_t e = cudaMalloc((void**)&scal_, n * sizeof(SolverScalars));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&scal_host_, n * sizeof(SolverScalars));
-  long long tiles_fine = 0;
-  for (const auto& c : cs) tiles_fine += tiles_of(c.g, kc);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&partial_, (size_t)(tiles_fine * 4 + 64) * sizeof(double));
   if (e != cudaSuccess) {
     release();
     return impact_set_error(e, "engine allocation", __FILE__, __LINE__);
@@ -3116,7 +3161,6 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       J.z1 = pre_on ? C.z1 : C.pp;
       J.z2 = pre_on ? C.z2 : C.rr;
       J.sc = scal_ + c;
-      kt[c] = tiles_of(C.g, kc);
     }
     // the vector kernels take the jobs whose rows hold whole 16-byte vectors and whose fields are
     // 16-byte aligned: FP32 (k_kr_ax32v) n1 % 4 == 0, n1 >= 8, with uniform x and z weights (it
@@ -3133,7 +3177,40 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       nv += J.vec;
     }
     kr_vec_ = nv == 0 ? 0 : (nv == n ? 1 : 2);
+    // FP64 with JOR sweeps (about 100 iterations) keeps kc: so many iterations carry the last bits
+    // of the inner products up to the solve's tolerance, and another depth would sum them in
+    // another order
+    constexpr bool f32 = std::is_same<T, float>::value;
+    const bool adapt = f32 || use_mg;
+    auto depths = [&](auto slots) {
+      long long tiles = 0;
+      for (int c = 0; c < n; ++c) {
+        kj[c].kc = adapt ? krylov_depth(kj[c].g, kc, slots(kj[c])) : kc;
+        kt[c] = tiles_of(kj[c].g, kj[c].kc);
+        tiles += kt[c];
+      }
+      return tiles;
+    };
+    const long long ta = depths([&](const KrylovJob<T>& J) {
+      return std::min(J.vec ? (f32 ? g_axv_grid : g_axd_grid) : (f32 ? g_axs32_grid : g_axs64_grid),
+                      device_sms() * kVecBlocksPerSm);
+    });
     kr_list_ = arena_.add(kj, kt);
+    const long long tv = depths([&](const KrylovJob<T>&) { return device_sms() * kVecBlocksPerSm; });
+    kv_list_ = arena_.add(kj, kt);
+    std::vector<Geom> gs;
+    for (const auto& J : kj) gs.push_back(J.g);
+    const int dl = list_depth(gs, kc, device_sms() * kVecBlocksPerSm);
+    for (int c = 0; c < n; ++c) {
+      kj[c].kc = dl;
+      kt[c] = tiles_of(kj[c].g, dl);
+    }
+    ku_list_ = arena_.add(kj, kt);
+    e = cudaMalloc((void**)&partial_, (size_t)(std::max(ta, tv) * 4 + 64) * sizeof(double));
+    if (e != cudaSuccess) {
+      release();
+      return impact_set_error(e, "engine allocation", __FILE__, __LINE__);
+    }
   }
   // ---- preconditioner schedules ----
   auto lvjob = [&](int c, int g, int variant) {
@@ -3193,6 +3270,8 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     double c = 0.0;
     for (const auto& C : cs) c += vol(C.g);
     note(kr_list_, c, 0.0, 0.0);
+    note(kv_list_, c, 0.0, 0.0);
+    note(ku_list_, c, 0.0, 0.0);
   }
   // vec: allow several columns per thread (lists walked by the smoothing and residual kernels);
   // the restriction lists keep one column per thread.  fusedS > 0: a list of the fused smoothing
@@ -3511,23 +3590,27 @@ void Engine<T>::enqueue_precond(int variant) {
 template <typename T>
 void Engine<T>::enqueue_iteration() {
   const DevList& K = arena_.lists[kr_list_];
+  const DevList& W = arena_.lists[kv_list_];
+  const DevList& U = arena_.lists[ku_list_];
   const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
+  const KrylovJob<T>* JW = static_cast<const KrylovJob<T>*>(W.jobs);
+  const KrylovJob<T>* JU = static_cast<const KrylovJob<T>*>(U.jobs);
   const int n = K.njobs;
-  const int grid = grid_for(K.ntiles);
+  const int grid = grid_for(K.ntiles), gw = grid_for(W.ntiles), gu = grid_for(U.ntiles);
   cudaStream_t s = s_;
   const double fb = sizeof(T) * cells_[kr_list_];
   k_ebegin<<<(n + 31) / 32, 32, 0, s>>>(scal_, n);
   prof::count(1);
-  IMPACT_PROF(prof::K_P_UPDATE, 4 * fb, s, (k_kr_p<T><<<grid, kBlock, 0, s>>>(J, K.ts, n, K.ntiles)));
+  IMPACT_PROF(prof::K_P_UPDATE, 4 * fb, s, (k_kr_p<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(0);
   IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_)));
   k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 1, 0, EFIN_ALPHA, scal_, nullptr);
-  IMPACT_PROF(prof::K_R_UPDATE, 3 * fb, s, (k_kr_r<T><<<grid, kBlock, 0, s>>>(J, K.ts, n, K.ntiles)));
+  IMPACT_PROF(prof::K_R_UPDATE, 3 * fb, s, (k_kr_r<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(1);
   IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_)));
   k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 2, 0, EFIN_OMEGA, scal_, nullptr);
-  IMPACT_PROF(prof::K_X_UPDATE, 8 * fb, s, (k_kr_x<T><<<grid, kBlock, 0, s>>>(J, K.ts, n, K.ntiles, partial_)));
-  k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 3, 1, EFIN_NORMS, scal_, nullptr);
+  IMPACT_PROF(prof::K_X_UPDATE, 8 * fb, s, (k_kr_x<T><<<gw, kBlock, 0, s>>>(JW, W.ts, n, W.ntiles, partial_)));
+  k_efin<<<n, 256, 0, s>>>(W.ts, partial_, 3, 1, EFIN_NORMS, scal_, nullptr);
   prof::count(3);
 }
 
@@ -3566,6 +3649,9 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
   const DevList& K = arena_.lists[kr_list_];
   const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
   const int grid = grid_for(K.ntiles);
+  const DevList& W = arena_.lists[kv_list_];
+  const KrylovJob<T>* JW = static_cast<const KrylovJob<T>*>(W.jobs);
+  const int gw = grid_for(W.ntiles);
   if (zero_phi && ext_partial) {  // rh = bb = pp = r0 and its norms come from the caller's kernel
     k_efin<<<n, 256, 0, s_>>>(ext_ts, ext_partial, 4, 1, EFIN_INIT_EXT, scal_, nullptr);
     prof::count(1);
@@ -3575,8 +3661,8 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
       prof::count(1);
     }
     IMPACT_PROF(prof::K_KR_INIT, 4.0 * sizeof(T) * cells_[kr_list_], s_,
-                (k_kr_init<T><<<grid, kBlock, 0, s_>>>(J, K.ts, n, K.ntiles, zero_phi, partial_)));
-    k_efin<<<n, 256, 0, s_>>>(K.ts, partial_, 4, 1, EFIN_INIT, scal_, nullptr);
+                (k_kr_init<T><<<gw, kBlock, 0, s_>>>(JW, W.ts, n, W.ntiles, zero_phi, partial_)));
+    k_efin<<<n, 256, 0, s_>>>(W.ts, partial_, 4, 1, EFIN_INIT, scal_, nullptr);
     prof::count(1);
   }
   const int chunk = p_.check_every > 0 ? p_.check_every : 1;
@@ -3625,8 +3711,8 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
       if (scal_host_[c].status == 4) reset = true;
     if (reset) {
       // rhr == 0: new shadow residual rh = rr, as the reference does, then redo the iteration start
-      k_kr_reset<T><<<grid, kBlock, 0, s_>>>(J, K.ts, n, K.ntiles, partial_);
-      k_efin<<<n, 256, 0, s_>>>(K.ts, partial_, 1, 0, EFIN_RESET, scal_, nullptr);
+      k_kr_reset<T><<<gw, kBlock, 0, s_>>>(JW, W.ts, n, W.ntiles, partial_);
+      k_efin<<<n, 256, 0, s_>>>(W.ts, partial_, 1, 0, EFIN_RESET, scal_, nullptr);
       prof::count(2);
       continue;
     }
@@ -3688,6 +3774,11 @@ int Engine<T>::bench(int kind, int iters, double* ms, double* bytes) {
   const DevList& K = arena_.lists[kr_list_];
   const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
   const int grid = grid_for(K.ntiles);
+  const DevList& W = arena_.lists[kv_list_];
+  const KrylovJob<T>* JW = static_cast<const KrylovJob<T>*>(W.jobs);
+  const DevList& U = arena_.lists[ku_list_];
+  const KrylovJob<T>* JU = static_cast<const KrylovJob<T>*>(U.jobs);
+  const int gw = grid_for(W.ntiles), gu = grid_for(U.ntiles);
   const double sz = sizeof(T), fc = cells_[kr_list_];
   double by = 0.0;
   std::function<void()> f;
@@ -3723,15 +3814,15 @@ int Engine<T>::bench(int kind, int iters, double* ms, double* bytes) {
       break;
     case 7:
       by = 8 * sz * fc;
-      f = [&]() { k_kr_x<T><<<grid, kBlock, 0, s_>>>(J, K.ts, n, K.ntiles, partial_); };
+      f = [&]() { k_kr_x<T><<<gw, kBlock, 0, s_>>>(JW, W.ts, n, W.ntiles, partial_); };
       break;
     case 8:
       by = 4 * sz * fc;
-      f = [&]() { k_kr_p<T><<<grid, kBlock, 0, s_>>>(J, K.ts, n, K.ntiles); };
+      f = [&]() { k_kr_p<T><<<gu, kBlock, 0, s_>>>(JU, U.ts, n, U.ntiles); };
       break;
     case 9:
       by = 3 * sz * fc;
-      f = [&]() { k_kr_r<T><<<grid, kBlock, 0, s_>>>(J, K.ts, n, K.ntiles); };
+      f = [&]() { k_kr_r<T><<<gu, kBlock, 0, s_>>>(JU, U.ts, n, U.ntiles); };
       break;
     case 10:
       f = [this]() { enqueue_precond(0); };
@@ -3807,10 +3898,7 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
   int rc = inner_.build(ic, p, s);
   if (rc) return rc;
   const int kc = inner_.params().kc;
-  long long tiles = 0;
-  for (const Case& c : cs) tiles += tiles_of(c.g, kc);
-  cudaError_t e = cudaMalloc((void**)&partial_, (size_t)(tiles * 4 + 64) * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&q_, (size_t)n * 4 * sizeof(double));
+  cudaError_t e = cudaMalloc((void**)&q_, (size_t)n * 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&q_host_, (size_t)n * 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc((void**)&oscal_, (size_t)n * sizeof(SolverScalars));
   if (e != cudaSuccess) {
@@ -3820,13 +3908,16 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
   cudaMemsetAsync(oscal_, 0, (size_t)n * sizeof(SolverScalars), s);
   std::vector<KrylovJob<double>> aj(n);
   std::vector<MixJob> mj(n);
-  std::vector<int> t(n);
+  std::vector<int> t(n), tm(n);
+  long long tiles = 0;
+  std::vector<Geom> gs;
+  for (const Case& c : cs) gs.push_back(c.g);
+  const int dl = list_depth(gs, kc, device_sms() * kVecBlocksPerSm);
   for (int c = 0; c < n; ++c) {
     const Case& C = cs[c];
     KrylovJob<double>& A = aj[c];
     A = KrylovJob<double>{};
     A.g = C.g;
-    A.kc = kc;
     for (int m = 0; m < 3; ++m) A.W[m] = C.W64[m];
     A.zuni = C.zuni;
     A.xuni = C.xuni;
@@ -3842,7 +3933,6 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
     MixJob& M = mj[c];
     M = MixJob{};
     M.g = C.g;
-    M.kc = kc;
     M.bb = C.bb;
     M.x = C.x;
     M.r64 = C.r64;
@@ -3850,7 +3940,16 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
     M.e32 = C.e32;
     M.q = q_ + 4 * c;
     M.isc = inner_.scal_dev() + c;
-    t[c] = tiles_of(C.g, kc);
+    A.kc = krylov_depth(C.g, kc, A.vec ? g_axd_grid : g_axs64_grid);
+    t[c] = tiles_of(C.g, A.kc);
+    tiles += t[c];
+    M.kc = dl;
+    tm[c] = tiles_of(C.g, dl);
+  }
+  e = cudaMalloc((void**)&partial_, (size_t)(tiles * 4 + 64) * sizeof(double));
+  if (e != cudaSuccess) {
+    release();
+    return impact_set_error(e, "mixed engine allocation", __FILE__, __LINE__);
   }
   {
     int nv = 0;
@@ -3858,7 +3957,7 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
     ax_vec_ = nv == 0 ? 0 : (nv == n ? 1 : 2);
   }
   ax_list_ = arena_.add(aj, t);
-  mix_list_ = arena_.add(mj, t);
+  mix_list_ = arena_.add(mj, tm);
   rc = arena_.upload(s);
   if (rc) {
     release();
@@ -3892,7 +3991,7 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
   for (const auto& c : cs_) cells += (double)c.g.n1 * c.g.n2 * c.g.n3;
   const KrylovJob<double>* AJ = static_cast<const KrylovJob<double>*>(AL.jobs);
   const MixJob* MJ = static_cast<const MixJob*>(ML.jobs);
-  const int grid = grid_for(ML.ntiles);
+  const int grid = grid_for(AL.ntiles), gm = grid_for(ML.ntiles);
   auto push_flags = [&]() -> int {
     for (int c = 0; c < n; ++c) {
       osc[c] = SolverScalars{};
@@ -3987,7 +4086,7 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
     }
     rc = push_flags();
     if (rc) return rc;
-    IMPACT_PROF(prof::K_MX_APPLY, 20.0 * cells, s_, (k_mx_apply<<<grid, kBlock, 0, s_>>>(MJ, ML.ts, n, ML.ntiles, oscal_)));
+    IMPACT_PROF(prof::K_MX_APPLY, 20.0 * cells, s_, (k_mx_apply<<<gm, kBlock, 0, s_>>>(MJ, ML.ts, n, ML.ntiles, oscal_)));
   }
   for (int c = 0; c < n; ++c) res[c].iterations = outer_it[c];
   return 0;

@@ -203,7 +203,9 @@ class Engine {
   cudaStream_t s_ = nullptr;
   bool built_ = false;
   ListArena arena_;
-  int kr_list_ = -1;
+  int kr_list_ = -1;           // the operator over the fine grids
+  int kv_list_ = -1;           // the vector updates with partial sums (their own tile depth)
+  int ku_list_ = -1;           // the vector updates without (a depth for the whole list)
   int down0_ = -1, rs1_ = -1;  // finest-level list of the first schedule, restriction to level 2
   int pre0_ = -1, post0_ = -1; // its fused pre- and post-smoothing lists (-1: not fused)
   std::vector<Phase> vc_[2];  // preconditioner schedules: z1 = M pp, z2 = M rr

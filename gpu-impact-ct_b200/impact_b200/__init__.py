@@ -238,7 +238,7 @@ def solver_params(tol_rel=1e-8, tol_abs_inf=0.0, max_it=2000, n_sweeps=4, omega=
                   check_every=4, inner_tol_rel=1e-3, inner_max_it=0, precond=0, mg_down=4, mg_up=4,
                   mg_bottom=4, tile_kc=0, smooth_unfused=0, bottom_cheb=0) -> SolverParams:
     """precond 0: n_sweeps damped-Jacobi sweeps; 1: multigrid V-cycle (mg_down/up/bottom sweeps).
-    tile_kc: z-planes per tile of the solver kernels (0: library default).  smooth_unfused: 1 runs
+    tile_kc: most z-planes per tile of the solver kernels (0: library default; small grids take fewer).  smooth_unfused: 1 runs
     every V-cycle sweep as its own launch instead of one fused kernel per smoothing phase.
     bottom_cheb: d > 0 replaces the coarsest level's Jacobi sweeps by d Chebyshev steps (fused
     schedule, coarsest level within the one-block tail)."""

@@ -276,7 +276,8 @@ typedef struct {
   int precond;         /* 0: n_sweeps damped-Jacobi sweeps; 1: multigrid V-cycle (multigridV,
                           mod_solvers.f90:456-585; needs the coordinates at case creation) */
   int mg_down, mg_up, mg_bottom; /* V-cycle sweeps (n_relax_down / _up / _bottom), relaxation omega */
-  int tile_kc;         /* z-planes per tile of the solver kernels (0: library default); chosen by
+  int tile_kc;         /* most z-planes per tile of the solver kernels (0: library default; a grid
+                          of few tiles takes shallower ones, so that they fill the GPU); chosen by
                           the autotuner of the Python package, no counterpart in the reference */
   int smooth_unfused;  /* 0 (default): the sweeps of each V-cycle smoothing phase (and, before a
                           restriction, the residual after them) run as one z-marching kernel;

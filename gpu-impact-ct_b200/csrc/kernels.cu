@@ -9,6 +9,7 @@
 // by 8).
 #include "kernels.cuh"
 #include "stencil25d.cuh"
+#include "stencil3.cuh"
 
 namespace impact {
 
@@ -24,100 +25,42 @@ static inline dim3 grid3(const Geom& g) {
   const int k = blockIdx.z + 1;                     \
   if (i > g.n1 || j > g.n2) return;
 
-// coordinate / extent / stride of axis a (0,1,2)
-__device__ __forceinline__ int coord(int a, int i, int j, int k) { return a == 0 ? i : (a == 1 ? j : k); }
-__device__ __forceinline__ int extent(const Geom& g, int a) { return a == 0 ? g.n1 : (a == 1 ? g.n2 : g.n3); }
-__device__ __forceinline__ long long stride(const Geom& g, int a) {
-  return a == 0 ? 1LL : (a == 1 ? (long long)g.nx : g.nxy);
-}
-
-// s = sum_{l=LO}^{LO+CNT-1} c(l,row) f(q+l along axis a), in the reference's order.
-template <typename T, int LO, int CNT>
-__device__ __forceinline__ T stencil_axis(const T* __restrict__ c, int row, const T* __restrict__ f,
-                                          long long base, long long st, int q, int n) {
-  const T* cr = c + (long long)row * CNT;
-  T s = cr[0] * __ldg(f + base + (long long)(wrapi(q + LO, n) + 3) * st);
-#pragma unroll
-  for (int l = 1; l < CNT; ++l) s = s + cr[l] * __ldg(f + base + (long long)(wrapi(q + LO + l, n) + 3) * st);
-  return s;
-}
-// same, accumulating into s0 first (divergence for m = 2, 3)
-template <typename T, int LO, int CNT>
-__device__ __forceinline__ T stencil_axis_acc(T s, const T* __restrict__ c, int row,
-                                              const T* __restrict__ f, long long base, long long st,
-                                              int q, int n) {
-  const T* cr = c + (long long)row * CNT;
-#pragma unroll
-  for (int l = 0; l < CNT; ++l) s = s + cr[l] * __ldg(f + base + (long long)(wrapi(q + LO + l, n) + 3) * st);
-  return s;
-}
-// base offset of (i,j,k) with the coordinate along axis a removed (Fortran index -3 there)
-__device__ __forceinline__ long long base_off(const Geom& g, int a, int i, int j, int k) {
-  return off(g, a == 0 ? -3 : i, a == 1 ? -3 : j, a == 2 ? -3 : k);
-}
-
 // ------------------------------------------------------------------------------------
 // gradient (mod_diff.f90:309-414; gradient_kernel.cu): pressure -> velocity point m
 // ------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_gradient(int a, Geom g, const T* __restrict__ cG,
-                                                     const T* __restrict__ phi, T* __restrict__ grad) {
-  POINT_PROLOGUE
-  const int q = coord(a, i, j, k);
-  grad[off(g, i, j, k)] = stencil_axis<T, G_LO, NG>(cG, q, phi, base_off(g, a, i, j, k), stride(g, a), q, extent(g, a));
-}
-template <typename T>
 void launch_gradient(int m, const Geom& g, const T* cG, const T* phi, T* grad, cudaStream_t s) {
-  if (launch_march1<T, G_LO, NG, 0>(m - 1, g, cG, nullptr, phi, nullptr, grad, 0, s)) return;
-  k_gradient<T><<<grid3(g), dim3(BX, BY), 0, s>>>(m - 1, g, cG, phi, grad);
+  launch_march1<T, G_LO, NG, 0>(m - 1, g, cG, nullptr, phi, nullptr, grad, 0, s);
 }
 
 // ------------------------------------------------------------------------------------
 // divergence (mod_diff.f90:52-118; divergence_kernel.cu): m = 1 overwrites, 2,3 accumulate
 // ------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_divergence(int a, Geom g, const T* __restrict__ cD,
-                                                       const T* __restrict__ phi, T* __restrict__ div) {
-  POINT_PROLOGUE
-  const int q = coord(a, i, j, k);
-  const long long p = off(g, i, j, k);
-  if (a == 0)
-    div[p] = stencil_axis<T, D_LO, ND>(cD, q, phi, base_off(g, a, i, j, k), 1, q, g.n1);
-  else
-    div[p] = stencil_axis_acc<T, D_LO, ND>(div[p], cD, q, phi, base_off(g, a, i, j, k), stride(g, a), q, extent(g, a));
-}
-template <typename T>
 void launch_divergence(int m, const Geom& g, const T* cD, const T* phi, T* div, cudaStream_t s) {
-  if (m == 1 ? launch_march1<T, D_LO, ND, 0>(0, g, cD, nullptr, phi, nullptr, div, 0, s)
-             : launch_march1<T, D_LO, ND, 1>(m - 1, g, cD, nullptr, phi, nullptr, div, 0, s))
-    return;
-  k_divergence<T><<<grid3(g), dim3(BX, BY), 0, s>>>(m - 1, g, cD, phi, div);
+  if (m == 1)
+    launch_march1<T, D_LO, ND, 0>(0, g, cD, nullptr, phi, nullptr, div, 0, s);
+  else
+    launch_march1<T, D_LO, ND, 1>(m - 1, g, cD, nullptr, phi, nullptr, div, 0, s);
 }
 
 // ------------------------------------------------------------------------------------
 // divergence2 (mod_diff.f90:130-215; divergence2_kernel.cu): div = D1 u + D2 v + D3 w
 // ------------------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ T div2_point(const Geom& g, const T* __restrict__ cD1, const T* __restrict__ cD2,
-                                        const T* __restrict__ cD3, const T* __restrict__ u,
-                                        const T* __restrict__ v, const T* __restrict__ w, int i, int j, int k) {
-  T s = stencil_axis<T, D_LO, ND>(cD1, i, u, off(g, -3, j, k), 1, i, g.n1);
-  s = stencil_axis_acc<T, D_LO, ND>(s, cD2, j, v, off(g, i, -3, k), g.nx, j, g.n2);
-  s = stencil_axis_acc<T, D_LO, ND>(s, cD3, k, w, off(g, i, j, -3), g.nxy, k, g.n3);
-  return s;
-}
-template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_divergence2(Geom g, const T* __restrict__ cD1, const T* __restrict__ cD2,
-                                                        const T* __restrict__ cD3, const T* __restrict__ u,
-                                                        const T* __restrict__ v, const T* __restrict__ w,
-                                                        T* __restrict__ div) {
-  POINT_PROLOGUE
-  div[off(g, i, j, k)] = div2_point(g, cD1, cD2, cD3, u, v, w, i, j, k);
-}
-template <typename T>
 void launch_divergence2(const Geom& g, const T* cD1, const T* cD2, const T* cD3, const T* u, const T* v,
                         const T* w, T* div, cudaStream_t s) {
-  k_divergence2<T><<<grid3(g), dim3(BX, BY), 0, s>>>(g, cD1, cD2, cD3, u, v, w, div);
+  TriArgs<T, T> a{};
+  a.c[0] = cD1;
+  a.c[1] = cD2;
+  a.c[2] = cD3;
+  a.f[0] = u;
+  a.f[1] = v;
+  a.f[2] = w;
+  a.o[0] = div;
+  a.ahead = tri_ahead(g, sizeof(T));
+  const void* f[4] = {u, v, w, div};
+  launch_tri<TRI_DIV2, T, T>(g, a, tri_grid(g, sizeof(T), tri_vectorable(g, sizeof(T), f, 4)), s);
 }
 
 // ------------------------------------------------------------------------------------
@@ -125,48 +68,32 @@ void launch_divergence2(const Geom& g, const T* cD1, const T* cD2, const T* cD3,
 // nl -= multL * (cx u_xx + cy u_yy + cz u_zz), 7-point second derivatives
 // ------------------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ T lap7_point(const Geom& g, const T* __restrict__ cx, const T* __restrict__ cy,
-                                        const T* __restrict__ cz, const T* __restrict__ vel, int i, int j, int k) {
-  T dd = stencil_axis<T, B_LO, NB>(cx, i, vel, off(g, -3, j, k), 1, i, g.n1);
-  dd = stencil_axis_acc<T, B_LO, NB>(dd, cy, j, vel, off(g, i, -3, k), g.nx, j, g.n2);
-  dd = stencil_axis_acc<T, B_LO, NB>(dd, cz, k, vel, off(g, i, j, -3), g.nxy, k, g.n3);
-  return dd;
-}
-template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_helmholtz(Geom g, const T* __restrict__ cx, const T* __restrict__ cy,
-                                                      const T* __restrict__ cz, T multL, const T* __restrict__ vel,
-                                                      T* __restrict__ nl) {
-  POINT_PROLOGUE
-  const long long p = off(g, i, j, k);
-  nl[p] = nl[p] - multL * lap7_point(g, cx, cy, cz, vel, i, j, k);
-}
-template <typename T>
 void launch_helmholtz(int m, const Geom& g, const T* cx, const T* cy, const T* cz, T multL, const T* vel, T* nl,
                       cudaStream_t s) {
   (void)m;
-  if (launch_helm_march<T>(g, cx, cy, cz, multL, vel, nl, s)) return;
-  k_helmholtz<T><<<grid3(g), dim3(BX, BY), 0, s>>>(g, cx, cy, cz, multL, vel, nl);
+  TriArgs<T, T> a{};
+  a.c[0] = cx;
+  a.c[1] = cy;
+  a.c[2] = cz;
+  a.f[0] = vel;
+  a.s[0] = nl;
+  a.o[0] = nl;
+  a.alpha = multL;
+  a.ahead = tri_ahead(g, sizeof(T));
+  const void* f[2] = {vel, nl};
+  launch_tri<TRI_HELM, T, T>(g, a, tri_grid(g, sizeof(T), tri_vectorable(g, sizeof(T), f, 2)), s);
 }
 
 // ------------------------------------------------------------------------------------
 // interpolations (mod_diff.f90:1567-1648 and :1740-1825; interpolate2_*_kernel.cu)
 // ------------------------------------------------------------------------------------
-template <typename T, int LO, int CNT>
-__global__ void __launch_bounds__(BX* BY) k_interp(int a, Geom g, const T* __restrict__ cI, const T* __restrict__ phi,
-                                                   T* __restrict__ out) {
-  POINT_PROLOGUE
-  const int q = coord(a, i, j, k);
-  out[off(g, i, j, k)] = stencil_axis<T, LO, CNT>(cI, q, phi, base_off(g, a, i, j, k), stride(g, a), q, extent(g, a));
-}
 template <typename T>
 void launch_interp_pre_vel(int m, const Geom& g, const T* cI, const T* phi, T* out, cudaStream_t s) {
-  if (launch_march1<T, G_LO, NG, 0>(m - 1, g, cI, nullptr, phi, nullptr, out, 0, s)) return;
-  k_interp<T, G_LO, NG><<<grid3(g), dim3(BX, BY), 0, s>>>(m - 1, g, cI, phi, out);
+  launch_march1<T, G_LO, NG, 0>(m - 1, g, cI, nullptr, phi, nullptr, out, 0, s);
 }
 template <typename T>
 void launch_interp_vel_pre(int m, const Geom& g, const T* cI, const T* phi, T* out, cudaStream_t s) {
-  if (launch_march1<T, D_LO, ND, 0>(m - 1, g, cI, nullptr, phi, nullptr, out, 0, s)) return;
-  k_interp<T, D_LO, ND><<<grid3(g), dim3(BX, BY), 0, s>>>(m - 1, g, cI, phi, out);
+  launch_march1<T, D_LO, ND, 0>(m - 1, g, cI, nullptr, phi, nullptr, out, 0, s);
 }
 
 // ------------------------------------------------------------------------------------
@@ -174,38 +101,10 @@ void launch_interp_vel_pre(int m, const Geom& g, const T* cI, const T* phi, T* o
 // component_id = 3(m-1) + a; the first axis of a component overwrites nl
 // ------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_nl_upwind(int a, int first, Geom g, const T* __restrict__ cU,
-                                                      const T* __restrict__ cDn, const T* __restrict__ pp,
-                                                      const T* __restrict__ vel, T* __restrict__ nl) {
-  POINT_PROLOGUE
-  const long long p = off(g, i, j, k);
-  const int q = coord(a, i, j, k);
-  const T ppv = pp[p];
-  const T* tab = (ppv >= T(0)) ? cU : cDn;
-  const T dd = stencil_axis<T, B_LO, NB>(tab, q, vel, base_off(g, a, i, j, k), stride(g, a), q, extent(g, a));
-  nl[p] = first ? dd * ppv : nl[p] + dd * ppv;
-}
-template <typename T>
 void launch_nonlinear_upwind(int cid, const Geom& g, const T* cU, const T* cDn, const T* pp, const T* vel, T* nl,
                              cudaStream_t s) {
   const int a = (cid - 1) % 3;
-  if (launch_march1<T, B_LO, NB, 2>(a, g, cU, cDn, vel, pp, nl, a == 0, s)) return;
-  k_nl_upwind<T><<<grid3(g), dim3(BX, BY), 0, s>>>(a, a == 0, g, cU, cDn, pp, vel, nl);
-}
-
-// ------------------------------------------------------------------------------------
-// axpby (axpby_kernel.cu:6-17)
-// ------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_axpby(Geom g, T a, T b, const T* __restrict__ x, const T* __restrict__ y,
-                                                  T* __restrict__ z) {
-  POINT_PROLOGUE
-  const long long p = off(g, i, j, k);
-  z[p] = a * x[p] + b * y[p];
-}
-template <typename T>
-void launch_axpby(const Geom& g, T a, T b, const T* x, const T* y, T* z, cudaStream_t s) {
-  k_axpby<T><<<grid3(g), dim3(BX, BY), 0, s>>>(g, a, b, x, y, z);
+  launch_march1<T, B_LO, NB, 2>(a, g, cU, cDn, vel, pp, nl, a == 0, s);
 }
 
 // ------------------------------------------------------------------------------------
@@ -254,22 +153,6 @@ __device__ __forceinline__ T jacobi_point(const Geom& g, const T* a, const T* b,
   return omega * (bb - a[0] * n.xm - a[2] * n.xp - b[0] * n.ym - b[2] * n.yp - c[0] * n.zm - c[2] * n.zp) /
              (a[1] + b[1] + c[1]) +
          (T(1) - omega) * n.c;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(BX* BY) k_jacobi(Geom g, const T* __restrict__ c1, const T* __restrict__ c2,
-                                                   const T* __restrict__ c3, T omega, const T* __restrict__ bb,
-                                                   const T* __restrict__ rel, T* __restrict__ out) {
-  POINT_PROLOGUE
-  const long long p = off(g, i, j, k);
-  const Nb7<T> n = load_nb7(g, rel, i, j, k);
-  out[p] = jacobi_point(g, c1 + 3 * (i - 1), c2 + 3 * (j - 1), c3 + 3 * (k - 1), omega, __ldg(bb + p), n);
-}
-template <typename T>
-void launch_jacobi(const Geom& g, const T* c1, const T* c2, const T* c3, T omega, const T* bb, const T* rel, T* out,
-                   cudaStream_t s) {
-  if (launch_jacobi_march<T>(g, c1, c2, c3, omega, bb, rel, out, s)) return;
-  k_jacobi<T><<<grid3(g), dim3(BX, BY), 0, s>>>(g, c1, c2, c3, omega, bb, rel, out);
 }
 
 // init sweep: rel = omega*bb/diag (mod_laplace.f90:~470, r == 1 .AND. init_yes)
@@ -569,10 +452,7 @@ void launch_finalize(const double* partial, int nq, const int* kinds_host, doubl
   template void launch_interp_vel_pre<T>(int, const Geom&, const T*, const T*, T*, cudaStream_t);            \
   template void launch_nonlinear_upwind<T>(int, const Geom&, const T*, const T*, const T*, const T*, T*,      \
                                            cudaStream_t);                                                     \
-  template void launch_axpby<T>(const Geom&, T, T, const T*, const T*, T*, cudaStream_t);                     \
   template void launch_dg_relax<T>(const Geom&, const T*, const T*, const T*, const T*, T*, cudaStream_t);    \
-  template void launch_jacobi<T>(const Geom&, const T*, const T*, const T*, T, const T*, const T*, T*,        \
-                                 cudaStream_t);                                                               \
   template void launch_jacobi_init2<T>(const Geom&, const T*, const T*, const T*, T, const T*, T*,            \
                                        cudaStream_t);                                                         \
   template void launch_jacobi_init1<T>(const Geom&, const T*, const T*, const T*, T, const T*, T*,            \

@@ -1,20 +1,28 @@
-// march.cu -- the one-axis stencil operators of the launcher FFI as streaming passes.
+// march.cu -- the one-axis stencil operators of the launcher FFI, the JOR sweep and axpby as
+// streaming passes.
 //
 // gradient (mod_diff.f90:309-414), divergence per axis (:52-118), both interpolations
 // (:1567-1648, :1740-1825) and the upwind advection term (:784-1424) are 6- or 7-point stencils
 // along one axis a: out(q) = sum_{l} c(l, q) f(q + LO + l), q the coordinate along a, with the
-// row of coefficients c(., q) of that coordinate.  Here every thread owns one 16-byte vector of
-// x points (2 doubles or 4 floats; rows are 16-byte aligned when n1 is divisible by the vector
-// width) and:
-//   a = y or z: marches along a over a segment of the axis, keeping the CNT vectors of its
-//               stencil in registers (one new 16-byte load and one 16-byte store per step), the
-//               coefficient row of the step being the same for the whole block;
-//   a = x:      marches z as well, with the coefficient rows of its points loaded once; each
-//               plane takes the few aligned vectors of the row that its points' stencils span
-//               (neighbouring vectors, periodic images at the row ends).
-// Periodic wrapping is applied to the coordinate along a only.  Each point sums its terms in
-// table order with the same fused multiply-adds as the one-point-per-thread kernels of
-// kernels.cu, so both give the same bits.
+// row of coefficients c(., q) of that coordinate.  A thread owns one vector of V x points (V = 16
+// bytes where the rows hold whole aligned vectors, else V = 1) and walks a segment in blocks of U
+// steps, all loads of a block issued before its stores:
+//   a = y or z: marches along a, the stencil's values in registers, one new vector per step; the
+//               coefficient row of a step is the same for the whole block;
+//   a = x:      marches z with the coefficient rows of its points loaded once; each plane takes the
+//               aligned vectors of the row that its points' stencils span (V = 1: its taps).
+// Threads are numbered along the vectors of a row and then along the rows, so that narrow grids
+// fill their warps, and a segment is as short as 4 steps where a small grid would otherwise leave
+// SMs idle.  Periodic wrapping is applied to the coordinate along a only; each point sums its
+// terms in table order with fused multiply-adds.
+//
+// Bound by DRAM on large grids and by latency on small ones.  256 x 256 x 512 FP64 (270 MB a
+// field, 6.5 TB/s copy bandwidth): the y and z interpolations 96 us (5.6 TB/s; 118 - 125 us with one
+// step's loads at a time and segments of 64), along x 127 us, the upwind terms 244 / 196 us (234 /
+// 252), axpby 126 us (146).  Segments beyond 16 steps lost 8 % on every pass there.  187 x 131 x 157
+// FP32, rows of odd length: 12.6 us (one point per thread with its taps wrapped one by one: 25), the
+// upwind terms 19 - 21 us (29).  64 x 64 x 128 FP64: JOR sweep 6.4 us (10.8), interpolations 5.2 us
+// (8.4).
 #include "kernels.cuh"
 
 namespace impact {
@@ -90,74 +98,102 @@ __device__ __forceinline__ T point_value(const T* __restrict__ ca, const T* __re
   return s;
 }
 
-constexpr int MBX = 32, MBY = 8;
+constexpr int MT = 256;  // threads per block
 
-// a = 1 (y) or 2 (z): thread (vector vx, other in-plane coordinate o) marches q = q0 .. q1
-template <typename T, int LO, int CNT, int OP>
-__global__ void __launch_bounds__(MBX* MBY) k_march_yz(int a, Geom g, const T* __restrict__ cA, const T* __restrict__ cB,
-                                                       const T* __restrict__ f, const T* __restrict__ pp,
-                                                       T* __restrict__ out, int first, int seg) {
-  constexpr int W = V16<T>::W;
-  const int i = 1 + W * (blockIdx.x * MBX + threadIdx.x);
-  const int o = blockIdx.y * MBY + threadIdx.y + 1;
+template <typename T, int V>
+__device__ __forceinline__ void ldv(const T* p, T (&o)[V]) {
+  if constexpr (V == 1)
+    o[0] = __ldg(p);
+  else
+    vld(p, o);
+}
+template <typename T, int V>
+__device__ __forceinline__ void ldv_plain(const T* p, T (&o)[V]) {  // may alias the output
+  if constexpr (V == 1)
+    o[0] = p[0];
+  else
+    vld_plain(p, o);
+}
+template <typename T, int V>
+__device__ __forceinline__ void stv(T* p, const T (&o)[V]) {
+  if constexpr (V == 1)
+    p[0] = o[0];
+  else
+    vst(p, o);
+}
+// a = 1 (y) or 2 (z): thread (vector, other in-plane coordinate o) marches q = q0 .. q1
+template <typename T, int V, int LO, int CNT, int OP>
+__global__ void __launch_bounds__(MT) k_march_yz(int a, Geom g, const T* __restrict__ cA, const T* __restrict__ cB,
+                                                 const T* __restrict__ f, const T* __restrict__ pp,
+                                                 T* __restrict__ out, int first, int seg) {
+  constexpr int U = 4, NW = CNT - 1 + U;
+  const int nvx = g.n1 / V;
+  const unsigned idx = blockIdx.x * MT + threadIdx.x;
+  const int o = (int)(idx / (unsigned)nvx) + 1;
+  const int i = 1 + V * (int)(idx % (unsigned)nvx);
   const int na = a == 2 ? g.n3 : g.n2, no = a == 2 ? g.n2 : g.n3;
-  if (i > g.n1 || o > no) return;
+  if (o > no) return;
   const long long sa = a == 2 ? g.nxy : (long long)g.nx;
   const long long so = a == 2 ? (long long)g.nx : g.nxy;
   const long long base = (i + 3) + so * (o + 3) + sa * 3;  // (i, o, q = 0)
-  const int q0 = blockIdx.z * seg + 1, q1 = min(na, q0 + seg - 1);
-  T win[CNT][W];
+  const int q0 = blockIdx.y * seg + 1, q1 = min(na, q0 + seg - 1);
+  T win[NW][V];
 #pragma unroll
-  for (int l = 0; l < CNT; ++l) vld(f + base + sa * wrapi(q0 + LO + l, na), win[l]);
-  for (int q = q0; q <= q1; ++q) {
-    const long long p = base + sa * q;
-    T old[W], pv[W], r[W];
-    if (OP != 0) vld_plain(out + p, old);
-    if (OP == 2) vld(pp + p, pv);
-    const T* ca = cA + (long long)q * CNT;
-    const T* cb = OP == 2 ? cB + (long long)q * CNT : ca;
-    T ca_r[CNT], cb_r[CNT];
+  for (int l = 0; l < CNT - 1; ++l) ldv<T, V>(f + base + sa * wrapi(q0 + LO + l, na), win[l]);
+  for (int q = q0; q <= q1; q += U) {
+    T old[U][V], pv[U][V];
 #pragma unroll
-    for (int l = 0; l < CNT; ++l) {
-      ca_r[l] = __ldg(ca + l);
-      cb_r[l] = OP == 2 ? __ldg(cb + l) : ca_r[l];
-    }
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || q + u <= q1) {
+        ldv<T, V>(f + base + sa * wrapi(q + u + LO + CNT - 1, na), win[CNT - 1 + u]);
+        const long long p = base + sa * (q + u);
+        if (OP != 0) ldv_plain<T, V>(out + p, old[u]);
+        if (OP == 2) ldv<T, V>(pp + p, pv[u]);
+      }
 #pragma unroll
-    for (int v = 0; v < W; ++v) {
-      T wv[CNT];
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || q + u <= q1) {
+        T ca[CNT], cb[CNT], r[V];
 #pragma unroll
-      for (int l = 0; l < CNT; ++l) wv[l] = win[l][v];
-      r[v] = point_value<T, CNT, OP>(ca_r, cb_r, wv, OP != 0 ? old[v] : T(0), OP == 2 ? pv[v] : T(0), first);
-    }
-    vst(out + p, r);
+        for (int l = 0; l < CNT; ++l) {
+          ca[l] = __ldg(cA + (long long)(q + u) * CNT + l);
+          cb[l] = OP == 2 ? __ldg(cB + (long long)(q + u) * CNT + l) : ca[l];
+        }
 #pragma unroll
-    for (int l = 0; l + 1 < CNT; ++l)
+        for (int v = 0; v < V; ++v) {
+          T wv[CNT];
 #pragma unroll
-      for (int v = 0; v < W; ++v) win[l][v] = win[l + 1][v];
-    if (q < q1) vld(f + base + sa * wrapi(q + 1 + LO + CNT - 1, na), win[CNT - 1]);
+          for (int l = 0; l < CNT; ++l) wv[l] = win[u + l][v];
+          r[v] = point_value<T, CNT, OP>(ca, cb, wv, OP != 0 ? old[u][v] : T(0), OP == 2 ? pv[u][v] : T(0), first);
+        }
+        stv<T, V>(out + base + sa * (q + u), r);
+      }
+#pragma unroll
+    for (int l = 0; l < CNT - 1; ++l)
+#pragma unroll
+      for (int v = 0; v < V; ++v) win[l][v] = win[l + U][v];
   }
 }
 
-// a = 0 (x): thread (vector, row j) marches z over a segment; the coefficient rows of its W
-// points are loaded once, and each plane takes the few aligned vectors of the row that the W
-// points' stencils span (neighbouring vectors, periodic images at the row ends)
-template <typename T, int LO, int CNT, int OP>
-__global__ void __launch_bounds__(MBX* MBY) k_march_x(Geom g, const T* __restrict__ cA, const T* __restrict__ cB,
-                                                      const T* __restrict__ f, const T* __restrict__ pp,
-                                                      T* __restrict__ out, int first, int seg) {
-  constexpr int W = V16<T>::W;
-  constexpr int FV = (LO - (W - 1)) / W;          // floor(LO / W) for LO < 0
-  constexpr int LV = (W - 1 + LO + CNT - 1) / W;  // floor of the last position / W (>= 0)
+// a = 0 (x): thread (vector, row j) marches z
+template <typename T, int V, int LO, int CNT, int OP>
+__global__ void __launch_bounds__(MT, V == 1 ? (OP == 2 ? 4 : 2) : (OP == 2 ? 2 : 4)) k_march_x(Geom g, const T* __restrict__ cA, const T* __restrict__ cB,
+                                                const T* __restrict__ f, const T* __restrict__ pp,
+                                                T* __restrict__ out, int first, int seg) {
+  constexpr int U = OP == 2 ? 1 : (sizeof(T) == 8 && V > 1 ? 2 : 4);
+  constexpr int FV = (LO - (V - 1)) / V;          // floor(LO / V) for LO < 0
+  constexpr int LV = (V - 1 + LO + CNT - 1) / V;  // floor of the last position / V (>= 0)
   constexpr int NV = LV - FV + 1;
-  const int vx = blockIdx.x * MBX + threadIdx.x;
-  const int nvx = g.n1 / W;
-  const int j = blockIdx.y * MBY + threadIdx.y + 1;
-  if (vx >= nvx || j > g.n2) return;
-  const int i = 1 + W * vx;
-  const int k0 = blockIdx.z * seg + 1, k1 = min(g.n3, k0 + seg - 1);
-  T ca[W][CNT], cb[W][CNT];
+  const int nvx = g.n1 / V;
+  const unsigned idx = blockIdx.x * MT + threadIdx.x;
+  const int j = (int)(idx / (unsigned)nvx) + 1;
+  const int vx = (int)(idx % (unsigned)nvx);
+  if (j > g.n2) return;
+  const int i = 1 + V * vx;
+  const int k0 = blockIdx.y * seg + 1, k1 = min(g.n3, k0 + seg - 1);
+  T ca[V][CNT], cb[V][CNT];
 #pragma unroll
-  for (int v = 0; v < W; ++v)
+  for (int v = 0; v < V; ++v)
 #pragma unroll
     for (int l = 0; l < CNT; ++l) {
       ca[v][l] = __ldg(cA + (long long)(i + v) * CNT + l);
@@ -167,239 +203,221 @@ __global__ void __launch_bounds__(MBX* MBY) k_march_x(Geom g, const T* __restric
 #pragma unroll
   for (int n = 0; n < NV; ++n) {
     const int u = vx + FV + n;
-    us[n] = W * (u < 0 ? u + nvx : (u >= nvx ? u - nvx : u));
+    us[n] = V * (u < 0 ? u + nvx : (u >= nvx ? u - nvx : u));
   }
   const long long rowj = 4 + (long long)g.nx * (j + 3);  // offset of (1, j, k = -3)
-  for (int k = k0; k <= k1; ++k) {
-    const long long row = rowj + g.nxy * (k + 3);
-    T val[NV * W];
+  for (int k = k0; k <= k1; k += U) {
+    T val[U][NV * V], old[U][V], pv[U][V];
 #pragma unroll
-    for (int n = 0; n < NV; ++n) {
-      T tmp[W];
-      vld(f + row + us[n], tmp);
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || k + u <= k1) {
+        const long long row = rowj + g.nxy * (k + u + 3);
 #pragma unroll
-      for (int v = 0; v < W; ++v) val[n * W + v] = tmp[v];
-    }
-    const long long p = row + (i - 1);
-    T old[W], pv[W], r[W];
-    if (OP != 0) vld_plain(out + p, old);
-    if (OP == 2) vld(pp + p, pv);
+        for (int n = 0; n < NV; ++n) {
+          T tmp[V];
+          ldv<T, V>(f + row + us[n], tmp);
 #pragma unroll
-    for (int v = 0; v < W; ++v) {
-      T wv[CNT];
-#pragma unroll
-      for (int l = 0; l < CNT; ++l) wv[l] = val[v + LO + l - FV * W];
-      r[v] = point_value<T, CNT, OP>(ca[v], cb[v], wv, OP != 0 ? old[v] : T(0), OP == 2 ? pv[v] : T(0), first);
-    }
-    vst(out + p, r);
-  }
-}
-
-// Helmholtz_explicit (mod_diff.f90:549-762): nl = nl - multL (cx u_xx + cy u_yy + cz u_zz), the
-// three 7-point second derivatives summed in one chain x, then y, then z (as lap7_point in
-// kernels.cu).  Thread (vector, row j) marches z over a segment: the column's z values k-3..k+3
-// in registers, x neighbours from the aligned vectors of the row, y neighbours from the vectors
-// of rows j-3..j+3 (shared with the block's other rows through L1).
-template <typename T>
-__global__ void __launch_bounds__(MBX* MBY) k_helm_march(Geom g, const T* __restrict__ cx, const T* __restrict__ cy,
-                                                         const T* __restrict__ cz, T multL, const T* __restrict__ vel,
-                                                         T* __restrict__ nl, int seg) {
-  constexpr int W = V16<T>::W;
-  constexpr int FV = (B_LO - (W - 1)) / W, LV = (W - 1 + B_LO + NB - 1) / W, NV = LV - FV + 1;
-  const int vx = blockIdx.x * MBX + threadIdx.x;
-  const int nvx = g.n1 / W;
-  const int j = blockIdx.y * MBY + threadIdx.y + 1;
-  if (vx >= nvx || j > g.n2) return;
-  const int i = 1 + W * vx;
-  const int k0 = blockIdx.z * seg + 1, k1 = min(g.n3, k0 + seg - 1);
-  const long long rowj = 4 + (long long)g.nx * (j + 3);  // (1, j, k = -3)
-  long long rows[NB];                                     // (1, j-3+l, k = -3)
-#pragma unroll
-  for (int l = 0; l < NB; ++l) rows[l] = 4 + (long long)g.nx * (wrapi(j + B_LO + l, g.n2) + 3);
-  int us[NV];
-#pragma unroll
-  for (int n = 0; n < NV; ++n) {
-    const int u = vx + FV + n;
-    us[n] = W * (u < 0 ? u + nvx : (u >= nvx ? u - nvx : u));
-  }
-  T zc[NB][W];  // z window of the column: k-3 .. k+3
-#pragma unroll
-  for (int l = 0; l < NB; ++l) vld(vel + rowj + (long long)g.nxy * (wrapi(k0 + B_LO + l, g.n3) + 3) + (i - 1), zc[l]);
-  T ycr[NB];
-#pragma unroll
-  for (int l = 0; l < NB; ++l) ycr[l] = __ldg(cy + (long long)j * NB + l);
-  for (int k = k0; k <= k1; ++k) {
-    const long long pz = g.nxy * (k + 3);
-    T xv[NV * W];
-#pragma unroll
-    for (int n = 0; n < NV; ++n) {
-      T tmp[W];
-      vld(vel + rowj + pz + us[n], tmp);
-#pragma unroll
-      for (int v = 0; v < W; ++v) xv[n * W + v] = tmp[v];
-    }
-    T yv[NB][W];
-#pragma unroll
-    for (int l = 0; l < NB; ++l) {
-      if (l == -B_LO) {
-#pragma unroll
-        for (int v = 0; v < W; ++v) yv[l][v] = zc[-B_LO][v];
-      } else {
-        vld(vel + rows[l] + pz + (i - 1), yv[l]);
+          for (int v = 0; v < V; ++v) val[u][n * V + v] = tmp[v];
+        }
+        const long long p = row + (i - 1);
+        if (OP != 0) ldv_plain<T, V>(out + p, old[u]);
+        if (OP == 2) ldv<T, V>(pp + p, pv[u]);
       }
-    }
-    T zcr[NB];
 #pragma unroll
-    for (int l = 0; l < NB; ++l) zcr[l] = __ldg(cz + (long long)k * NB + l);
-    const long long p = rowj + pz + (i - 1);
-    T old[W], r[W];
-    vld_plain(nl + p, old);
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || k + u <= k1) {
+        T r[V];
 #pragma unroll
-    for (int v = 0; v < W; ++v) {
-      const T* xr = cx + (long long)(i + v) * NB;
-      T d = mulT(__ldg(xr), xv[v + B_LO - FV * W]);
+        for (int v = 0; v < V; ++v) {
+          T wv[CNT];
 #pragma unroll
-      for (int l = 1; l < NB; ++l) d = fmaT(__ldg(xr + l), xv[v + B_LO + l - FV * W], d);
-#pragma unroll
-      for (int l = 0; l < NB; ++l) d = fmaT(ycr[l], yv[l][v], d);
-#pragma unroll
-      for (int l = 0; l < NB; ++l) d = fmaT(zcr[l], zc[l][v], d);
-      r[v] = fmaT(-multL, d, old[v]);
-    }
-    vst(nl + p, r);
-#pragma unroll
-    for (int l = 0; l + 1 < NB; ++l)
-#pragma unroll
-      for (int v = 0; v < W; ++v) zc[l][v] = zc[l + 1][v];
-    if (k < k1) vld(vel + rowj + (long long)g.nxy * (wrapi(k + 1 - B_LO, g.n3) + 3) + (i - 1), zc[NB - 1]);
+          for (int l = 0; l < CNT; ++l) wv[l] = val[u][v + LO + l - FV * V];
+          r[v] = point_value<T, CNT, OP>(ca[v], cb[v], wv, OP != 0 ? old[u][v] : T(0), OP == 2 ? pv[u][v] : T(0), first);
+        }
+        stv<T, V>(out + rowj + g.nxy * (k + u + 3) + (i - 1), r);
+      }
   }
 }
 
 // relaxation_div_grad / the JOR sweep (mod_laplace.f90:339-613, jacobi_kernel.cu):
-// out = omega (bb - sum of the six off-diagonal terms of cdg) / diag + (1 - omega) rel, as
-// jacobi_point in kernels.cu.  Thread (vector, row j) marches z with the column's rel at k-1..k+1
-// in registers.
-template <typename T>
-__global__ void __launch_bounds__(MBX* MBY) k_jacobi_march(Geom g, const T* __restrict__ c1, const T* __restrict__ c2,
-                                                           const T* __restrict__ c3, T omega, const T* __restrict__ bb,
-                                                           const T* __restrict__ rel, T* __restrict__ out, int seg) {
-  constexpr int W = V16<T>::W;
-  const int vx = blockIdx.x * MBX + threadIdx.x;
-  const int nvx = g.n1 / W;
-  const int j = blockIdx.y * MBY + threadIdx.y + 1;
-  if (vx >= nvx || j > g.n2) return;
-  const int i = 1 + W * vx;
-  const int k0 = blockIdx.z * seg + 1, k1 = min(g.n3, k0 + seg - 1);
-  const long long rowj = 4 + (long long)g.nx * (j + 3);
-  const long long rowm = 4 + (long long)g.nx * (wrapi(j - 1, g.n2) + 3), rowp = 4 + (long long)g.nx * (wrapi(j + 1, g.n2) + 3);
-  const int um = W * (vx == 0 ? nvx - 1 : vx - 1), up = W * (vx == nvx - 1 ? 0 : vx + 1);
-  T zc[3][W];
+// out = omega (bb - sum of the six off-diagonal terms of cdg) / diag + (1 - omega) rel.  Thread
+// (vector, row j) marches z with the column's rel at k-1..k+1 in registers.
+template <typename T, int V>
+__global__ void __launch_bounds__(MT) k_jacobi_march(Geom g, const T* __restrict__ c1, const T* __restrict__ c2,
+                                                     const T* __restrict__ c3, T omega, const T* __restrict__ bb,
+                                                     const T* __restrict__ rel, T* __restrict__ out, int seg) {
+  constexpr int U = 2;
+  const int nvx = g.n1 / V;
+  const unsigned idx = blockIdx.x * MT + threadIdx.x;
+  const int j = (int)(idx / (unsigned)nvx) + 1;
+  const int i = 1 + V * (int)(idx % (unsigned)nvx);
+  if (j > g.n2) return;
+  const int k0 = blockIdx.y * seg + 1, k1 = min(g.n3, k0 + seg - 1);
+  const long long row = (i + 3) + (long long)g.nx * (j + 3);  // (i, j, k = -3)
+  const int dW = i == 1 ? g.n1 - 1 : -1, dE = i + V - 1 == g.n1 ? 1 - i : V;
+  const int dS = (wrapi(j - 1, g.n2) - j) * g.nx, dN = (wrapi(j + 1, g.n2) - j) * g.nx;
+  T a0[V], a1[V], a2[V];
 #pragma unroll
-  for (int l = 0; l < 3; ++l) vld(rel + rowj + (long long)g.nxy * (wrapi(k0 - 1 + l, g.n3) + 3) + (i - 1), zc[l]);
+  for (int v = 0; v < V; ++v) {
+    const T* a = c1 + 3 * (i + v - 1);
+    a0[v] = __ldg(a);
+    a1[v] = __ldg(a + 1);
+    a2[v] = __ldg(a + 2);
+  }
   const T b0 = __ldg(c2 + 3 * (j - 1)), b1 = __ldg(c2 + 3 * (j - 1) + 1), b2 = __ldg(c2 + 3 * (j - 1) + 2);
-  for (int k = k0; k <= k1; ++k) {
-    const long long pz = g.nxy * (k + 3);
-    const long long p = rowj + pz + (i - 1);
-    T lm[W], rp[W], ym[W], yp[W], bv[W], r[W];
-    vld(rel + rowj + pz + um, lm);
-    vld(rel + rowj + pz + up, rp);
-    vld(rel + rowm + pz + (i - 1), ym);
-    vld(rel + rowp + pz + (i - 1), yp);
-    vld(bb + p, bv);
-    const T e0 = __ldg(c3 + 3 * (k - 1)), e1 = __ldg(c3 + 3 * (k - 1) + 1), e2 = __ldg(c3 + 3 * (k - 1) + 2);
+  T zc[2 + U][V];
+  ldv<T, V>(rel + row + (long long)g.nxy * (wrapi(k0 - 1, g.n3) + 3), zc[0]);
+  ldv<T, V>(rel + row + (long long)g.nxy * (k0 + 3), zc[1]);
+  for (int k = k0; k <= k1; k += U) {
+    T w[U], e[U], ym[U][V], yp[U][V], bv[U][V];
 #pragma unroll
-    for (int v = 0; v < W; ++v) {
-      const T* a = c1 + 3 * (i + v - 1);
-      const T a0 = __ldg(a), a1 = __ldg(a + 1), a2 = __ldg(a + 2);
-      const T xm = v == 0 ? lm[W - 1] : zc[1][v - 1];
-      const T xp = v == W - 1 ? rp[0] : zc[1][v + 1];
-      r[v] = omega * (bv[v] - a0 * xm - a2 * xp - b0 * ym[v] - b2 * yp[v] - e0 * zc[0][v] - e2 * zc[2][v]) /
-                 (a1 + b1 + e1) +
-             (T(1) - omega) * zc[1][v];
-    }
-    vst(out + p, r);
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || k + u <= k1) {
+        const long long p = row + (long long)g.nxy * (k + u + 3);
+        ldv<T, V>(rel + row + (long long)g.nxy * (wrapi(k + u + 1, g.n3) + 3), zc[2 + u]);
+        w[u] = __ldg(rel + p + dW);
+        e[u] = __ldg(rel + p + dE);
+        ldv<T, V>(rel + p + dS, ym[u]);
+        ldv<T, V>(rel + p + dN, yp[u]);
+        ldv<T, V>(bb + p, bv[u]);
+      }
 #pragma unroll
-    for (int v = 0; v < W; ++v) {
-      zc[0][v] = zc[1][v];
-      zc[1][v] = zc[2][v];
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || k + u <= k1) {
+        const T e0 = __ldg(c3 + 3 * (k + u - 1)), e1 = __ldg(c3 + 3 * (k + u - 1) + 1), e2 = __ldg(c3 + 3 * (k + u - 1) + 2);
+        T r[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const T xm = v == 0 ? w[u] : zc[1 + u][v == 0 ? 0 : v - 1];
+          const T xp = v == V - 1 ? e[u] : zc[1 + u][v == V - 1 ? v : v + 1];
+          r[v] = omega * (bv[u][v] - a0[v] * xm - a2[v] * xp - b0 * ym[u][v] - b2 * yp[u][v] - e0 * zc[u][v] -
+                          e2 * zc[2 + u][v]) /
+                     (a1[v] + b1 + e1) +
+                 (T(1) - omega) * zc[1 + u][v];
+        }
+        stv<T, V>(out + row + (long long)g.nxy * (k + u + 3), r);
+      }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      zc[0][v] = zc[U][v];
+      zc[1][v] = zc[U + 1][v];
     }
-    if (k < k1) vld(rel + rowj + (long long)g.nxy * (wrapi(k + 2, g.n3) + 3) + (i - 1), zc[2]);
+  }
+}
+
+// z = a x + b y (axpby_kernel.cu:6-17)
+template <typename T, int V>
+__global__ void __launch_bounds__(MT) k_axpby(Geom g, T a, T b, const T* __restrict__ x, const T* __restrict__ y,
+                                              T* __restrict__ z, int seg) {
+  constexpr int U = 4;
+  const int nvx = g.n1 / V;
+  const unsigned idx = blockIdx.x * MT + threadIdx.x;
+  const int j = (int)(idx / (unsigned)nvx) + 1;
+  const int i = 1 + V * (int)(idx % (unsigned)nvx);
+  if (j > g.n2) return;
+  const int k0 = blockIdx.y * seg + 1, k1 = min(g.n3, k0 + seg - 1);
+  long long p = off(g, i, j, k0);
+  for (int k = k0; k <= k1; k += U, p += U * g.nxy) {
+    T xv[U][V], yv[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || k + u <= k1) {
+        ldv<T, V>(x + p + u * g.nxy, xv[u]);
+        ldv<T, V>(y + p + u * g.nxy, yv[u]);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u == 0 || k + u <= k1) {
+        T r[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) r[v] = a * xv[u][v] + b * yv[u][v];
+        stv<T, V>(z + p + u * g.nxy, r);
+      }
   }
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// planes per marching thread: enough blocks for several waves, 16 .. 64 points per thread
-inline int march_seg(long long blocks_xy, int na) {
-  long long seg = blocks_xy * na / (148LL * 8);
-  seg = seg < 16 ? 16 : (seg > 64 ? 64 : seg);
+// steps per marching thread, 4 .. 16 in whole blocks of 4: as many as leave about `per_sm` threads
+// per SM (a segment re-reads the CNT - 1 values before it, mostly from L2, and pays its set-up
+// once).  Along x the set-up loads the coefficient rows of the thread's points, strided over the
+// warp, which for whole vectors costs as much as some ten planes: at least 8 steps there (16 with
+// the upwind term's two tables in FP32), and half the threads.
+inline int march_seg(long long threads, int na, int per_sm, int least) {
+  long long seg = threads * na / (148LL * per_sm) / 4 * 4;
+  seg = seg < least ? least : (seg > 16 ? 16 : seg);
   return (int)std::min<long long>(seg, na);
+}
+// grid of a pass: threads (vectors of one row x no rows), na steps
+inline dim3 march_grid(const Geom& g, int V, int no, int na, int& seg, int per_sm = 1024, int least = 4) {
+  const long long threads = (long long)(g.n1 / V) * no;
+  seg = march_seg(threads, na, per_sm, least);
+  return dim3((unsigned)((threads + MT - 1) / MT), (na + seg - 1) / seg);
+}
+
+template <typename T, int V, int LO, int CNT, int OP>
+void march1(int a, const Geom& g, const T* cA, const T* cB, const T* f, const T* pp, T* out, int first,
+            cudaStream_t s) {
+  int seg = 0;
+  if (a == 0) {
+    const dim3 grid = V > 1 ? march_grid(g, V, g.n2, g.n3, seg, 512, OP == 2 && V == 4 ? 16 : 8) : march_grid(g, V, g.n2, g.n3, seg);
+    k_march_x<T, V, LO, CNT, OP><<<grid, MT, 0, s>>>(g, cA, cB, f, pp, out, first, seg);
+  } else {
+    const dim3 grid = march_grid(g, V, a == 2 ? g.n2 : g.n3, a == 2 ? g.n3 : g.n2, seg);
+    k_march_yz<T, V, LO, CNT, OP><<<grid, MT, 0, s>>>(a, g, cA, cB, f, pp, out, first, seg);
+  }
 }
 
 }  // namespace
 
 template <typename T, int LO, int CNT, int OP>
-bool launch_march1(int a, const Geom& g, const T* cA, const T* cB, const T* f, const T* pp, T* out, int first,
+void launch_march1(int a, const Geom& g, const T* cA, const T* cB, const T* f, const T* pp, T* out, int first,
                    cudaStream_t s) {
   constexpr int W = V16<T>::W;
-  if (g.n1 % W != 0 || !aligned16(f) || !aligned16(out) || (OP == 2 && !aligned16(pp))) return false;
-  const int nvx = g.n1 / W;
-  if (a == 0) {
-    const long long bx = (nvx + MBX - 1) / MBX, by = (g.n2 + MBY - 1) / MBY;
-    const int seg = march_seg(bx * by, g.n3);
-    const dim3 grid((unsigned)bx, (unsigned)by, (g.n3 + seg - 1) / seg);
-    k_march_x<T, LO, CNT, OP><<<grid, dim3(MBX, MBY), 0, s>>>(g, cA, cB, f, pp, out, first, seg);
+  if (g.n1 % W == 0 && aligned16(f) && aligned16(out) && (OP != 2 || aligned16(pp)))
+    march1<T, W, LO, CNT, OP>(a, g, cA, cB, f, pp, out, first, s);
+  else
+    march1<T, 1, LO, CNT, OP>(a, g, cA, cB, f, pp, out, first, s);
+}
+
+template <typename T>
+void launch_jacobi(const Geom& g, const T* c1, const T* c2, const T* c3, T omega, const T* bb, const T* rel, T* out,
+                   cudaStream_t s) {
+  constexpr int W = V16<T>::W;
+  int seg = 0;
+  if (g.n1 % W == 0 && aligned16(bb) && aligned16(rel) && aligned16(out)) {
+    const dim3 grid = march_grid(g, W, g.n2, g.n3, seg);
+    k_jacobi_march<T, W><<<grid, MT, 0, s>>>(g, c1, c2, c3, omega, bb, rel, out, seg);
   } else {
-    const int na = a == 2 ? g.n3 : g.n2, no = a == 2 ? g.n2 : g.n3;
-    const long long bx = (nvx + MBX - 1) / MBX, by = (no + MBY - 1) / MBY;
-    const int seg = march_seg(bx * by, na);
-    const dim3 grid((unsigned)bx, (unsigned)by, (na + seg - 1) / seg);
-    k_march_yz<T, LO, CNT, OP><<<grid, dim3(MBX, MBY), 0, s>>>(a, g, cA, cB, f, pp, out, first, seg);
+    const dim3 grid = march_grid(g, 1, g.n2, g.n3, seg);
+    k_jacobi_march<T, 1><<<grid, MT, 0, s>>>(g, c1, c2, c3, omega, bb, rel, out, seg);
   }
-  return true;
 }
-
 template <typename T>
-bool launch_helm_march(const Geom& g, const T* cx, const T* cy, const T* cz, T multL, const T* vel, T* nl,
-                       cudaStream_t s) {
+void launch_axpby(const Geom& g, T a, T b, const T* x, const T* y, T* z, cudaStream_t s) {
   constexpr int W = V16<T>::W;
-  if (g.n1 % W != 0 || !aligned16(vel) || !aligned16(nl)) return false;
-  const long long bx = (g.n1 / W + MBX - 1) / MBX, by = (g.n2 + MBY - 1) / MBY;
-  const int seg = march_seg(bx * by, g.n3);
-  k_helm_march<T><<<dim3((unsigned)bx, (unsigned)by, (g.n3 + seg - 1) / seg), dim3(MBX, MBY), 0, s>>>(g, cx, cy, cz, multL,
-                                                                                                    vel, nl, seg);
-  return true;
+  int seg = 0;
+  if (g.n1 % W == 0 && aligned16(x) && aligned16(y) && aligned16(z)) {
+    const dim3 grid = march_grid(g, W, g.n2, g.n3, seg);
+    k_axpby<T, W><<<grid, MT, 0, s>>>(g, a, b, x, y, z, seg);
+  } else {
+    const dim3 grid = march_grid(g, 1, g.n2, g.n3, seg);
+    k_axpby<T, 1><<<grid, MT, 0, s>>>(g, a, b, x, y, z, seg);
+  }
 }
-
-template <typename T>
-bool launch_jacobi_march(const Geom& g, const T* c1, const T* c2, const T* c3, T omega, const T* bb, const T* rel,
-                         T* out, cudaStream_t s) {
-  constexpr int W = V16<T>::W;
-  if (g.n1 % W != 0 || !aligned16(bb) || !aligned16(rel) || !aligned16(out)) return false;
-  const long long bx = (g.n1 / W + MBX - 1) / MBX, by = (g.n2 + MBY - 1) / MBY;
-  const int seg = march_seg(bx * by, g.n3);
-  k_jacobi_march<T><<<dim3((unsigned)bx, (unsigned)by, (g.n3 + seg - 1) / seg), dim3(MBX, MBY), 0, s>>>(
-      g, c1, c2, c3, omega, bb, rel, out, seg);
-  return true;
-}
-template bool launch_helm_march<double>(const Geom&, const double*, const double*, const double*, double,
-                                        const double*, double*, cudaStream_t);
-template bool launch_helm_march<float>(const Geom&, const float*, const float*, const float*, float, const float*,
-                                       float*, cudaStream_t);
-template bool launch_jacobi_march<double>(const Geom&, const double*, const double*, const double*, double,
-                                          const double*, const double*, double*, cudaStream_t);
-template bool launch_jacobi_march<float>(const Geom&, const float*, const float*, const float*, float, const float*,
-                                         const float*, float*, cudaStream_t);
 
 #define MARCH_INST(T)                                                                                             \
-  template bool launch_march1<T, G_LO, NG, 0>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
+  template void launch_march1<T, G_LO, NG, 0>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
                                               cudaStream_t);                                                      \
-  template bool launch_march1<T, D_LO, ND, 0>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
+  template void launch_march1<T, D_LO, ND, 0>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
                                               cudaStream_t);                                                      \
-  template bool launch_march1<T, D_LO, ND, 1>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
+  template void launch_march1<T, D_LO, ND, 1>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
                                               cudaStream_t);                                                      \
-  template bool launch_march1<T, B_LO, NB, 2>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
-                                              cudaStream_t);
+  template void launch_march1<T, B_LO, NB, 2>(int, const Geom&, const T*, const T*, const T*, const T*, T*, int,  \
+                                              cudaStream_t);                                                      \
+  template void launch_jacobi<T>(const Geom&, const T*, const T*, const T*, T, const T*, const T*, T*,            \
+                                 cudaStream_t);                                                                   \
+  template void launch_axpby<T>(const Geom&, T, T, const T*, const T*, T*, cudaStream_t);
 MARCH_INST(double)
 MARCH_INST(float)
 #undef MARCH_INST

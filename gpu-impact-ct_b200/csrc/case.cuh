@@ -7,14 +7,9 @@
 #include "engine.cuh"
 #include "mg.cuh"
 #include "solver.cuh"
+#include "stencil3.cuh"
 
 namespace impact {
-
-// per-axis row sums used by get_dtime: sum_l |cpp(l,i)| and sum_l |cp1(l,i)|
-struct DtRows {
-  const double* spp[3];
-  const double* sp1[3];
-};
 
 struct CaseState {
   int device = 0;

@@ -14,6 +14,8 @@
 // themselves.  Now bound by that path still (65 % of its cycles; 12 vector loads per 2 points) and by
 // the latency of 16 warps per SM.  256 x 256 x 512 FP64: Helmholtz 250 us (295), divergence2 257 us
 // (389); 128 x 128 x 224 FP32: 17 us (19), 15 us (41); 187 x 131 x 157 FP32: 31 us (50), 27 us (43).
+// 384 x 384 x 768 FP64, in the time step: interpolate_vel 1.09 ms (1.44; with get_dtime's bound
+// in the same pass, which took another 1.94), divergence2 0.82 ms (1.33), projection 1.35 (1.44).
 // The same with the tiles staged in shared memory by cp.async, four planes in a ring: 255 and
 // 262 us, and slower on small grids.
 #include <algorithm>
@@ -90,6 +92,15 @@ __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+
+// The first two terms of a sum.  The Helmholtz term rounds the first product and adds the second
+// by fused multiply-add, as the one-axis passes do; the others round the second product, as the
+// passes of the time step always have (a velocity's last bit decides which way the mixed solve's
+// FP32 image of the residual rounds).
+template <int KIND, typename T>
+__device__ __forceinline__ T head(T c0, T f0, T c1, T f1) {
+  return KIND == TRI_HELM ? fma_(c1, f1, mul_(c0, f0)) : fma_(c0, f0, mul_(c1, f1));
+}
 
 // get_dtime's bound radius / limit(angle) of one point, raised into `best`.  The limit of a ray is
 // at least the smallest of the table, so a point whose radius cannot beat `best` even there is
@@ -217,9 +228,9 @@ __device__ __forceinline__ void tri_block(const Geom& g, const TriArgs<T, TO>& A
     T X[V], Y[V], Z[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-      X[v] = mul_(cx[v][0], xv[v + LO - FV * V]);
+      X[v] = head<KIND>(cx[v][0], xv[v + LO - FV * V], cx[v][1], xv[v + LO + 1 - FV * V]);
 #pragma unroll
-      for (int l = 1; l < CNT; ++l) X[v] = fma_(cx[v][l], xv[v + LO + l - FV * V], X[v]);
+      for (int l = 2; l < CNT; ++l) X[v] = fma_(cx[v][l], xv[v + LO + l - FV * V], X[v]);
     }
     constexpr bool CHAIN = KIND == TRI_DIV2 || KIND == TRI_HELM;  // one sum over the axes
 #pragma unroll
@@ -228,8 +239,8 @@ __device__ __forceinline__ void tri_block(const Geom& g, const TriArgs<T, TO>& A
       for (int v = 0; v < V; ++v) {
         if (CHAIN)
           X[v] = fma_(cy[l], yv[l][v], X[v]);
-        else
-          Y[v] = l == 0 ? mul_(cy[l], yv[l][v]) : fma_(cy[l], yv[l][v], Y[v]);
+        else if (l > 0)
+          Y[v] = l == 1 ? head<KIND>(cy[0], yv[0][v], cy[1], yv[1][v]) : fma_(cy[l], yv[l][v], Y[v]);
       }
 #pragma unroll
     for (int l = 0; l < CNT; ++l)
@@ -237,8 +248,8 @@ __device__ __forceinline__ void tri_block(const Geom& g, const TriArgs<T, TO>& A
       for (int v = 0; v < V; ++v) {
         if (CHAIN)
           X[v] = fma_(cz[l], win[l][v], X[v]);
-        else
-          Z[v] = l == 0 ? mul_(cz[l], win[l][v]) : fma_(cz[l], win[l][v], Z[v]);
+        else if (l > 0)
+          Z[v] = l == 1 ? head<KIND>(cz[0], win[0][v], cz[1], win[1][v]) : fma_(cz[l], win[l][v], Z[v]);
       }
     if constexpr (KIND == TRI_DIV2) {
       stv<TO, T, V>(A.o[0] + p, X);

@@ -2,11 +2,13 @@
 // life cycle (the GPU_setup / GPU_malloc / GPU_memcopy / GPU_memfree of mod_mem_GPU.f90:18-437).
 //
 // The substep (mod_timeint.f90:275-377) is reorganised into fused passes:
-//   interpolate_vel  -> k_interp_vel3   (3 interpolations, one pass)
+//   get_dtime, interpolate_vel -> TRI_INTERP (3 interpolations in one pass, stencil3.cu; the first
+//                                 substep's also forms get_dtime's bound, from the same values)
 //   rhs_vel          -> k_rhs_march     (pp interpolation, 3 upwind terms, explicit Helmholtz and
 //                                        both RK updates of one component in one z-marching pass,
 //                                        rhs.cu)
-//   explicit         -> divergence2 of rhs, Poisson solve, k_project (vel = rhs - G pre, 3 comps)
+//   explicit         -> divergence2 of rhs (TRI_DIV2), Poisson solve, vel = rhs - G pre in three
+//                       components (TRI_PROJECT)
 // Every pass keeps the reference's order of floating-point operations per point.
 #include <algorithm>
 #include <cmath>
@@ -31,67 +33,6 @@ static inline dim3 grid3(const Geom& g) { return dim3((g.n1 + BX - 1) / BX, (g.n
 static const double aRK[3] = {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
 static const double bRK[3] = {0.0, -17.0 / 60.0, -5.0 / 12.0};
 
-#define PT                                                  \
-  const int i = blockIdx.x * BX + threadIdx.x + 1;          \
-  const int j = blockIdx.y * BY + threadIdx.y + 1;          \
-  const int k = blockIdx.z + 1;                             \
-  if (i > g.n1 || j > g.n2) return;                         \
-  const long long p = off(g, i, j, k);
-
-__device__ __forceinline__ int crd(int a, int i, int j, int k) { return a == 0 ? i : (a == 1 ? j : k); }
-__device__ __forceinline__ int ext(const Geom& g, int a) { return a == 0 ? g.n1 : (a == 1 ? g.n2 : g.n3); }
-__device__ __forceinline__ long long strd(const Geom& g, int a) { return a == 0 ? 1LL : (a == 1 ? (long long)g.nx : g.nxy); }
-
-// WRAP = false: the whole block lies at least 3 points inside the periodic box, so the stencil
-// points are p + l * stride without any index wrapping (same values, same operation order)
-template <int LO, int CNT, bool WRAP>
-__device__ __forceinline__ double st1w(const double* __restrict__ c, const double* __restrict__ f, const Geom& g, int a,
-                                       int i, int j, int k, long long p) {
-  if (WRAP) {
-    const int q = crd(a, i, j, k), n = ext(g, a);
-    const long long s = strd(g, a);
-    const long long base = p - (long long)q * s;
-    const double* cr = c + (long long)q * CNT;
-    double v = cr[0] * __ldg(f + base + (long long)wrapi(q + LO, n) * s);
-#pragma unroll
-    for (int l = 1; l < CNT; ++l) v = v + cr[l] * __ldg(f + base + (long long)wrapi(q + LO + l, n) * s);
-    return v;
-  }
-  const int q = crd(a, i, j, k);
-  const long long s = strd(g, a);
-  const double* cr = c + (long long)q * CNT;
-  const double* fp = f + p + (long long)LO * s;
-  double v = cr[0] * __ldg(fp);
-#pragma unroll
-  for (int l = 1; l < CNT; ++l) v = v + cr[l] * __ldg(fp + l * s);
-  return v;
-}
-template <int LO, int CNT, bool WRAP>
-__device__ __forceinline__ double st1w_acc(double v, const double* __restrict__ c, const double* __restrict__ f,
-                                           const Geom& g, int a, int i, int j, int k, long long p) {
-  if (WRAP) {
-    const int q = crd(a, i, j, k), n = ext(g, a);
-    const long long s = strd(g, a);
-    const long long base = p - (long long)q * s;
-    const double* cr = c + (long long)q * CNT;
-#pragma unroll
-    for (int l = 0; l < CNT; ++l) v = v + cr[l] * __ldg(f + base + (long long)wrapi(q + LO + l, n) * s);
-    return v;
-  }
-  const int q = crd(a, i, j, k);
-  const long long s = strd(g, a);
-  const double* cr = c + (long long)q * CNT;
-  const double* fp = f + p + (long long)LO * s;
-#pragma unroll
-  for (int l = 0; l < CNT; ++l) v = v + cr[l] * __ldg(fp + l * s);
-  return v;
-}
-// the points of block (bx, by) on plane k and their 3-point halos stay inside 1..n on every axis
-__device__ __forceinline__ bool block_interior(const Geom& g, int bx, int by, int k) {
-  const int i0 = bx * BX + 1, j0 = by * BY + 1;
-  return i0 - 3 >= 1 && i0 + BX - 1 + 3 <= g.n1 && j0 - 3 >= 1 && j0 + BY - 1 + 3 <= g.n2 && k - 3 >= 1 &&
-         k + 3 <= g.n3;
-}
 // the point of this thread in block (bx, by, bz) of a grid3 launch; returns false outside the grid
 #define PTB(bx, by, bz)                                      \
   const int i = (bx) * BX + threadIdx.x + 1;                 \
@@ -100,100 +41,24 @@ __device__ __forceinline__ bool block_interior(const Geom& g, int bx, int by, in
   if (i > g.n1 || j > g.n2) return;                          \
   const long long p = off(g, i, j, k);
 
-// interpolate_vel (mod_diff.f90:1436-1472): work_m = I_{u_m -> p} vel_m, three components, in
-// FP64 from the FP64 velocity; TO = float stores the FP32 work fields of a mixed-precision case
-template <typename TO>
-__device__ __forceinline__ void interp_vel3_block(const Geom& g, const Coeffs<double>& c, const double* __restrict__ u,
-                                                  const double* __restrict__ v, const double* __restrict__ w,
-                                                  TO* __restrict__ w1, TO* __restrict__ w2, TO* __restrict__ w3,
-                                                  int bx, int by, int bz) {
-  const bool wrap = !block_interior(g, bx, by, bz + 1);
-  PTB(bx, by, bz)
-  if (wrap) {
-    w1[p] = (TO)st1w<D_LO, ND, true>(c.cIup[0], u, g, 0, i, j, k, p);
-    w2[p] = (TO)st1w<D_LO, ND, true>(c.cIup[1], v, g, 1, i, j, k, p);
-    w3[p] = (TO)st1w<D_LO, ND, true>(c.cIup[2], w, g, 2, i, j, k, p);
-  } else {
-    w1[p] = (TO)st1w<D_LO, ND, false>(c.cIup[0], u, g, 0, i, j, k, p);
-    w2[p] = (TO)st1w<D_LO, ND, false>(c.cIup[1], v, g, 1, i, j, k, p);
-    w3[p] = (TO)st1w<D_LO, ND, false>(c.cIup[2], w, g, 2, i, j, k, p);
-  }
+// The pressure scaling of the substeps: pre * ab * dt before a solve (mod_timeint.f90:318), pre /
+// ab / dt after the projection (:372).  Between two substeps nothing reads the pressure, so one
+// pass divides by the previous substep's factor and multiplies by the next one's (ab_old = 0: only
+// the multiplication; ab_new = 0: only the division).
+__device__ __forceinline__ double scaled_pre(double v, double ab_old, double ab_new, double dt) {
+  if (ab_old != 0.0) v = v / ab_old / dt;
+  if (ab_new != 0.0) v = v * ab_new * dt;
+  return v;
 }
-__global__ void __launch_bounds__(NT) k_interp_vel3_32(Geom g, Coeffs<double> c, const double* __restrict__ u,
-                                                       const double* __restrict__ v, const double* __restrict__ w,
-                                                       float* __restrict__ w1, float* __restrict__ w2,
-                                                       float* __restrict__ w3) {
-  interp_vel3_block<float>(g, c, u, v, w, w1, w2, w3, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-__global__ void __launch_bounds__(NT) k_interp_vel3(Geom g, Coeffs<double> c, const double* __restrict__ u,
-                                                    const double* __restrict__ v, const double* __restrict__ w,
-                                                    double* __restrict__ w1, double* __restrict__ w2,
-                                                    double* __restrict__ w3) {
-  interp_vel3_block<double>(g, c, u, v, w, w1, w2, w3, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-// pre = pre * ab * dt  (mod_timeint.f90:318)  /  pre = pre / ab / dt  (:372)
-__device__ __forceinline__ void scale_pre_block(const Geom& g, double ab, double dt, int divide,
+__device__ __forceinline__ void scale_pre_block(const Geom& g, double ab_old, double ab_new, double dt,
                                                 double* __restrict__ pre, int bx, int by, int bz) {
   PTB(bx, by, bz)
-  pre[p] = divide ? pre[p] / ab / dt : pre[p] * ab * dt;
+  pre[p] = scaled_pre(pre[p], ab_old, ab_new, dt);
 }
-__global__ void __launch_bounds__(NT) k_scale_pre(Geom g, double ab, double dt, int divide, double* __restrict__ pre) {
-  scale_pre_block(g, ab, dt, divide, pre, blockIdx.x, blockIdx.y, blockIdx.z);
+__global__ void __launch_bounds__(NT) k_scale_pre(Geom g, double ab_old, double ab_new, double dt,
+                                                  double* __restrict__ pre) {
+  scale_pre_block(g, ab_old, ab_new, dt, pre, blockIdx.x, blockIdx.y, blockIdx.z);
 }
-
-// explicit (mod_solvers.f90:180-330): vel_m = rhs_m - G_m pre for the three components
-__device__ __forceinline__ void project_block(const Geom& g, const Coeffs<double>& c, const double* __restrict__ pre,
-                                              const double* __restrict__ r1, const double* __restrict__ r2,
-                                              const double* __restrict__ r3, double* __restrict__ u,
-                                              double* __restrict__ v, double* __restrict__ w, int bx, int by, int bz) {
-  const bool wrap = !block_interior(g, bx, by, bz + 1);
-  PTB(bx, by, bz)
-  if (wrap) {
-    u[p] = 1.0 * r1[p] + (-1.0) * st1w<G_LO, NG, true>(c.cG[0], pre, g, 0, i, j, k, p);
-    v[p] = 1.0 * r2[p] + (-1.0) * st1w<G_LO, NG, true>(c.cG[1], pre, g, 1, i, j, k, p);
-    w[p] = 1.0 * r3[p] + (-1.0) * st1w<G_LO, NG, true>(c.cG[2], pre, g, 2, i, j, k, p);
-  } else {
-    u[p] = 1.0 * r1[p] + (-1.0) * st1w<G_LO, NG, false>(c.cG[0], pre, g, 0, i, j, k, p);
-    v[p] = 1.0 * r2[p] + (-1.0) * st1w<G_LO, NG, false>(c.cG[1], pre, g, 1, i, j, k, p);
-    w[p] = 1.0 * r3[p] + (-1.0) * st1w<G_LO, NG, false>(c.cG[2], pre, g, 2, i, j, k, p);
-  }
-}
-__global__ void __launch_bounds__(NT) k_project(Geom g, Coeffs<double> c, const double* __restrict__ pre,
-                                                const double* __restrict__ r1, const double* __restrict__ r2,
-                                                const double* __restrict__ r3, double* __restrict__ u,
-                                                double* __restrict__ v, double* __restrict__ w) {
-  project_block(g, c, pre, r1, r2, r3, u, v, w, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-// divergence2 (mod_diff.f90:130-215) of the provisional velocity into the pressure equation's
-// right-hand side: x stencil, then y and z added in table order
-__device__ __forceinline__ void div2_block(const Geom& g, const Coeffs<double>& c, const double* __restrict__ u,
-                                           const double* __restrict__ v, const double* __restrict__ w,
-                                           double* __restrict__ div, int bx, int by, int bz) {
-  const bool wrap = !block_interior(g, bx, by, bz + 1);
-  PTB(bx, by, bz)
-  double d;
-  if (wrap) {
-    d = st1w<D_LO, ND, true>(c.cD[0], u, g, 0, i, j, k, p);
-    d = st1w_acc<D_LO, ND, true>(d, c.cD[1], v, g, 1, i, j, k, p);
-    d = st1w_acc<D_LO, ND, true>(d, c.cD[2], w, g, 2, i, j, k, p);
-  } else {
-    d = st1w<D_LO, ND, false>(c.cD[0], u, g, 0, i, j, k, p);
-    d = st1w_acc<D_LO, ND, false>(d, c.cD[1], v, g, 1, i, j, k, p);
-    d = st1w_acc<D_LO, ND, false>(d, c.cD[2], w, g, 2, i, j, k, p);
-  }
-  div[p] = d;
-}
-__global__ void __launch_bounds__(NT) k_div2(Geom g, Coeffs<double> c, const double* __restrict__ u,
-                                             const double* __restrict__ v, const double* __restrict__ w,
-                                             double* __restrict__ div) {
-  div2_block(g, c, u, v, w, div, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-
-// get_dtime (mod_lib.f90:46-250), timeint_mode 1: block max of radius / stabilitylimit(angle)
-__constant__ double c_stab[41];
 
 __device__ __forceinline__ double wmax_d(double v) {
 #pragma unroll
@@ -204,57 +69,6 @@ __device__ __forceinline__ double wsum_d(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-__device__ __forceinline__ void dtime_block(const Geom& g, const Coeffs<double>& c, const DtRows& dr, double Re,
-                                            const double* __restrict__ u, const double* __restrict__ v,
-                                            const double* __restrict__ w, double* __restrict__ partial, int bx,
-                                            int by, int bz, int gx, int gy) {
-  const int i = bx * BX + threadIdx.x + 1;
-  const int j = by * BY + threadIdx.y + 1;
-  const int k = bz + 1;
-  double beta = 0.0;
-  const bool wrap = !block_interior(g, bx, by, k);
-  if (i <= g.n1 && j <= g.n2) {
-    const long long p = off(g, i, j, k);
-    double w1, w2, w3;
-    if (wrap) {
-      w1 = st1w<D_LO, ND, true>(c.cIup[0], u, g, 0, i, j, k, p);
-      w2 = st1w<D_LO, ND, true>(c.cIup[1], v, g, 1, i, j, k, p);
-      w3 = st1w<D_LO, ND, true>(c.cIup[2], w, g, 2, i, j, k, p);
-    } else {
-      w1 = st1w<D_LO, ND, false>(c.cIup[0], u, g, 0, i, j, k, p);
-      w2 = st1w<D_LO, ND, false>(c.cIup[1], v, g, 1, i, j, k, p);
-      w3 = st1w<D_LO, ND, false>(c.cIup[2], w, g, 2, i, j, k, p);
-    }
-    double are = dr.spp[0][i] + dr.spp[1][j];
-    are = are + dr.spp[2][k];
-    are = are / Re;
-    double aim = dr.sp1[0][i] * fabs(w1);
-    aim = aim + dr.sp1[1][j] * fabs(w2);
-    aim = aim + dr.sp1[2][k] * fabs(w3);
-    const double pi = 3.14159265358979323846;
-    const double angle = (fabs(aim) < 1e-16) ? pi / 2.0 : atan(are / aim);
-    const double radius = sqrt(are * are + aim * aim);
-    long long idx = llround(2.0 * 40.0 * angle / pi);
-    idx = idx < 0 ? 0 : (idx > 40 ? 40 : idx);
-    beta = radius / c_stab[idx];
-  }
-  __shared__ double sh[NT / 32];
-  const int tid = threadIdx.x + BX * threadIdx.y;
-  beta = wmax_d(beta);
-  if ((tid & 31) == 0) sh[tid >> 5] = beta;
-  __syncthreads();
-  if (tid < 32) {
-    double x = tid < NT / 32 ? sh[tid] : 0.0;
-    x = wmax_d(x);
-    if (tid == 0) partial[bx + (long long)gx * (by + (long long)gy * bz)] = x;
-  }
-}
-__global__ void __launch_bounds__(NT) k_dtime(Geom g, Coeffs<double> c, DtRows dr, double Re, const double* __restrict__ u,
-                                              const double* __restrict__ v, const double* __restrict__ w,
-                                              double* __restrict__ partial) {
-  dtime_block(g, c, dr, Re, u, v, w, partial, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
 }
 
 // fixed-order max / sum over n partials (single block)
@@ -287,12 +101,18 @@ __global__ void k_widen(const float* __restrict__ a, double* __restrict__ b, lon
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
     b[q] = (double)a[q];
 }
-__device__ __forceinline__ void sum_block(const Geom& g, const double* __restrict__ a, double* __restrict__ partial,
-                                          int bx, int by, int bz, int gx, int gy) {
+// ... after the last substep's division by ab dt, written back
+__device__ __forceinline__ void scale_sum_block(const Geom& g, double ab, double dt, double* __restrict__ a,
+                                                double* __restrict__ partial, int bx, int by, int bz, int gx, int gy) {
   const int i = bx * BX + threadIdx.x + 1;
   const int j = by * BY + threadIdx.y + 1;
   const int k = bz + 1;
-  double s = (i <= g.n1 && j <= g.n2) ? a[off(g, i, j, k)] : 0.0;
+  double s = 0.0;
+  if (i <= g.n1 && j <= g.n2) {
+    const long long p = off(g, i, j, k);
+    s = scaled_pre(a[p], ab, 0.0, dt);
+    a[p] = s;
+  }
   __shared__ double sh[NT / 32];
   const int tid = threadIdx.x + BX * threadIdx.y;
   s = wsum_d(s);
@@ -304,8 +124,9 @@ __device__ __forceinline__ void sum_block(const Geom& g, const double* __restric
     if (tid == 0) partial[bx + (long long)gx * (by + (long long)gy * bz)] = x;
   }
 }
-__global__ void __launch_bounds__(NT) k_sum(Geom g, const double* __restrict__ a, double* __restrict__ partial) {
-  sum_block(g, a, partial, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
+__global__ void __launch_bounds__(NT) k_scale_sum(Geom g, double ab, double dt, double* __restrict__ a,
+                                                  double* __restrict__ partial) {
+  scale_sum_block(g, ab, dt, a, partial, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, gridDim.y);
 }
 __device__ __forceinline__ void sub_mean_block(const Geom& g, const double* __restrict__ sum, double* __restrict__ pre,
                                                int bx, int by, int bz) {
@@ -353,21 +174,15 @@ struct StepScal {  // per case and step: time step, Reynolds number, inflow at t
 };
 struct ExJob {
   Geom g;
-  Coeffs<double> c;
-  DtRows dr;
   double* vel[3];
-  double* nl[3];
-  double* rhs[3];
-  double* work[3];
-  float* work32[3];  // mixed precision: the FP32 interpolated velocities (null in FP64)
   double* pre;
-  double* res;
   const uint8_t* label;
   double* partial;
   double* dscal;
   const StepScal* sc;  // this case's scalars of the current step
   int gx, gy, gz, b0;  // grid3 blocks (one plane each) of the case, from block b0 on
   int pb0;             // blocks of XPL planes (the point kernels), from block pb0 on
+  int ndt;             // partials of get_dtime's bound
 };
 
 __device__ __forceinline__ int ex_job(const ExJob* __restrict__ jobs, int nj, int b) {
@@ -406,50 +221,28 @@ __device__ __forceinline__ int ex_pjob(const ExJob* __restrict__ jobs, int nj, i
 __constant__ double RKA_D[3] = {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
 __constant__ double RKB_D[3] = {0.0, -17.0 / 60.0, -5.0 / 12.0};
 
-__global__ void __launch_bounds__(NT) k_b_dtime(const ExJob* __restrict__ jobs, int nj) {
-  EX_BLOCK
-  dtime_block(g, J.c, J.dr, J.sc->Re, J.vel[0], J.vel[1], J.vel[2], J.partial, bx, by, bz, J.gx, J.gy);
-}
 // one block per case: out = dscal[slot] of the case
 // one block per case: the case's dscal[slot], or out[case] when out is given
 __global__ void __launch_bounds__(1024) k_b_reduce(const ExJob* __restrict__ jobs, int is_max, int slot, int only_lp,
                                                    double* __restrict__ out) {
   const ExJob& J = jobs[blockIdx.x];
   if (only_lp && !J.sc->level_pressure) return;
-  reduce_partials_block(J.partial, (long long)J.gx * J.gy * J.gz, is_max, out ? out + blockIdx.x : J.dscal + slot);
+  reduce_partials_block(J.partial, is_max ? J.ndt : (long long)J.gx * J.gy * J.gz, is_max, out ? out + blockIdx.x : J.dscal + slot);
 }
-__global__ void __launch_bounds__(NT) k_b_interp(const ExJob* __restrict__ jobs, int nj, int f32) {
+__global__ void __launch_bounds__(NT) k_b_scale_pre(const ExJob* __restrict__ jobs, int nj, int sub_old, int sub_new) {
   EX_PBLOCK
-  for (int bz = kb0; bz < kb1; ++bz) {
-    if (f32)
-      interp_vel3_block<float>(g, J.c, J.vel[0], J.vel[1], J.vel[2], J.work32[0], J.work32[1], J.work32[2], bx, by,
-                               bz);
-    else
-      interp_vel3_block<double>(g, J.c, J.vel[0], J.vel[1], J.vel[2], J.work[0], J.work[1], J.work[2], bx, by, bz);
-  }
-}
-__global__ void __launch_bounds__(NT) k_b_scale_pre(const ExJob* __restrict__ jobs, int nj, int sub, int divide) {
-  EX_PBLOCK
-  for (int bz = kb0; bz < kb1; ++bz) scale_pre_block(g, RKA_D[sub] + RKB_D[sub], J.sc->dt, divide, J.pre, bx, by, bz);
-}
-__global__ void __launch_bounds__(NT) k_b_div2(const ExJob* __restrict__ jobs, int nj) {
-  EX_PBLOCK
-  for (int bz = kb0; bz < kb1; ++bz) div2_block(g, J.c, J.rhs[0], J.rhs[1], J.rhs[2], J.res, bx, by, bz);
-}
-__global__ void __launch_bounds__(NT) k_b_project(const ExJob* __restrict__ jobs, int nj) {
-  EX_PBLOCK
-  for (int bz = kb0; bz < kb1; ++bz)
-    project_block(g, J.c, J.pre, J.rhs[0], J.rhs[1], J.rhs[2], J.vel[0], J.vel[1], J.vel[2], bx, by, bz);
+  const double o = sub_old >= 0 ? RKA_D[sub_old] + RKB_D[sub_old] : 0.0;
+  const double w = sub_new >= 0 ? RKA_D[sub_new] + RKB_D[sub_new] : 0.0;
+  for (int bz = kb0; bz < kb1; ++bz) scale_pre_block(g, o, w, J.sc->dt, J.pre, bx, by, bz);
 }
 __global__ void __launch_bounds__(NT) k_b_mask(const ExJob* __restrict__ jobs, int nj) {
   EX_PBLOCK
   for (int bz = kb0; bz < kb1; ++bz)
     mask_block(g, J.label, J.sc->u_in, J.sc->inflow_on, J.vel[0], J.vel[1], J.vel[2], bx, by, bz);
 }
-__global__ void __launch_bounds__(NT) k_b_sum(const ExJob* __restrict__ jobs, int nj) {
+__global__ void __launch_bounds__(NT) k_b_scale_sum(const ExJob* __restrict__ jobs, int nj, int sub) {
   EX_BLOCK
-  if (!J.sc->level_pressure) return;
-  sum_block(g, J.pre, J.partial, bx, by, bz, J.gx, J.gy);
+  scale_sum_block(g, RKA_D[sub] + RKB_D[sub], J.sc->dt, J.pre, J.partial, bx, by, bz, J.gx, J.gy);
 }
 __global__ void __launch_bounds__(NT) k_b_sub_mean(const ExJob* __restrict__ jobs, int nj) {
   EX_PBLOCK
@@ -1342,17 +1135,66 @@ static int upload_stab(cudaStream_t st) {
     stability_limits(stab_host);
     stab_ready = true;
   }
-  IMPACT_CUDA_CHECK(cudaMemcpyToSymbolAsync(c_stab, stab_host, sizeof(stab_host), 0, cudaMemcpyHostToDevice, st));
-  return 0;
+  return tri_upload_limits(stab_host, st);
 }
 
-// get_dtime: the CFL bound beta of the case lands in s.dscal[0]
+// the three-axis passes of one case
+static TriArgs<double, double> tri_args(CaseState& s, int kind) {
+  TriArgs<double, double> a{};
+  for (int m = 0; m < 3; ++m) {
+    a.c[m] = kind == TRI_DIV2 ? s.c64.cD[m] : (kind == TRI_INTERP ? s.c64.cIup[m] : s.c64.cG[m]);
+    a.f[m] = kind == TRI_DIV2 ? s.f[IMPACT_B200_RHS1 + m] : s.f[IMPACT_B200_VEL1 + m];
+    a.s[m] = s.f[IMPACT_B200_RHS1 + m];
+    a.o[m] = kind == TRI_INTERP ? s.work[m] : s.f[IMPACT_B200_VEL1 + m];
+  }
+  if (kind == TRI_DIV2) a.o[0] = s.f[IMPACT_B200_RES];
+  if (kind == TRI_PROJECT) a.f[0] = s.f[IMPACT_B200_PRE];
+  a.ahead = tri_ahead(s.g, sizeof(double));
+  return a;
+}
+static bool tri_vec(const CaseState& s) {  // every field of a case is one allocation of the pool
+  const void* f[14];
+  int n = 0;
+  for (int q = 0; q < IMPACT_B200_NFIELDS; ++q) f[n++] = s.f[q];
+  for (int q = 0; q < 3; ++q) f[n++] = s.work[q];
+  bool ok = tri_vectorable(s.g, sizeof(double), f, n);
+  for (int q = 0; q < 3; ++q) ok = ok && (reinterpret_cast<uintptr_t>(s.work32[q]) & 7) == 0;
+  return ok;
+}
+// interpolate_vel; with p also get_dtime's bound of every block into s.partial.  f32: the FP32
+// work fields
+static void step_interp(CaseState& s, int f32, const impact_b200_step_params* p, cudaStream_t st) {
+  const TriGrid tg = tri_grid(s.g, sizeof(double), tri_vec(s));
+  const TriArgs<double, double> a = tri_args(s, TRI_INTERP);
+  auto with_dt = [&](auto& t) {
+    t.dr = s.dt;
+    t.ReV = p ? p->Re : 1.0;
+    t.partial = p ? s.partial : nullptr;
+  };
+  if (f32) {
+    TriArgs<double, float> b{};
+    for (int m = 0; m < 3; ++m) {
+      b.c[m] = a.c[m];
+      b.f[m] = a.f[m];
+      b.o[m] = s.work32[m];
+    }
+    b.ahead = a.ahead;
+    with_dt(b);
+    launch_tri<TRI_INTERP, double, float>(s.g, b, tg, st);
+  } else {
+    TriArgs<double, double> b = a;
+    with_dt(b);
+    launch_tri<TRI_INTERP, double, double>(s.g, b, tg, st);
+  }
+  prof::count(1);
+}
+
+// get_dtime: the CFL bound beta of the case lands in s.dscal[0]; the interpolated velocities it
+// is formed from are the first substep's work fields
 static void step_beta(CaseState& s, const impact_b200_step_params* p, cudaStream_t st) {
-  const Geom& g = s.g;
-  k_dtime<<<grid3(g), dim3(BX, BY), 0, st>>>(g, s.c64, s.dt, p->Re, s.f[IMPACT_B200_VEL1], s.f[IMPACT_B200_VEL2],
-                                             s.f[IMPACT_B200_VEL3], s.partial);
-  k_reduce_partials<<<1, 1024, 0, st>>>(s.partial, nblocks(g), 1, s.dscal);
-  prof::count(2);
+  step_interp(s, s.precision == 1 && p->explicit_fp32, p, st);
+  k_reduce_partials<<<1, 1024, 0, st>>>(s.partial, tri_grid(s.g, sizeof(double), tri_vec(s)).blocks(), 1, s.dscal);
+  prof::count(1);
 }
 
 static double dt_from_beta(double beta1, const impact_b200_step_params* p, const impact_b200_step_state* stt) {
@@ -1377,17 +1219,15 @@ static void substep_rhs(CaseState& s, const impact_b200_step_params* p, double d
   const double multL = 1.0 / p->Re;
   const double mb = dt * bRK[sub], ma = dt * aRK[sub];
   const int use_old = sub != 0;
-  if (s.precision == 1 && p->explicit_fp32) {  // FP32 rhs_vel pass: FP32 work fields and nonlinear term
-    k_interp_vel3_32<<<gr, bl, 0, st>>>(g, s.c64, vel[0], vel[1], vel[2], s.work32[0], s.work32[1], s.work32[2]);
-    prof::count(1);
+  const int f32 = s.precision == 1 && p->explicit_fp32;
+  if (sub > 0) step_interp(s, f32, nullptr, st);  // the first substep's came with get_dtime
+  if (f32) {  // FP32 rhs_vel pass: FP32 work fields and nonlinear term
     // bytes: vel 8 (the staged tile and the point), work 3 x 4, nl 4 (+4 old), rhs 8
     const double nlb = (use_old ? 36.0 : 32.0) * cells;
     for (int m = 0; m < 3; ++m)
       IMPACT_PROF(prof::K_NL_RHS, nlb, st,
                   launch_rhs_march32(m, g, s.c32, multL, mb, ma, use_old, vel[m], s.work32, s.nl32[m], rhs[m], st));
   } else {
-    k_interp_vel3<<<gr, bl, 0, st>>>(g, s.c64, vel[0], vel[1], vel[2], s.work[0], s.work[1], s.work[2]);
-    prof::count(1);
     const double nlb = (use_old ? 7.0 : 6.0) * 8.0 * cells;
     for (int m = 0; m < 3; ++m)
       IMPACT_PROF(prof::K_NL_RHS, nlb, st,
@@ -1396,27 +1236,29 @@ static void substep_rhs(CaseState& s, const impact_b200_step_params* p, double d
   // divergence2 reads no pressure: it runs before the pressure's first read, so that a deferred
   // pressure upload overlaps it too
   IMPACT_PROF(prof::K_DIV2, 4.0 * 8.0 * cells, st,
-              (k_div2<<<gr, bl, 0, st>>>(g, s.c64, rhs[0], rhs[1], rhs[2], s.f[IMPACT_B200_RES])));
-  const double ab = aRK[sub] + bRK[sub];
+              (launch_tri<TRI_DIV2, double, double>(g, tri_args(s, TRI_DIV2), tri_grid(g, sizeof(double), tri_vec(s)), st)));
   if (s.pre_wait) {  // a deferred pressure upload: wait for it here, at the step's first read
     cudaStreamWaitEvent(st, s.pre_wait, 0);
     s.pre_wait = nullptr;
   }
-  k_scale_pre<<<gr, bl, 0, st>>>(g, ab, dt, 0, s.f[IMPACT_B200_PRE]);
+  k_scale_pre<<<gr, bl, 0, st>>>(g, sub > 0 ? aRK[sub - 1] + bRK[sub - 1] : 0.0, aRK[sub] + bRK[sub], dt,
+                                 s.f[IMPACT_B200_PRE]);
   prof::count(1);
 }
 
-// projection vel = rhs - G pre and the pressure scaling back (mod_timeint.f90:372)
-static void substep_project(CaseState& s, double dt, int sub, cudaStream_t st) {
+// projection vel = rhs - G pre; after the last substep the pressure is scaled back
+// (mod_timeint.f90:372), with the partial sums of level_pressure when it follows
+static void substep_project(CaseState& s, const impact_b200_step_params* p, double dt, int sub, cudaStream_t st) {
   const Geom& g = s.g;
   const dim3 gr = grid3(g), bl(BX, BY);
   const double cells = (double)g.n1 * g.n2 * g.n3;
-  double* pre = s.f[IMPACT_B200_PRE];
   IMPACT_PROF(prof::K_PROJECT, 7.0 * 8.0 * cells, st,
-              k_project<<<gr, bl, 0, st>>>(g, s.c64, pre, s.f[IMPACT_B200_RHS1], s.f[IMPACT_B200_RHS2],
-                                           s.f[IMPACT_B200_RHS3], s.f[IMPACT_B200_VEL1], s.f[IMPACT_B200_VEL2],
-                                           s.f[IMPACT_B200_VEL3]));
-  k_scale_pre<<<gr, bl, 0, st>>>(g, aRK[sub] + bRK[sub], dt, 1, pre);
+              (launch_tri<TRI_PROJECT, double, double>(g, tri_args(s, TRI_PROJECT), tri_grid(g, sizeof(double), tri_vec(s)), st)));
+  if (sub < 2) return;
+  if (p->level_pressure)
+    k_scale_sum<<<gr, bl, 0, st>>>(g, aRK[sub] + bRK[sub], dt, s.f[IMPACT_B200_PRE], s.partial);
+  else
+    k_scale_pre<<<gr, bl, 0, st>>>(g, aRK[sub] + bRK[sub], 0.0, dt, s.f[IMPACT_B200_PRE]);
   prof::count(1);
 }
 
@@ -1456,10 +1298,9 @@ static void step_finish(CaseState& s, const impact_b200_step_params* p, impact_b
   k_mask<<<gr, bl, 0, st>>>(g, s.label, u_in, on, s.f[IMPACT_B200_VEL1], s.f[IMPACT_B200_VEL2], s.f[IMPACT_B200_VEL3]);
   prof::count(1);
   if (p->level_pressure) {
-    k_sum<<<gr, bl, 0, st>>>(g, s.f[IMPACT_B200_PRE], s.partial);
     k_reduce_partials<<<1, 1024, 0, st>>>(s.partial, nblocks(g), 0, s.dscal + 1);
     k_sub_mean<<<gr, bl, 0, st>>>(g, s.dscal + 1, s.f[IMPACT_B200_PRE]);
-    prof::count(3);
+    prof::count(2);
   }
 }
 
@@ -1488,7 +1329,7 @@ extern "C" int impact_b200_case_step(impact_b200_case* c, const impact_b200_step
       int rc = run_poisson(s, s.f[IMPACT_B200_RES], s.f[IMPACT_B200_PRE], &p->poisson, &r);
       if (rc) return rc;
       record_solve(st, sub, r);
-      substep_project(s, dt, sub, s.stream);
+      substep_project(s, p, dt, sub, s.stream);
     }
     step_finish(s, p, st, dt, s.stream);
   }
@@ -1513,10 +1354,12 @@ struct impact_b200_batch {
   // the explicit part's job lists (built on the first step) and per-step scalars
   ExJob* d_ex = nullptr;
   RhsJob* d_rhs = nullptr;
+  TriJob* d_tri = nullptr;
   StepScal* d_sc = nullptr;
   StepScal* h_sc = nullptr;  // pinned
   double* d_beta = nullptr;
-  int ex_blocks = 0, ex_pblocks = 0, rhs_blocks = 0;  // grid3 blocks, XPL-plane blocks, rhs_vel blocks
+  // grid3 blocks, XPL-plane blocks, rhs_vel blocks, blocks of the three-axis passes
+  int ex_blocks = 0, ex_pblocks = 0, rhs_blocks = 0, tri_blocks = 0;
 };
 
 extern "C" int impact_b200_batch_destroy(impact_b200_batch* b) {
@@ -1529,6 +1372,7 @@ extern "C" int impact_b200_batch_destroy(impact_b200_batch* b) {
   if (b->h_sc) cudaFreeHost(b->h_sc);
   cudaFree(b->d_ex);
   cudaFree(b->d_rhs);
+  cudaFree(b->d_tri);
   cudaFree(b->d_sc);
   cudaFree(b->d_beta);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -1567,7 +1411,13 @@ static int batch_jobs(impact_b200_batch* b) {
   const int n = (int)b->cases.size();
   std::vector<ExJob> ex(n);
   std::vector<RhsJob> rj(n);
-  int eb = 0, rb = 0;
+  std::vector<TriJob> tj(n);
+  int eb = 0, rb = 0, tb = 0;
+  double total = 0.0;
+  for (int c = 0; c < n; ++c) {
+    const Geom& g = b->cases[c]->s.g;
+    total += (double)g.n1 * g.n2 * g.n3;
+  }
   cudaError_t e = cudaMalloc((void**)&b->d_sc, n * sizeof(StepScal));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_sc, n * sizeof(StepScal));
   if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_beta, n * sizeof(double));
@@ -1582,17 +1432,8 @@ static int batch_jobs(impact_b200_batch* b) {
     ExJob& J = ex[c];
     J = ExJob{};
     J.g = s.g;
-    J.c = s.c64;
-    J.dr = s.dt;
-    for (int m = 0; m < 3; ++m) {
-      J.vel[m] = s.f[IMPACT_B200_VEL1 + m];
-      J.nl[m] = s.f[IMPACT_B200_NL1 + m];
-      J.rhs[m] = s.f[IMPACT_B200_RHS1 + m];
-      J.work[m] = s.work[m];
-      J.work32[m] = s.work32[m];
-    }
+    for (int m = 0; m < 3; ++m) J.vel[m] = s.f[IMPACT_B200_VEL1 + m];
     J.pre = s.f[IMPACT_B200_PRE];
-    J.res = s.f[IMPACT_B200_RES];
     J.label = s.label;
     J.partial = s.partial;
     J.dscal = s.dscal;
@@ -1605,6 +1446,29 @@ static int batch_jobs(impact_b200_batch* b) {
     eb += J.gx * J.gy * J.gz;
     J.pb0 = pb;
     pb += J.gx * J.gy * ((J.gz + XPL - 1) / XPL);
+    TriJob& T = tj[c];
+    T = TriJob{};
+    T.g = s.g;
+    T.tg = tri_grid(s.g, sizeof(double), tri_vec(s), (long long)total);
+    T.b0 = tb;
+    tb += T.tg.blocks();
+    for (int kind : {(int)TRI_DIV2, (int)TRI_INTERP, (int)TRI_PROJECT}) {
+      T.a[kind] = tri_args(s, kind);
+      T.a[kind].ahead = total * 24.0 > 96e6;
+    }
+    T.a[TRI_INTERP].dr = s.dt;
+    T.a[TRI_INTERP].Re = &b->d_sc[c].Re;
+    T.a[TRI_INTERP].partial = s.partial;
+    for (int m = 0; m < 3; ++m) {
+      T.a32.c[m] = T.a[TRI_INTERP].c[m];
+      T.a32.f[m] = T.a[TRI_INTERP].f[m];
+      T.a32.o[m] = s.work32[m];
+    }
+    T.a32.ahead = T.a[TRI_INTERP].ahead;
+    T.a32.dr = s.dt;
+    T.a32.Re = T.a[TRI_INTERP].Re;
+    T.a32.partial = s.partial;
+    J.ndt = T.tg.blocks();
     RhsJob& R = rj[c];
     R = RhsJob{};
     R.g = s.g;
@@ -1614,11 +1478,11 @@ static int batch_jobs(impact_b200_batch* b) {
     R.dt = &b->d_sc[c].dt;
     for (int m = 0; m < 3; ++m) {
       R.vel[m] = J.vel[m];
-      R.work[m] = J.work[m];
-      R.nl[m] = J.nl[m];
+      R.work[m] = s.work[m];
+      R.nl[m] = s.f[IMPACT_B200_NL1 + m];
       R.work32[m] = s.work32[m];
       R.nl32[m] = s.nl32[m];
-      R.rhs[m] = J.rhs[m];
+      R.rhs[m] = s.f[IMPACT_B200_RHS1 + m];
     }
     rhs_march_job_grid(s.g, R, kz_batch);
     R.b0 = rb;
@@ -1628,6 +1492,8 @@ static int batch_jobs(impact_b200_batch* b) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_rhs, n * sizeof(RhsJob));
   if (e == cudaSuccess) e = cudaMemcpy(b->d_ex, ex.data(), n * sizeof(ExJob), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_rhs, rj.data(), n * sizeof(RhsJob), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_tri, n * sizeof(TriJob));
+  if (e == cudaSuccess) e = cudaMemcpy(b->d_tri, tj.data(), n * sizeof(TriJob), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(b->d_ex);
     b->d_ex = nullptr;
@@ -1636,6 +1502,7 @@ static int batch_jobs(impact_b200_batch* b) {
   b->ex_blocks = eb;
   b->ex_pblocks = pb;
   b->rhs_blocks = rb;
+  b->tri_blocks = tb;
   return 0;
 }
 
@@ -1733,6 +1600,7 @@ extern "C" int impact_b200_batch_step(impact_b200_batch* b, const impact_b200_st
   std::vector<int> its;
   if (batch_jobs(b)) return -1;
   const ExJob* EJ = b->d_ex;
+  const TriJob* TJ = b->d_tri;
   double cells = 0.0;
   for (auto* c : b->cases) cells += (double)c->s.g.n1 * c->s.g.n2 * c->s.g.n3;
   const dim3 bl(BX, BY);
@@ -1742,7 +1610,8 @@ extern "C" int impact_b200_batch_step(impact_b200_batch* b, const impact_b200_st
       b->h_sc[c] = StepScal{0.0, p[c].Re, 0.0, 1, p[c].level_pressure};
     }
     IMPACT_CUDA_CHECK(cudaMemcpyAsync(b->d_sc, b->h_sc, n * sizeof(StepScal), cudaMemcpyHostToDevice, bs));
-    k_b_dtime<<<b->ex_blocks, bl, 0, bs>>>(EJ, n);
+    const int f32 = b->precision == 1 && p[0].explicit_fp32;
+    launch_tri_batch(TRI_INTERP, f32, 1, TJ, n, b->tri_blocks, bs);  // the first substep's work fields too
     k_b_reduce<<<n, 1024, 0, bs>>>(EJ, 1, 0, 0, b->d_beta);
     prof::count(2);
     IMPACT_CUDA_CHECK(cudaMemcpyAsync(b->hbeta, b->d_beta, n * sizeof(double), cudaMemcpyDeviceToHost, bs));
@@ -1757,19 +1626,20 @@ extern "C" int impact_b200_batch_step(impact_b200_batch* b, const impact_b200_st
     IMPACT_CUDA_CHECK(cudaMemcpyAsync(b->d_sc, b->h_sc, n * sizeof(StepScal), cudaMemcpyHostToDevice, bs));
     for (int sub = 0; sub < 3; ++sub) {
       // rhs_vel and the pressure equation's right-hand side of every case, one launch per kernel
-      const int f32 = b->precision == 1 && p[0].explicit_fp32;
-      k_b_interp<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n, f32);
-      prof::count(1);
+      if (sub > 0) {
+        launch_tri_batch(TRI_INTERP, f32, 0, TJ, n, b->tri_blocks, bs);
+        prof::count(1);
+      }
       for (int m = 0; m < 3; ++m)
         IMPACT_PROF(prof::K_NL_RHS, (f32 ? (sub != 0 ? 36.0 : 32.0) : (sub != 0 ? 56.0 : 48.0)) * cells, bs,
                     launch_rhs_march_batch(m, b->d_rhs, n, b->rhs_blocks, sub, f32, bs));
-      IMPACT_PROF(prof::K_DIV2, 4.0 * 8.0 * cells, bs, (k_b_div2<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n)));
+      IMPACT_PROF(prof::K_DIV2, 4.0 * 8.0 * cells, bs, launch_tri_batch(TRI_DIV2, 0, 0, TJ, n, b->tri_blocks, bs));
       for (auto* c : b->cases)
         if (c->s.pre_wait) {  // a deferred pressure upload: wait for it at the first read
           IMPACT_CUDA_CHECK(cudaStreamWaitEvent(bs, c->s.pre_wait, 0));
           c->s.pre_wait = nullptr;
         }
-      k_b_scale_pre<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n, sub, 0);
+      k_b_scale_pre<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n, sub - 1, sub);
       prof::count(1);
       for (int c = 0; c < n; ++c) {
         init[c] = SolverScalars{};
@@ -1796,9 +1666,7 @@ extern "C" int impact_b200_batch_step(impact_b200_batch* b, const impact_b200_st
         r.b_two = res[c].b_two;
         record_solve(&st[c], sub, r);
       }
-      IMPACT_PROF(prof::K_PROJECT, 7.0 * 8.0 * cells, bs, (k_b_project<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n)));
-      k_b_scale_pre<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n, sub, 1);
-      prof::count(1);
+      IMPACT_PROF(prof::K_PROJECT, 7.0 * 8.0 * cells, bs, launch_tri_batch(TRI_PROJECT, 0, 0, TJ, n, b->tri_blocks, bs));
     }
     // mask forcing at the new time and level_pressure of every case
     bool lp = false;
@@ -1809,11 +1677,14 @@ extern "C" int impact_b200_batch_step(impact_b200_batch* b, const impact_b200_st
     }
     k_b_mask<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n);
     prof::count(1);
-    if (lp) {
-      k_b_sum<<<b->ex_blocks, bl, 0, bs>>>(EJ, n);
+    if (lp) {  // the pressure scaled back, with the partial sums of its mean
+      k_b_scale_sum<<<b->ex_blocks, bl, 0, bs>>>(EJ, n, 2);
       k_b_reduce<<<n, 1024, 0, bs>>>(EJ, 0, 1, 1, nullptr);
       k_b_sub_mean<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n);
       prof::count(3);
+    } else {
+      k_b_scale_pre<<<b->ex_pblocks, bl, 0, bs>>>(EJ, n, 2, -1);
+      prof::count(1);
     }
   }
   IMPACT_CUDA_CHECK(cudaStreamSynchronize(bs));
@@ -1845,16 +1716,16 @@ extern "C" int impact_b200_case_kernel_bench(impact_b200_case* c, int kid, int i
       double* vel[3] = {s.f[IMPACT_B200_VEL1], s.f[IMPACT_B200_VEL2], s.f[IMPACT_B200_VEL3]};
       double* nl[3] = {s.f[IMPACT_B200_NL1], s.f[IMPACT_B200_NL2], s.f[IMPACT_B200_NL3]};
       double* rhs[3] = {s.f[IMPACT_B200_RHS1], s.f[IMPACT_B200_RHS2], s.f[IMPACT_B200_RHS3]};
-      const dim3 gr = grid3(g), bl(BX, BY);
+      const TriGrid tg = tri_grid(g, sizeof(double), tri_vec(s));
       switch (kid) {
         case 10: case 11: case 12: {
           const int m = kid - 10;
           launch_rhs_march(m, g, s.c64, 2e-3, -0.01, 0.02, 1, vel[m], s.work, nl[m], rhs[m], s.stream);
           break;
         }
-        case 13: k_interp_vel3<<<gr, bl, 0, s.stream>>>(g, s.c64, vel[0], vel[1], vel[2], s.work[0], s.work[1], s.work[2]); break;
-        case 14: k_project<<<gr, bl, 0, s.stream>>>(g, s.c64, s.f[IMPACT_B200_PRE], rhs[0], rhs[1], rhs[2], vel[0], vel[1], vel[2]); break;
-        case 15: k_div2<<<gr, bl, 0, s.stream>>>(g, s.c64, rhs[0], rhs[1], rhs[2], s.f[IMPACT_B200_RES]); break;
+        case 13: launch_tri<TRI_INTERP, double, double>(g, tri_args(s, TRI_INTERP), tg, s.stream); break;
+        case 14: launch_tri<TRI_PROJECT, double, double>(g, tri_args(s, TRI_PROJECT), tg, s.stream); break;
+        case 15: launch_tri<TRI_DIV2, double, double>(g, tri_args(s, TRI_DIV2), tg, s.stream); break;
         default: return -1;
       }
       return 0;

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(MT) k_axpby(Geom g, T a, T b, const T* __restr
       if (u == 0 || k + u <= k1) {
         T r[V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) r[v] = fmaT(b, yv[u][v], mulT(a, xv[u][v]));
+        for (int v = 0; v < V; ++v) r[v] = fmaT(a, xv[u][v], mulT(b, yv[u][v]));
         stv<T, V>(z + p + u * g.nxy, r);
       }
   }

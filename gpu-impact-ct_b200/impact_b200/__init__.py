@@ -239,7 +239,7 @@ def solver_params(tol_rel=1e-8, tol_abs_inf=0.0, max_it=2000, n_sweeps=4, omega=
                   mg_bottom=4, tile_kc=0, smooth_unfused=0, bottom_cheb=0) -> SolverParams:
     """precond 0: n_sweeps damped-Jacobi sweeps; 1: multigrid V-cycle (mg_down/up/bottom sweeps).
     tile_kc: most z-planes per tile of the solver kernels (0: library default; small grids take fewer).  smooth_unfused: 1 runs
-    every V-cycle sweep as its own launch instead of one fused kernel per smoothing phase.
+    every sweep (V-cycle, JOR preconditioner) as its own launch instead of one fused kernel per phase.
     bottom_cheb: d > 0 replaces the coarsest level's Jacobi sweeps by d Chebyshev steps (fused
     schedule, coarsest level within the one-block tail)."""
     return SolverParams(tol_rel, tol_abs_inf, max_it, n_sweeps, omega, init_yes, check_every,

@@ -280,8 +280,8 @@ typedef struct {
                           of few tiles takes shallower ones, so that they fill the GPU); chosen by
                           the autotuner of the Python package, no counterpart in the reference */
   int smooth_unfused;  /* 0 (default): the sweeps of each V-cycle smoothing phase (and, before a
-                          restriction, the residual after them) run as one z-marching kernel;
-                          1: one sweep per launch.  Same results bit for bit; no counterpart in
+                          restriction, the residual after them), and the 2 to 4 sweeps of the
+                          JOR preconditioner, run as one z-marching kernel; 1: one sweep per launch.  Same results bit for bit; no counterpart in
                           the reference */
   int bottom_cheb;     /* 0 (default): the coarsest level of the V-cycle gets mg_bottom damped-Jacobi
                           sweeps, then mg_bottom more (relax_bottom, mod_solvers.f90:420-450);

@@ -1,7 +1,8 @@
 """The one-block coarse tail of the V-cycle (k_lv_tail) at the edges of its thread mapping and of
 its shared memory: levels with more columns than threads, one plane or a partial segment per
 thread, two-point axes, and tables too long to be staged.  Like every fused phase it must give the
-iterate of the one-launch-per-phase schedule (which has no tail) bit for bit."""
+iterate of the one-launch-per-phase schedule (which has no tail) bit for bit; so must the JOR
+preconditioner's fused sweeps."""
 import numpy as np
 import pytest
 
@@ -29,5 +30,20 @@ def test_coarse_tail_equals_one_launch_per_phase(gi, sw, precision):
                                                    smooth_unfused=unfused))
         out.append(g.interior(case.download("pre")).copy())
     assert np.isfinite(out[0]).all()
+    assert np.array_equal(out[0], out[1])
+    case.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("N", [(9, 9, 9), (33, 29, 41), (60, 48, 84), (65, 65, 33)], ids=lambda n: "x".join(str(v - 1) for v in n))
+@pytest.mark.parametrize("sweeps", [1, 2, 3, 4, 5])
+def test_fused_jor_preconditioner_equals_one_sweep_per_launch(sweeps, N, precision):
+    g = I.Grid(N, (1.0, 0.8, 1.3), (0, 0, int(N[0] == 33)))
+    case = I.Case(g, precision=precision)
+    case.upload("res", np.random.default_rng(32).uniform(-1.0, 1.0, g.shape))
+    out = []
+    for unfused in (1, 0):
+        case.precond("res", "pre", I.solver_params(precond=0, n_sweeps=sweeps, smooth_unfused=unfused))
+        out.append(g.interior(case.download("pre")).copy())
     assert np.array_equal(out[0], out[1])
     case.close()

@@ -3899,6 +3899,8 @@ void MixedEngine::release() {
   if (q_) cudaFree(q_);
   if (q_host_) cudaFreeHost(q_host_);
   if (oscal_) cudaFree(oscal_);
+  if (oscal_host_) cudaFreeHost(oscal_host_);
+  oscal_host_ = nullptr;
   partial_ = nullptr;
   q_ = nullptr;
   q_host_ = nullptr;
@@ -3926,6 +3928,7 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
   cudaError_t e = cudaMalloc((void**)&q_, (size_t)n * 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMallocHost((void**)&q_host_, (size_t)n * 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc((void**)&oscal_, (size_t)n * sizeof(SolverScalars));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&oscal_host_, (size_t)n * sizeof(SolverScalars));
   if (e != cudaSuccess) {
     release();
     return impact_set_error(e, "mixed engine allocation", __FILE__, __LINE__);
@@ -4004,7 +4007,6 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
   res.assign(n, SolverResult{});
   inner_its.assign(n, 0);
   std::vector<int> done(n, 0), outer_it(n, 0), retries(n, 0);
-  std::vector<SolverScalars> osc(n);
   for (int c = 0; c < n; ++c) {
     done[c] = outer[c].done;
     res[c].status = 1;
@@ -4017,14 +4019,25 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
   const KrylovJob<double>* AJ = static_cast<const KrylovJob<double>*>(AL.jobs);
   const MixJob* MJ = static_cast<const MixJob*>(ML.jobs);
   const int grid = grid_for(AL.ntiles), gm = grid_for(ML.ntiles);
+  // the cases' done flags on the device, sent when they changed.  The copies read pinned memory and
+  // nobody waits for them; the buffer is rewritten only after a wait for the stream (the residual's
+  // norms or an inner poll), which the copy before has passed.
+  bool sent = false;
   auto push_flags = [&]() -> int {
-    for (int c = 0; c < n; ++c) {
-      osc[c] = SolverScalars{};
-      osc[c].done = done[c];
+    bool same = sent;
+    for (int c = 0; c < n && same; ++c) same = oscal_host_[c].done == done[c];
+    if (same) return 0;
+    if (sent) {
+      const cudaError_t w = cudaStreamSynchronize(s_);
+      if (w != cudaSuccess) return impact_set_error(w, "mixed engine flags", __FILE__, __LINE__);
     }
-    cudaError_t e = cudaMemcpyAsync(oscal_, osc.data(), n * sizeof(SolverScalars), cudaMemcpyHostToDevice, s_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s_);  // osc is pageable and reused
+    for (int c = 0; c < n; ++c) {
+      oscal_host_[c] = SolverScalars{};
+      oscal_host_[c].done = done[c];
+    }
+    const cudaError_t e = cudaMemcpyAsync(oscal_, oscal_host_, n * sizeof(SolverScalars), cudaMemcpyHostToDevice, s_);
     if (e != cudaSuccess) return impact_set_error(e, "mixed engine flags", __FILE__, __LINE__);
+    sent = true;
     return 0;
   };
   std::vector<SolverScalars> init(n);
@@ -4088,8 +4101,6 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
       any = true;
     }
     if (!any) break;
-    rc = push_flags();
-    if (rc) return rc;
     // e from 0, not written before the first x update; rr and the norms from the residual kernel
     rc = inner_.solve(init, 2, ir, AL.ts, partial_);
     if (rc) return rc;

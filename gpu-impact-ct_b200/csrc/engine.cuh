@@ -264,6 +264,7 @@ class MixedEngine {
   double* q_ = nullptr;       // device, 4 per case
   double* q_host_ = nullptr;  // pinned
   SolverScalars* oscal_ = nullptr;  // outer scalars (only done/status are used by the kernels)
+  SolverScalars* oscal_host_ = nullptr;  // pinned
 };
 
 // collapsed product_div_grad weights of one axis: W(i, o) = sum_{a+b=o} cD(a, i) cG(b, wrap(i+a)),

@@ -74,7 +74,8 @@ struct KrylovJob {
   const T* W[3];  // collapsed product_div_grad weights, row (i-1) holds offsets -5..5
   int zuni;       // 1: every z row of W[2] is the same (uniform z spacing)
   int xuni;       // 1: every x row of W[0] is the same (uniform x spacing)
-  int vec;        // FP32: the operator of this job runs in the 4-point vector kernel
+  int vec;        // the operator of this job runs in the vector kernel
+  int vecu;       // the vector updates move 16 bytes per thread (n1 a multiple of the vector, aligned fields)
   const T* bb;
   T* phi;
   T *rr, *rh, *pp, *Ap, *Ar, *z1, *z2;
@@ -87,6 +88,7 @@ struct KrylovJob {
 struct MixJob {
   Geom g;
   int kc;
+  int vecu;  // as KrylovJob::vecu
   const double* bb;
   double* x;
   double* r64;

@@ -9,6 +9,8 @@
 //   restrict                mod_solvers.f90:588-808     k_lv_restrict
 //   interpolate             mod_solvers.f90:955-1141    k_lv_prolong
 //   product_scalar/get_norms mod_solvers.f90:2319-2470  per-tile partials + fixed-order k_efin
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -23,6 +25,8 @@
 namespace impact {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 enum EFin { EFIN_RAW = 0, EFIN_INIT, EFIN_ALPHA, EFIN_OMEGA, EFIN_NORMS, EFIN_RESET, EFIN_INIT_EXT };
 
@@ -2669,21 +2673,33 @@ __global__ void __launch_bounds__(MNT, 1) k_lv_multi(const LevelJob<T>* __restri
 // global memory, and only the warps that own cells of a level meet at its barriers.  Against one
 // block whose threads take single cells strided by the block (coefficients from global memory,
 // omega / diag and index divisions per cell), V-cycle times in us: 32x32x64 FP32 106 -> 64 (its
-// tail 79 -> 36), FP64 89 -> 78, 128x128x256 FP32 233 -> 192, 104x104x208 with 32 Chebyshev steps
-// FP32 224 -> 189, FP64 295 -> 255.  Slower here: 256 and 1024 threads, z-fastest storage with
-// 16-byte accesses (more instructions per pass on the small levels), one run-time choice of the
-// pass in place of the four instances, loads of two or four planes ahead.
+// tail 79 -> 36), FP64 89 -> 78, 128x128x256 FP32 233 -> 192.  Slower here: 256 and 1024 threads,
+// z-fastest storage with 16-byte accesses (more instructions per pass on the small levels), one
+// run-time choice of the pass in place of the four instances, loads of two or four planes ahead.
+//
+// SLAB: a cluster of up to 8 blocks shares a case.  Every level is cut into z slabs, one per block,
+// with a ghost plane at either end that the neighbours write into each other's shared memory in
+// every pass, and a pass ends with the cluster's barrier.  That barrier takes longer than the
+// warps' own, so the cut pays where many passes run on a level large enough for one SM's
+// instructions to bound it: the Chebyshev steps of a coarsest level of at least TAIL_SPLIT cells.  104x104x208, 32 steps on 13x13x26: V-cycle FP32 189 -> 160 us, FP64 255 -> 207.  With
+// Jacobi bottoms (levels halved down to a few cells) the cut is slower at every size measured:
+// 128x128x256 FP32 192 -> 199 us, FP64 290 -> 297.
 constexpr int TNT = 512;
 constexpr size_t TAIL_BYTES = 200 * 1024;     // the levels' fields
 constexpr size_t TAIL_TAB_BYTES = 22 * 1024;  // their tables (longer ones are read from global memory)
+constexpr int TAIL_CLUSTER = 8;               // most blocks per case with Chebyshev steps
+constexpr int TAIL_SPLIT = 1536;              // cells of a coarsest level from which they are used
 
 // one level inside the tail: extents, thread mapping, shared-memory offsets (elements)
 struct TailLevel {
   int n1, n2, n3, zuni;
   int ncol, len, ncs;    // columns, planes per segment, column segments
   int nthr;              // threads of the warps that own segments
+  // a level cut into z slabs (block r of the cluster: planes r P ..): planes per block; set in the
+  // kernel for its own block: first plane, planes, the blocks below and above, planes of the one below
+  int P, kb, np, lo, hi, lo_np;
   int rf[3], rc[3];      // coarsening factors from the next finer level and to the next coarser one
-  int oA, oX[2];         // fields (compact, i fastest)
+  int oA, oX[2];         // plane 0 of the fields (compact, i fastest; slabs: ghost planes -1 and P)
   int tcd[3], tcI[3];    // cdg and interpolation tables, offsets from TailJob::tab
 };
 template <typename T>
@@ -2703,13 +2719,13 @@ struct TailJob {
 // the column segment of a thread: coefficients and neighbour offsets
 template <typename T>
 struct TailCol {
-  int i, j, k0, nk;      // 1-based column, 0-based first plane, planes (0: none)
+  int i, j, k0, nk;      // 1-based column, 0-based first plane (of the slab), planes (0: none)
   int p;                 // index of (i, j, k0) in the level's compact layout
   int dW, dE, dS, dN;
   T a0, a2, b0, b2, s1;  // lateral weights, sum of the x and y diagonal parts
   T inv;                 // uniform z: omega / diag
 };
-template <typename T>
+template <typename T, bool SLAB>
 __device__ __forceinline__ TailCol<T> tail_col(const TailLevel& L, const T* __restrict__ tb, int c, T omega) {
   TailCol<T> C;
   const bool own = c < L.ncs;
@@ -2718,7 +2734,7 @@ __device__ __forceinline__ TailCol<T> tail_col(const TailLevel& L, const T* __re
   C.i = i + 1;
   C.j = j + 1;
   C.k0 = seg * L.len;
-  C.nk = own ? min(L.len, L.n3 - C.k0) : 0;
+  C.nk = own ? min(L.len, (SLAB ? L.np : L.n3) - C.k0) : 0;
   C.p = col + C.k0 * L.ncol;
   C.dW = i == 0 ? L.n1 - 1 : -1;
   C.dE = i == L.n1 - 1 ? 1 - L.n1 : 1;
@@ -2735,10 +2751,29 @@ __device__ __forceinline__ TailCol<T> tail_col(const TailLevel& L, const T* __re
   return C;
 }
 
+// the places of a slab's boundary values in the neighbours' ghost planes (field at offset o)
+template <typename T, bool SLAB>
+struct TailGhost {
+  T *lo, *hi;
+  __device__ __forceinline__ TailGhost(const TailLevel& L, T* sm, int o) {
+    if constexpr (SLAB) {
+      cg::cluster_group cl = cg::this_cluster();
+      lo = cl.map_shared_rank(sm, L.lo) + o + L.lo_np * L.ncol;  // above the last plane of the block below
+      hi = cl.map_shared_rank(sm, L.hi) + o - L.ncol;            // below the first plane of the block above
+    }
+  }
+  __device__ __forceinline__ void put(const TailLevel& L, int k, int col, T v) const {
+    if constexpr (SLAB) {
+      if (k == 0) lo[col] = v;
+      if (k == L.np - 1) hi[col] = v;
+    }
+  }
+};
+
 // One pass over a column segment.  OP 0: dst = init(A); 1: dst = sweep(A, src);
 // 2: dst = A - cdg(src); 3: a Chebyshev step, dst = xm + w (x + g z - xm) with xm = dst's old
 // value (x itself on the first step).  oS, oD: shared-memory offsets of src and dst.
-template <typename T, int OP>
+template <typename T, int OP, bool SLAB>
 __device__ __forceinline__ void tail_seg(const TailLevel& L, const TailCol<T>& C, T* sm, const T* __restrict__ tb,
                                          T omega, int oS, int oD, T w, T gam, bool first) {
   const bool zu = L.zuni != 0;
@@ -2749,24 +2784,26 @@ __device__ __forceinline__ void tail_seg(const TailLevel& L, const TailCol<T>& C
   const T* A = sm + L.oA + C.p;
   const T* s = sm + oS + C.p;
   T* d = sm + oD + C.p;
+  const TailGhost<T, SLAB> gh(L, sm, oD);
   T xm = T(0), xc = T(0);
   if (OP != 0 && C.nk > 0) {
-    xm = s[C.k0 == 0 ? wz : -sz];
+    xm = s[!SLAB && C.k0 == 0 ? wz : -sz];
     xc = s[0];
   }
   for (int k = 0; k < C.nk; ++k) {
     T cm = zm0, cc = zc0, cp = zp0;
     if (!zu) {
-      cm = cz[3 * (C.k0 + k)];
-      cc = cz[3 * (C.k0 + k) + 1];
-      cp = cz[3 * (C.k0 + k) + 2];
+      const T* c3 = cz + 3 * ((SLAB ? L.kb : 0) + C.k0 + k);
+      cm = c3[0];
+      cc = c3[1];
+      cp = c3[2];
     }
     const T diag = C.s1 + cc;
     T o;
     if (OP == 0) {
       o = jinit(A[0], omega, zu, C.inv, diag);
     } else {
-      const T zn = s[C.k0 + k + 1 == n3 ? -wz : sz];
+      const T zn = s[!SLAB && C.k0 + k + 1 == n3 ? -wz : sz];
       if (OP == 1) {
         const T r = jres(A[0], C.a0, s[C.dW], C.a2, s[C.dE], C.b0, s[C.dS], C.b2, s[C.dN], cm, xm, cp, zn);
         o = jsweep(r, xc, omega, zu, C.inv, diag);
@@ -2781,13 +2818,14 @@ __device__ __forceinline__ void tail_seg(const TailLevel& L, const TailCol<T>& C
       xc = zn;
     }
     d[0] = o;
+    gh.put(L, C.k0 + k, C.p - C.k0 * sz, o);
     A += sz;
     s += sz;
     d += sz;
   }
 }
 
-template <typename T>
+template <typename T, bool SLAB>
 __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict__ jobs,
                                                                const int* __restrict__ ts, int nj, int ntiles, T omega,
                                                                int n_down, int n_up, int n_bottom) {
@@ -2797,7 +2835,16 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
   T* const sm = reinterpret_cast<T*>(tl_raw);
   T* const stab = sm + TAIL_BYTES / sizeof(T);
   const int tid = threadIdx.x;
-  for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cb = SLAB ? (int)cluster.num_blocks() : 1;
+  // the barrier of all threads of a case, for its shared memory
+  auto meet = [&]() {
+    if constexpr (SLAB)
+      cluster.sync();
+    else
+      __syncthreads();
+  };
+  for (int b = blockIdx.x / cb; b < ntiles; b += gridDim.x / cb) {
     const TailJob<T>& TJ = jobs[find_job(ts, nj, b)];
     if (e_halted(TJ.sc)) continue;
     const int nl = TJ.nl;
@@ -2807,26 +2854,44 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
     for (int t = tid; t < TJ.ntab; t += NT) stab[t] = gt[t];
     const T* const tb = TJ.ntab > 0 ? stab : gt;
     __syncthreads();
+    if constexpr (SLAB) {
+      if (tid < nl) {  // this block's part of every level
+        TailLevel& L = lev[tid];
+        const int r = (int)cluster.block_rank(), nb = (L.n3 + L.P - 1) / L.P;  // blocks with planes
+        L.kb = r * L.P;
+        L.np = max(0, min(L.P, L.n3 - L.kb));
+        const int segs = max(1, min(L.np, NT / L.ncol));
+        L.len = max(1, (L.np + segs - 1) / segs);
+        L.ncs = L.ncol * ((L.np + L.len - 1) / L.len);
+        L.lo = r == 0 || r >= nb ? nb - 1 : r - 1;
+        L.hi = r + 1 >= nb ? 0 : r + 1;
+        L.lo_np = min(L.P, L.n3 - L.lo * L.P);
+      }
+      cluster.sync();  // and every block runs: its shared memory may be written
+    }
     // this thread's segment of a level; a level of more segments than threads walks its further
     // ones from `each`
     TailCol<T> C;
-    auto take = [&](const TailLevel& L) { C = tail_col(L, tb, tid, omega); };
+    auto take = [&](const TailLevel& L) { C = tail_col<T, SLAB>(L, tb, tid, omega); };
     auto each = [&](const TailLevel& L, auto&& f) {
       f();
       if (L.ncs > NT) {
         for (int c = tid + NT; c < L.ncs; c += NT) {
-          C = tail_col(L, tb, c, omega);
+          C = tail_col<T, SLAB>(L, tb, c, omega);
           f();
         }
-        C = tail_col(L, tb, tid, omega);
+        C = tail_col<T, SLAB>(L, tb, tid, omega);
       }
     };
     auto pass = [&](const TailLevel& L, auto op, int oS, int oD, T w, T gam, bool first) {
-      each(L, [&]() { tail_seg<T, decltype(op)::value>(L, C, sm, tb, omega, oS, oD, w, gam, first); });
+      each(L, [&]() { tail_seg<T, decltype(op)::value, SLAB>(L, C, sm, tb, omega, oS, oD, w, gam, first); });
     };
-    // barrier of the warps that own cells of level L (the others do not come here)
+    // end of a pass: the cluster's barrier, or that of the warps that own cells of level L (the others
+    // do not come here)
     auto level_sync = [&](const TailLevel& L) {
-      if (L.nthr == NT)
+      if constexpr (SLAB)
+        cluster.sync();
+      else if (L.nthr == NT)
         __syncthreads();
       else
         asm volatile("bar.sync 1, %0;\n" ::"r"(L.nthr) : "memory");
@@ -2855,13 +2920,14 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
         const int xm = fi == 0 ? F.n1 - 1 : -1, xp = fi == F.n1 - 1 ? 1 - F.n1 : 1;
         const int ym = fj == 0 ? (F.n2 - 1) * F.n1 : -F.n1, yp = fj == F.n2 - 1 ? -(F.n2 - 1) * F.n1 : F.n1;
         const int wz = (F.n3 - 1) * F.ncol;
+        const int kb = SLAB ? L.kb : 0, fb = SLAB ? F.kb : 0;
         const T* d0 = sm + oD + fi + F.n1 * fj;
         T* a = sm + L.oA + C.p;
         for (int k = 0; k < C.nk; ++k) {
-          const int fk = L.rf[2] * (C.k0 + k);
-          const T* d = d0 + F.ncol * fk;
-          a[k * L.ncol] = restrict7(d[0], d[xm], d[xp], d[ym], d[yp], d[fk == 0 ? wz : -F.ncol],
-                                    d[fk == F.n3 - 1 ? -wz : F.ncol]);
+          const int fk = L.rf[2] * (kb + C.k0 + k);
+          const T* d = d0 + F.ncol * (fk - fb);
+          a[k * L.ncol] = restrict7(d[0], d[xm], d[xp], d[ym], d[yp], d[!SLAB && fk == 0 ? wz : -F.ncol],
+                                    d[!SLAB && fk == F.n3 - 1 ? -wz : F.ncol]);
         }
       });
     };
@@ -2880,21 +2946,25 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
         const T* xc = sm + oC;
         const T* xf = sm + oF + C.p;
         T* out = sm + oO + C.p;
+        const TailGhost<T, SLAB> gh(L, sm, oO);
         for (int k = 0; k < C.nk; ++k) {
-          const int kk = C.k0 + k + 1;
+          const int kk = (SLAB ? L.kb : 0) + C.k0 + k + 1;
           int zl, zh;
           bool mz;
           bracket(kk, L.rc[2], G.n3, zl, zh, mz);
           const T wz0 = cI3[2 * kk], wz1 = cI3[2 * kk + 1];
-          const T* pl = xc + (zl - 1) * G.ncol;
-          const T* ph = xc + (zh - 1) * G.ncol;
+          // a slab's plane above its last one is its ghost plane
+          const T* pl = xc + (zl - 1 - (SLAB ? G.kb : 0)) * G.ncol;
+          const T* ph = SLAB ? pl + (mz ? G.ncol : 0) : xc + (zh - 1) * G.ncol;
           const T Z0 = pmix(mz, wz0, pl[o0], wz1, ph[o0]);
           const T Z1 = pmix(mz, wz0, pl[o1], wz1, ph[o1]);
           const T Z2 = pmix(mz, wz0, pl[o2], wz1, ph[o2]);
           const T Z3 = pmix(mz, wz0, pl[o3], wz1, ph[o3]);
           const T Yl = pmix(my, wy0, Z0, wy1, Z1);
           const T Yh = pmix(my, wy0, Z2, wy1, Z3);
-          out[k * L.ncol] = xf[k * L.ncol] + pmix(mx, wx0, Yl, wx1, Yh);
+          const T v = xf[k * L.ncol] + pmix(mx, wx0, Yl, wx1, Yh);
+          out[k * L.ncol] = v;
+          gh.put(L, C.k0 + k, C.p - C.k0 * L.ncol, v);
         }
       });
     };
@@ -2904,7 +2974,7 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
       const Geom g = TJ.g;
       const T* __restrict__ src = TJ.A;
       each(L, [&]() {
-        const T* s = src + off(g, C.i, C.j, C.k0 + 1);
+        const T* s = src + off(g, C.i, C.j, (SLAB ? L.kb : 0) + C.k0 + 1);
         for (int k = 0; k < C.nk; ++k) cp_async1(sm + L.oA + C.p + k * L.ncol, s + k * g.nxy);
       });
     }
@@ -2913,14 +2983,14 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
     for (int q = 0; q + 1 < nl; ++q) {  // relax_restrict
       const TailLevel& L = lev[q];
       unsigned cur = 0;
-      if (tid < L.nthr) {
+      if (SLAB || tid < L.nthr) {
         smooth(L, cur, 1, n_down);
         level_sync(L);
         pass(L, std::integral_constant<int, 2>{}, L.oX[cur], L.oX[cur ^ 1], T(0), T(0), false);
       }
       cur = (n_down - 1) & 1;  // the same in the warps without cells
       put(q, cur);
-      __syncthreads();
+      meet();  // the residual is complete
       take(lev[q + 1]);
       restrict_down(L, lev[q + 1], L.oX[cur ^ 1]);
     }
@@ -2929,9 +2999,15 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
       unsigned cur = 0;
       if (TJ.cheb > 0) {  // Chebyshev semi-iteration on the coarsest level, from x = 0
         const int steps = TJ.cheb;
-        if (tid < L.nthr) {
+        if (SLAB || tid < L.nthr) {
           each(L, [&]() {
-            for (int k = 0; k < C.nk; ++k) sm[L.oX[0] + C.p + k * L.ncol] = sm[L.oX[1] + C.p + k * L.ncol] = T(0);
+            for (int o : {L.oX[0], L.oX[1]}) {
+              const TailGhost<T, SLAB> gh(L, sm, o);
+              for (int k = 0; k < C.nk; ++k) {
+                sm[o + C.p + k * L.ncol] = T(0);
+                gh.put(L, C.k0 + k, C.p - C.k0 * L.ncol, T(0));
+              }
+            }
           });
           const T gam = TJ.cgam, s2 = TJ.csig2;
           T w = T(1);
@@ -2944,19 +3020,19 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
         }
         cur = steps & 1;
       } else {  // relax_bottom: n_bottom sweeps from an init sweep, n_bottom more
-        if (tid < L.nthr) smooth(L, cur, 1, 2 * n_bottom);
+        if (SLAB || tid < L.nthr) smooth(L, cur, 1, 2 * n_bottom);
         cur = (2 * n_bottom - 1) & 1;
       }
       put(nl - 1, cur);
     }
     for (int q = nl - 2; q >= 0; --q) {  // interpolate_relax
       const TailLevel& L = lev[q];
-      __syncthreads();  // level q + 1's iterate is complete
+      meet();  // level q + 1's iterate is complete
       unsigned cur = get(q);
       take(L);
       prolong_up(L, lev[q + 1], L.oX[cur], L.oX[cur ^ 1], lev[q + 1].oX[get(q + 1)]);
       cur ^= 1;
-      if (tid < L.nthr && n_up > 0) {
+      if ((SLAB || tid < L.nthr) && n_up > 0) {
         level_sync(L);
         unsigned c = cur;
         smooth(L, c, 0, n_up);
@@ -2969,12 +3045,12 @@ __global__ void __launch_bounds__(TNT, 1) k_lv_tail(const TailJob<T>* __restrict
       T* __restrict__ dst = TJ.B;
       const int o = L.oX[get(0)];
       each(L, [&]() {
-        T* d = dst + off(g, C.i, C.j, C.k0 + 1);
+        T* d = dst + off(g, C.i, C.j, (SLAB ? L.kb : 0) + C.k0 + 1);
 #pragma unroll 4
         for (int k = 0; k < C.nk; ++k) d[k * g.nxy] = sm[o + C.p + k * L.ncol];
       });
     }
-    __syncthreads();  // shared memory is rewritten by the next case
+    meet();  // shared memory is rewritten by the next case; no block leaves while another writes to it
   }
 }
 
@@ -3070,8 +3146,10 @@ void ax_attributes() {
                                occ(k_kr_ax64v<2>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<3>, AXD_NT, axd_smem_bytes())});
   g_axs32_grid = nsm * occ(k_kr_ax32<1>, AXNT, axa_smem_bytes());
   g_axs64_grid = nsm * occ(k_kr_ax<double, 1>, AXNT, ax_smem_bytes<double>());
-  cudaFuncSetAttribute(k_lv_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
-  cudaFuncSetAttribute(k_lv_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
+  cudaFuncSetAttribute(k_lv_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
+  cudaFuncSetAttribute(k_lv_tail<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
+  cudaFuncSetAttribute(k_lv_tail<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
+  cudaFuncSetAttribute(k_lv_tail<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
 #define IMPACT_MULTI_ATTR(T, N, I, R)                                                                           \
   cudaFuncSetAttribute(k_lv_multi<T, N, I, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
                        (int)multi_smem_bytes<T, N, I, R>());                                                    \
@@ -3541,8 +3619,9 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       if (first >= 0 && (nlev[c] - first >= 2 || p_.bottom_cheb > 0)) lt[c] = first;
     }
   }
-  // the tail of case c from level lt on: level descriptions and the run of tables that holds theirs
-  auto tail_job = [&](int c, int lt0, int nlv, int variant) {
+  // the tail of case c from level lt on: level descriptions and the run of tables that holds theirs;
+  // cut into slabs for cb > 1 blocks (nl = 0: that layout does not fit in a block's shared memory)
+  auto tail_job = [&](int c, int lt0, int nlv, int variant, int cb) {
     TailJob<T> job{};
     const MGData<T>& mg = *cs[c].mg;
     const LevelJob<T> first = lvjob(c, lt0, variant);
@@ -3555,11 +3634,15 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     const Geom& gl = mg.lv[nlv - 1].g;
     const long long ntab = (mg.lv[nlv - 1].cI[2] + 2 * (gl.n3 + 2)) - job.tab;
     job.ntab = ntab > 0 && ntab * (long long)sizeof(T) <= (long long)TAIL_TAB_BYTES ? (int)ntab : 0;
-    int o = 0;
+    if (cb > 1)  // planes per block, so that a slab's coarse planes are the same block's slab of the next level
+      for (int q = job.nl - 1; q >= 0; --q)
+        job.lv[q].P = q == job.nl - 1 ? (gl.n3 + cb - 1) / cb : mg.lv[lt0 + q].ratio[2] * job.lv[q + 1].P;
+    long long o = 0;
     for (int q = 0; q < job.nl; ++q) {
       const MGLevel<T>& M = mg.lv[lt0 + q];
       TailLevel& L = job.lv[q];
-      const int m = M.g.n1 * M.g.n2 * M.g.n3;
+      const int gh = cb > 1 ? M.g.n1 * M.g.n2 : 0;
+      const int m = cb > 1 ? gh * L.P : M.g.n1 * M.g.n2 * M.g.n3;
       L.n1 = M.g.n1;
       L.n2 = M.g.n2;
       L.n3 = M.g.n3;
@@ -3569,10 +3652,10 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       L.len = (L.n3 + segs - 1) / segs;
       L.ncs = L.ncol * ((L.n3 + L.len - 1) / L.len);
       L.nthr = std::min(TNT, (L.ncs + 31) / 32 * 32);
-      L.oA = o;
-      L.oX[0] = o + m;
-      L.oX[1] = o + 2 * m;
-      o += 3 * m;
+      L.oA = (int)o;
+      L.oX[0] = (int)o + m + gh;
+      L.oX[1] = (int)o + 2 * m + 3 * gh;
+      o += 3LL * m + 4 * gh;
       for (int a = 0; a < 3; ++a) {
         L.rf[a] = lt0 + q > 0 ? mg.lv[lt0 + q - 1].ratio[a] : 1;
         L.rc[a] = M.ratio[a];
@@ -3580,8 +3663,26 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
         L.tcI[a] = (int)(M.cI[a] - job.tab);
       }
     }
+    for (int q = 0; cb > 1 && q < job.nl; ++q)
+      if (job.lv[q].P * cb < job.lv[q].n3 || o > (long long)(TAIL_BYTES / sizeof(T))) job.nl = 0;
     return job;
   };
+  tail_blocks_ = 1;
+  if (p_.bottom_cheb > 0) {
+    int ntails = 0;
+    bool want = false;
+    for (int c = 0; c < n; ++c) {
+      if (lt[c] < 0) continue;
+      const Geom& gl = cs[c].mg->lv[nlev[c] - 1].g;
+      ++ntails;
+      want |= gl.n1 * gl.n2 * gl.n3 >= TAIL_SPLIT;
+    }
+    for (int cb = TAIL_CLUSTER; want && cb > 1 && tail_blocks_ == 1; cb /= 2) {
+      bool ok = ntails * cb <= device_sms();
+      for (int c = 0; ok && c < n; ++c) ok = lt[c] < 0 || tail_job(c, lt[c], nlev[c], 0, cb).nl > 0;
+      if (ok) tail_blocks_ = cb;
+    }
+  }
   auto in_lists = [&](int c, int g) { return lt[c] < 0 || g < lt[c]; };
   if (use_mg) {
     // fused smoothing phases for the sweep counts that have kernels
@@ -3612,7 +3713,7 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
         if (lt[c] < 0) {
           bot.push_back({c, nlev[c] - 1});
         } else {
-          TailJob<T> job = tail_job(c, lt[c], nlev[c], v);
+          TailJob<T> job = tail_job(c, lt[c], nlev[c], v, tail_blocks_);
           if (p_.bottom_cheb > 0) {
             const double lo = std::max(1e-6, std::min(1.0, cs[c].mg->lv[nlev[c] - 1].lmin));
             const double sg = (2.0 - lo) / (2.0 + lo);
@@ -3730,6 +3831,23 @@ void launch_multi_post(int sweeps, bool fast, const LevelJob<T>* J, const DevLis
 }
 
 template <typename T>
+void launch_tail(int blocks, const DevList& L, T om, int n_down, int n_up, int n_bottom, cudaStream_t s) {
+  cudaLaunchAttribute at[1] = {};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(L.ntiles * blocks);
+  cfg.blockDim = dim3(TNT);
+  cfg.dynamicSmemBytes = TAIL_BYTES + TAIL_TAB_BYTES;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = blocks > 1;
+  cudaLaunchKernelEx(&cfg, blocks > 1 ? k_lv_tail<T, true> : k_lv_tail<T, false>, static_cast<const TailJob<T>*>(L.jobs),
+                     L.ts, L.njobs, L.ntiles, om, n_down, n_up, n_bottom);
+}
+
+template <typename T>
 void Engine<T>::enqueue_phase(const Phase& ph) {
   const DevList& L = arena_.lists[ph.list];
   if (L.ntiles == 0) return;
@@ -3772,10 +3890,9 @@ void Engine<T>::enqueue_phase(const Phase& ph) {
     case PH_JOR:  // n_sweeps 2 .. 4
       IMPACT_PROF(prof::K_MG_SWEEP, 2 * sz * c, s, launch_multi_jor<T>(p_.n_sweeps, fast_[ph.list] != 0, J, L, om, s));
       break;
-    case PH_TAIL:  // one block per case; bytes: read the first level's right-hand side, write its iterate
+    case PH_TAIL:  // one block or cluster per case; bytes: read the first level's right-hand side, write its iterate
       IMPACT_PROF(prof::K_MG_TAIL, 2 * sz * c, s,
-                  (k_lv_tail<T><<<L.ntiles, TNT, TAIL_BYTES + TAIL_TAB_BYTES, s>>>(static_cast<const TailJob<T>*>(L.jobs), L.ts, L.njobs,
-                                                                  L.ntiles, om, p_.mg_down, p_.mg_up, p_.mg_bottom)));
+                  launch_tail<T>(tail_blocks_, L, om, p_.mg_down, p_.mg_up, p_.mg_bottom, s));
       break;
     default:
       break;

@@ -144,7 +144,7 @@ struct Phase {
 // PH_PRE: init + (mg_down - 1) sweeps + residual in one kernel; PH_POST: mg_up sweeps in one
 // kernel (after a PH_PROLONG with flip = 1, which writes its result into C); for 2 or 3 sweeps
 // PH_JOR: the JOR preconditioner's init sweep and n_sweeps - 1 sweeps in one kernel
-// PH_TAIL: the coarsest levels of every case of the list in one block per case (k_lv_tail)
+// PH_TAIL: the coarsest levels of every case of the list in one block or cluster per case (k_lv_tail)
 enum { PH_INIT = 0, PH_SWEEP, PH_COPY, PH_RESID, PH_RESTRICT, PH_PROLONG, PH_PRE, PH_POST, PH_JOR, PH_TAIL };
 
 // device arena of job lists built on the host
@@ -223,6 +223,7 @@ class Engine {
   // the profiler)
   std::vector<double> cells_, cells_f_, cells_c_;
   std::vector<char> fast_;  // per list: every job vectorised with uniform z (k_lv_fast)
+  int tail_blocks_ = 1;     // blocks per coarse tail: 1, or a cluster cut into z slabs
   int kr_vec_ = 0;          // FP32 Krylov list: jobs in the vector kernel -- 0 none, 1 all, 2 some
 };
 

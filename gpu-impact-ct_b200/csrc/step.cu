@@ -221,7 +221,6 @@ __device__ __forceinline__ int ex_pjob(const ExJob* __restrict__ jobs, int nj, i
 __constant__ double RKA_D[3] = {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
 __constant__ double RKB_D[3] = {0.0, -17.0 / 60.0, -5.0 / 12.0};
 
-// one block per case: out = dscal[slot] of the case
 // one block per case: the case's dscal[slot], or out[case] when out is given
 __global__ void __launch_bounds__(1024) k_b_reduce(const ExJob* __restrict__ jobs, int is_max, int slot, int only_lp,
                                                    double* __restrict__ out) {

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import impact_b200 as I
+from impact_b200 import geometry as G
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +48,31 @@ def test_fused_jor_preconditioner_equals_one_sweep_per_launch(sweeps, N, precisi
         out.append(g.interior(case.download("pre")).copy())
     assert np.array_equal(out[0], out[1])
     case.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [(26, 26, 22), (38, 38, 10), (26, 26, 34), (10, 38, 38)], ids=lambda n: "%dx%dx%d" % n)
+def test_chebyshev_tail_cut_into_slabs_equals_one_block(n, precision):
+    """Alone, a case's Chebyshev tail is cut into z slabs over a cluster of blocks (here with a short
+    last slab, fewer planes than blocks, two levels in FP32); in a batch of more tails than half the
+    device's 148 SMs every tail runs in one block.  Both must give the same step bit for bit."""
+    def case():
+        g = I.Grid(tuple(k + 1 for k in n), tuple(k / 26.0 for k in n))
+        c = I.Case(g, precision=precision)
+        c.set_labels(G.straight_vessel(g))
+        return c
+    p = I.step_params(Re=200.0, U0=1.0, tol_rel=1e-8, omega=0.8, precond=1, mg_down=3, mg_up=3, mg_bottom=3,
+                      max_it=200 if precision == 0 else 40, inner_tol_rel=3e-3, bottom_cheb=12)
+    fields = ("vel1", "vel2", "vel3", "pre")
+    one = case()
+    one.step(p, 2)
+    made = [case() for _ in range(80)]
+    batch = I.Batch(made)
+    for _ in range(2):
+        batch.step([p] * len(made))
+    for f in fields:
+        want = one.download(f)
+        assert np.isfinite(want).all()
+        assert np.array_equal(made[0].download(f), want) and np.array_equal(made[-1].download(f), want), f
+    batch.close()
+    one.close()

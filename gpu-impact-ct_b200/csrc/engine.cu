@@ -1200,29 +1200,41 @@ __global__ void __launch_bounds__(AXNT, 3) k_kr_ax32(const KrylovJob<float>* __r
 // The FP32 operator on lists whose grids have n1 divisible by 4 and uniform x and z spacing
 // (every row of W[0] and of W[2] the same): the same collapsed 11-point product_div_grad as
 // k_kr_ax32, with the center weights of the three axes combined into one and every thread
-// owning one 16-byte vector of 4 consecutive x points of one row.
+// owning one 16-byte vector of 4 consecutive x points of two neighbouring rows.
 //
-// A block of 8 x 8 threads owns one 32 x 8-column tile over kc planes.  Each plane of the tile
-// with its 5-wide halo is staged by 16-byte cp.async into a ring of AXV_R slots (48 x 18 floats:
-// columns i0-8 .. i0+39, rows j0-5 .. j0+12; at the box ends each chunk from its periodic image),
-// together with the plane's inner-product partners (the tile's 32 x 8 points).  x neighbours come
-// from the thread's row of the slot (5 vectors), y neighbours from the 10 other rows (one vector
-// each).  The z values k-5 .. k+AXV_B+4 of the 4 points stay in a register window of vectors
-// moved on by AXV_B planes per step; the window's new planes are 16-byte loads from global
-// memory issued one step ahead.  The arithmetic runs on packed FP32 pairs (fma.rn.f32x2: two
-// IEEE fmas per instruction), the per-plane inner-product terms are summed in FP32 and added
-// in FP64.  The ring holds two groups of AXV_B planes: a step computes on one while the
-// next is in flight (35.8 KB of shared memory and 166 registers: 6 blocks per SM).
+// A block of 8 x 8 threads owns one 32 x 16-column tile over kc planes.  The 5-wide halo of each
+// plane of the tile is staged by 16-byte cp.async into a ring of AXV_R slots (48 x 26 floats:
+// columns i0-8 .. i0+39, rows j0-5 .. j0+20; at the box ends each chunk from its periodic image),
+// together with the plane's inner-product partners (the tile's 32 x 16 points).  The z values
+// k-5 .. k+AXV_B+4 of the thread's points stay in a register window of vectors moved on by AXV_B
+// planes per step; the window's new planes are 16-byte loads from global memory issued one step
+// ahead, and the tile's own points of a slot are written there from the window, so that they
+// cross from L2 once.  x neighbours come from the thread's rows of the slot (4 vectors each), y
+// neighbours from 10 other rows (one vector each, shared by the two rows).  The arithmetic runs on
+// packed FP32 pairs (fma.rn.f32x2: two IEEE fmas per instruction), the per-plane inner-product
+// terms are summed in FP32 and added in FP64.  The ring holds two groups of AXV_B planes: a step
+// computes on one while the next is in flight (42 KB of shared memory and 242 registers: 4 blocks
+// per SM).
+//
+// What bounds it: reads from L2 (1.4 of halo, 1 of window and 1 of partners per point, 1 written)
+// and the shared-memory loads (10 vectors per 4 points).  Operator of a 384 x 384 x 768 grid in us
+// (its compulsory bytes take 208): one row per thread and the whole plane staged 490, the own
+// points from the window 455, two rows 423, both 385; 256 x 256 x 512 161 -> 132, 128 x 128 x 256
+// 29 -> 23.  Slower: three rows (spills), steps of 1 or 3 planes, rings of three groups, fewer
+// registers for a fifth block; 32 x 32 tiles of 128 threads are 3 % faster there and 10 % slower
+// on 104 x 104 x 208.
 constexpr int AXV_TX = ETX / 4, AXV_NT = AXV_TX * ETY;   // 8 x 8 threads, 4 columns each
 constexpr int AXV_HX = 8;                                // staged columns left of the tile
 constexpr int AXV_W = ETX + 16;                          // staged row: 8 + 32 + 8 (5 needed each side)
-constexpr int AXV_H = ETY + 10;                          // staged rows
+constexpr int AXV_NR = 2;                                // rows per thread
+constexpr int AXV_Y = AXV_NR * ETY;                      // rows per tile
+constexpr int AXV_H = AXV_Y + 10;                        // staged rows
 constexpr int AXV_CR = AXV_W / 4;                        // 16-byte chunks per row
 constexpr int AXV_NCH = AXV_CR * AXV_H;                  // chunks per plane
 constexpr int AXV_PER = (AXV_NCH + AXV_NT - 1) / AXV_NT; // chunks per thread and plane
 constexpr int AXV_PLANE = AXV_W * AXV_H;                 // floats per slot
-constexpr int AXV_PP = ETX * ETY;                        // partner floats per slot
-constexpr int AXV_B = 4;                                 // planes per step
+constexpr int AXV_PP = ETX * AXV_Y;                      // partner floats per slot
+constexpr int AXV_B = 2;                                 // planes per step
 constexpr int AXV_G = 2;                                 // groups of AXV_B planes in the ring
 constexpr int AXV_R = AXV_B * AXV_G;                     // ring slots
 constexpr int AXV_ZW = AXV_B + 10;                       // z window (planes t-5 .. t+AXV_B+4)
@@ -1233,7 +1245,7 @@ __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpre
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 template <int MODE>
-__global__ void __launch_bounds__(AXV_NT, 5) k_kr_ax32v(const KrylovJob<float>* __restrict__ jobs,
+__global__ void __launch_bounds__(AXV_NT, 4) k_kr_ax32v(const KrylovJob<float>* __restrict__ jobs,
                                                         const int* __restrict__ ts, int nj, int ntiles,
                                                         double* __restrict__ partial) {
   static_assert(MODE >= 0 && MODE <= 2, "FP32 operator modes: 0 residual, 1 alpha, 2 omega");
@@ -1244,53 +1256,62 @@ __global__ void __launch_bounds__(AXV_NT, 5) k_kr_ax32v(const KrylovJob<float>* 
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = tx + AXV_TX * ty;
   const int cx = AXV_HX + 4 * tx;   // the thread's first column in a staged row
-  const int pq = ty * ETX + 4 * tx;  // the thread's vector in a partner slot
+  const int pq = AXV_NR * ty * ETX + 4 * tx;  // the thread's vector in a partner slot
   for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
     const int q = find_job(ts, nj, b);
     const KrylovJob<float>& J = jobs[q];
     const SolverScalars* sc = J.sc;
     if (!J.vec || (MODE == 0 ? (sc->done != 0) : e_halted(sc))) continue;  // the others: k_kr_ax32
     const Geom g = J.g;
-    const int ntx = (g.n1 + ETX - 1) / ETX, nty = (g.n2 + ETY - 1) / ETY;
+    const int ntx = (g.n1 + ETX - 1) / ETX, nty = (g.n2 + AXV_Y - 1) / AXV_Y;
     const int t0 = b - ts[q];
     const int ta = t0 % ntx, tr = t0 / ntx, tc = tr / nty;
-    const int i0 = ta * ETX + 1, j0 = (tr - tc * nty) * ETY + 1;
+    const int i0 = ta * ETX + 1, j0 = (tr - tc * nty) * AXV_Y + 1;
     const int k0 = tc * J.kc + 1, k1 = min(g.n3, k0 + J.kc - 1);
     const int nk = k1 - k0 + 1;
-    const int i = i0 + 4 * tx, j = j0 + ty;
-    const bool act = i <= g.n1 && j <= g.n2;  // n1 % 4 == 0: the 4 columns are valid together
+    const int i = i0 + 4 * tx, j = j0 + AXV_NR * ty;
+    const bool in_x = i <= g.n1;  // n1 % 4 == 0: the 4 columns are valid together
+    bool act[AXV_NR];             // (a second row past the last one holds its image, row 1, for the first)
+#pragma unroll
+    for (int r = 0; r < AXV_NR; ++r) act[r] = in_x && j + r <= g.n2;
     const float* __restrict__ x = MODE == 0 ? J.phi : (MODE == 1 ? J.z1 : J.z2);
     float* __restrict__ out = MODE == 0 ? J.rr : (MODE == 1 ? J.Ap : J.Ar);
     const float* __restrict__ d1 = MODE == 1 ? J.rh : J.rr;
     const long long nxy = g.nxy;
     // weights: x and z uniform (first rows), y of this thread's row; the three center weights
     // combined
-    float wx[AXW], wy[AXW], wz[AXW];
-    const int jr = j <= g.n2 ? j : 1;
+    float wx[AXW], wy[AXV_NR][AXW], wz[AXW], wc[AXV_NR];
+    int own[AXV_NR];  // in-plane offsets of the thread's vectors
 #pragma unroll
     for (int l = 0; l < AXW; ++l) {
       wx[l] = __ldg(J.W[0] + l);
-      wy[l] = __ldg(J.W[1] + (size_t)(jr - 1) * AXW + l);
       wz[l] = __ldg(J.W[2] + l);
     }
-    const float wc = __fadd_rn(__fadd_rn(wx[5], wy[5]), wz[5]);
+#pragma unroll
+    for (int r = 0; r < AXV_NR; ++r) {
+      const int jr = j + r <= g.n2 ? j + r : 1;
+#pragma unroll
+      for (int l = 0; l < AXW; ++l) wy[r][l] = __ldg(J.W[1] + (size_t)(jr - 1) * AXW + l);
+      wc[r] = __fadd_rn(__fadd_rn(wx[5], wy[r][5]), wz[5]);
+      own[r] = (in_x ? i + 3 : 4) + g.nx * (jr + 3);
+    }
     // this thread's chunks of a staged plane: chunk cq = tid + e*AXV_NT holds columns
     // i0-8+4(cq%12) .. +3 of row j0-5+cq/12.  The points of the tile read columns
     // i0-5 .. min(i0+31, n1)+5 and rows j0-5 .. min(j0+7, n2)+5; cb[e] is the chunk's in-plane
     // offset, -1 for a chunk nothing needs.  A chunk starts at a column = 1 (mod 4) and n1 % 4 == 0,
     // so a chunk outside 1..n1 lies whole in one periodic image (n1 >= 8): every chunk, at the box
     // ends too, is one 16-byte copy from its image.
-    const int ilast = min(i0 + ETX - 1, g.n1) + 5, jlast = min(j0 + ETY - 1, g.n2) + 5;
+    const int ilast = min(i0 + ETX - 1, g.n1) + 5, jlast = min(j0 + AXV_Y - 1, g.n2) + 5;
     int cb[AXV_PER];
 #pragma unroll
     for (int e = 0; e < AXV_PER; ++e) {
       const int cq = tid + e * AXV_NT;
       const int r = cq / AXV_CR, c0 = (cq % AXV_CR) * 4;
       const int jj = j0 - 5 + r, ii = i0 - AXV_HX + c0;
-      const bool need = cq < AXV_NCH && jj <= jlast && ii + 3 >= i0 - 5 && ii <= ilast;
+      const bool mine = c0 >= AXV_HX && c0 < AXV_HX + ETX && ii <= g.n1 && r >= 5 && r < 5 + AXV_Y && jj <= g.n2;
+      const bool need = cq < AXV_NCH && jj <= jlast && ii + 3 >= i0 - 5 && ii <= ilast && !mine;
       cb[e] = need ? (wrapi(ii, g.n1) + 3) + g.nx * (wrapi(jj, g.n2) + 3) : -1;
     }
-    const int own = (act ? i + 3 : 4) + g.nx * (jr + 3);  // in-plane offset of the thread's vector
     auto zoff = [&](int k) -> long long {  // plane k (periodic) + 3 ghost planes
       return (long long)((k < 1 ? k + g.n3 : (k > g.n3 ? k - g.n3 : k)) + 3) * nxy;
     };
@@ -1307,7 +1328,9 @@ __global__ void __launch_bounds__(AXV_NT, 5) k_kr_ax32v(const KrylovJob<float>* 
 #pragma unroll
           for (int e = 0; e < AXV_PER; ++e)
             if (cb[e] >= 0) cp_async16(dst + e * AXV_NT * 4, src + cb[e]);
-          if (MODE != 0 && act) cp_async16(pring + (size_t)(t % AXV_R) * AXV_PP + pq, d1 + zo + own);
+#pragma unroll
+          for (int r = 0; r < AXV_NR; ++r)
+            if (MODE != 0 && act[r]) cp_async16(pring + (size_t)(t % AXV_R) * AXV_PP + pq + r * ETX, d1 + zo + own[r]);
         }
       }
       cp_commit();
@@ -1316,97 +1339,131 @@ __global__ void __launch_bounds__(AXV_NT, 5) k_kr_ax32v(const KrylovJob<float>* 
 #pragma unroll
     for (int gi = 0; gi < AXV_G - 1; ++gi) stage_group(gi);
     // z window: planes k0-5 .. k0+AXV_B+4
-    float4 win[AXV_ZW];
+    float4 win[AXV_NR][AXV_ZW];
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int l = 0; l < AXV_ZW; ++l) win[l] = act ? ldg4(x + zoff(k0 - 5 + l) + own) : zero4;
+    for (int l = 0; l < AXV_ZW; ++l)
+#pragma unroll
+      for (int r = 0; r < AXV_NR; ++r) win[r][l] = in_x ? ldg4(x + zoff(k0 - 5 + l) + own[r]) : zero4;
+    // plane t of the tile's own points (window place l) into its slot
+    auto publish = [&](int t, int l) {
+      if (t < nk)
+#pragma unroll
+        for (int r = 0; r < AXV_NR; ++r)
+          if (act[r])
+            *reinterpret_cast<float4*>(ring + (size_t)(t % AXV_R) * AXV_PLANE + (AXV_NR * ty + r + 5) * AXV_W + cx) = win[r][l];
+    };
+#pragma unroll
+    for (int u = 0; u < AXV_B; ++u) publish(u, 5 + u);
     double v0 = 0.0, v1 = 0.0;
-    float* o = out + (long long)(k0 + 3) * nxy + own;
+    float* o = out + (long long)(k0 + 3) * nxy;
     const int nsteps = (nk + AXV_B - 1) / AXV_B;
     for (int s = 0; s < nsteps; ++s) {
       const int tb = s * AXV_B;
       cp_wait<AXV_G - 2>();  // this thread's copies of the step's group have landed
       __syncthreads();       // everybody's have; the previous step's group is free
       stage_group(s + AXV_G - 1);
-      // the next step's window planes
-      float4 nw[AXV_B];
-      const bool more = act && tb + AXV_B < nk;
 #pragma unroll
-      for (int u = 0; u < AXV_B; ++u) nw[u] = more ? ldg4(x + zoff(k0 + tb + AXV_B + 5 + u) + own) : zero4;
+      for (int u = 0; u < AXV_B; ++u) publish(tb + AXV_B + u, 5 + AXV_B + u);
+      // the next step's window planes
+      float4 nw[AXV_NR][AXV_B];
+      const bool more = tb + AXV_B < nk;
+#pragma unroll
+      for (int u = 0; u < AXV_B; ++u)
+#pragma unroll
+        for (int r = 0; r < AXV_NR; ++r)
+          nw[r][u] = more && in_x ? ldg4(x + zoff(k0 + tb + AXV_B + 5 + u) + own[r]) : zero4;
 #pragma unroll
       for (int u = 0; u < AXV_B; ++u) {
         const int t = tb + u;
         if (t < nk) {
           const float* sp = ring + (size_t)(t % AXV_R) * AXV_PLANE;
-          // x: the thread's row, columns cx-8 .. cx+11 (own vector at 8..11)
-          float xv[20];
-#pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            const float4 v = lds4(sp + (ty + 5) * AXV_W + cx - 8 + 4 * m);
-            xv[4 * m] = v.x;
-            xv[4 * m + 1] = v.y;
-            xv[4 * m + 2] = v.z;
-            xv[4 * m + 3] = v.w;
-          }
           // packed FP32 pairs (points 0,1 and 2,3; each lane one IEEE fma, the order of the
           // scalar chains): center, x (odd offsets from the aligned pairs of the row, even ones
           // per lane), y and z, then (x + y) + z
-          const float4 cc = win[u + 5];
-          float2 a01 = __fmul2_rn(make_float2(wc, wc), make_float2(cc.x, cc.y));
-          float2 a23 = __fmul2_rn(make_float2(wc, wc), make_float2(cc.z, cc.w));
+          float2 a01[AXV_NR], a23[AXV_NR], y01[AXV_NR], y23[AXV_NR];
 #pragma unroll
-          for (int l = 0; l < AXW; ++l) {
-            if (l == 5) continue;
-            if (l & 1) {
-              const float2 w2 = make_float2(wx[l], wx[l]);
-              a01 = __ffma2_rn(w2, make_float2(xv[3 + l], xv[4 + l]), a01);
-              a23 = __ffma2_rn(w2, make_float2(xv[5 + l], xv[6 + l]), a23);
-            } else {
-              a01.x = fmaT(wx[l], xv[3 + l], a01.x);
-              a01.y = fmaT(wx[l], xv[4 + l], a01.y);
-              a23.x = fmaT(wx[l], xv[5 + l], a23.x);
-              a23.y = fmaT(wx[l], xv[6 + l], a23.y);
+          for (int r = 0; r < AXV_NR; ++r) {
+            // x: the row's columns cx-8 .. cx+11 (own vector at 8..11)
+            float xv[20];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+              const float4 v = m == 2 ? win[r][u + 5] : lds4(sp + (AXV_NR * ty + r + 5) * AXV_W + cx - 8 + 4 * m);
+              xv[4 * m] = v.x;
+              xv[4 * m + 1] = v.y;
+              xv[4 * m + 2] = v.z;
+              xv[4 * m + 3] = v.w;
+            }
+            const float2 w0 = make_float2(wc[r], wc[r]);
+            a01[r] = __fmul2_rn(w0, make_float2(xv[8], xv[9]));
+            a23[r] = __fmul2_rn(w0, make_float2(xv[10], xv[11]));
+#pragma unroll
+            for (int l = 0; l < AXW; ++l) {
+              if (l == 5) continue;
+              if (l & 1) {
+                const float2 w2 = make_float2(wx[l], wx[l]);
+                a01[r] = __ffma2_rn(w2, make_float2(xv[3 + l], xv[4 + l]), a01[r]);
+                a23[r] = __ffma2_rn(w2, make_float2(xv[5 + l], xv[6 + l]), a23[r]);
+              } else {
+                a01[r].x = fmaT(wx[l], xv[3 + l], a01[r].x);
+                a01[r].y = fmaT(wx[l], xv[4 + l], a01[r].y);
+                a23[r].x = fmaT(wx[l], xv[5 + l], a23[r].x);
+                a23[r].y = fmaT(wx[l], xv[6 + l], a23[r].y);
+              }
+            }
+            y01[r] = y23[r] = make_float2(0.f, 0.f);
+          }
+          // y: each row of the thread's columns once for all its points
+#pragma unroll
+          for (int m = 0; m < AXW + AXV_NR - 1; ++m) {
+            const float4 v =
+                m >= 5 && m < 5 + AXV_NR ? win[m - 5][u + 5] : lds4(sp + (AXV_NR * ty + m) * AXV_W + cx);
+#pragma unroll
+            for (int r = 0; r < AXV_NR; ++r) {
+              const int l = m - r;
+              if (l < 0 || l >= AXW || l == 5) continue;
+              const float2 w2 = make_float2(wy[r][l], wy[r][l]);
+              y01[r] = __ffma2_rn(w2, make_float2(v.x, v.y), y01[r]);
+              y23[r] = __ffma2_rn(w2, make_float2(v.z, v.w), y23[r]);
             }
           }
-          float2 y01 = make_float2(0.f, 0.f), y23 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int l = 0; l < AXW; ++l) {
-            if (l == 5) continue;
-            const float4 v = lds4(sp + (ty + l) * AXV_W + cx);
-            const float2 w2 = make_float2(wy[l], wy[l]);
-            y01 = __ffma2_rn(w2, make_float2(v.x, v.y), y01);
-            y23 = __ffma2_rn(w2, make_float2(v.z, v.w), y23);
-          }
-          float2 z01 = make_float2(0.f, 0.f), z23 = make_float2(0.f, 0.f);
+          for (int r = 0; r < AXV_NR; ++r) {
+            float2 z01 = make_float2(0.f, 0.f), z23 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int l = 0; l < AXW; ++l) {
-            if (l == 5) continue;
-            const float2 w2 = make_float2(wz[l], wz[l]);
-            z01 = __ffma2_rn(w2, make_float2(win[u + l].x, win[u + l].y), z01);
-            z23 = __ffma2_rn(w2, make_float2(win[u + l].z, win[u + l].w), z23);
-          }
-          a01 = __fadd2_rn(__fadd2_rn(a01, y01), z01);
-          a23 = __fadd2_rn(__fadd2_rn(a23, y23), z23);
-          if (act) {
-            *reinterpret_cast<float4*>(o) = make_float4(a01.x, a01.y, a23.x, a23.y);
-            // the plane's 4 products summed in FP32, the sum added in FP64
-            if (MODE != 0) {
-              const float4 pv = lds4(pring + (size_t)(t % AXV_R) * AXV_PP + pq);
-              const float2 d = __ffma2_rn(a23, make_float2(pv.z, pv.w), __fmul2_rn(a01, make_float2(pv.x, pv.y)));
-              v0 += (double)__fadd_rn(d.x, d.y);
+            for (int l = 0; l < AXW; ++l) {
+              if (l == 5) continue;
+              const float2 w2 = make_float2(wz[l], wz[l]);
+              const float4 v = win[r][u + l];
+              z01 = __ffma2_rn(w2, make_float2(v.x, v.y), z01);
+              z23 = __ffma2_rn(w2, make_float2(v.z, v.w), z23);
             }
-            if (MODE == 2) {
-              const float2 d = __ffma2_rn(a23, a23, __fmul2_rn(a01, a01));
-              v1 += (double)__fadd_rn(d.x, d.y);
+            const float2 r01 = __fadd2_rn(__fadd2_rn(a01[r], y01[r]), z01);
+            const float2 r23 = __fadd2_rn(__fadd2_rn(a23[r], y23[r]), z23);
+            if (act[r]) {
+              *reinterpret_cast<float4*>(o + own[r]) = make_float4(r01.x, r01.y, r23.x, r23.y);
+              // the plane's 4 products summed in FP32, the sum added in FP64
+              if (MODE != 0) {
+                const float4 pv = lds4(pring + (size_t)(t % AXV_R) * AXV_PP + pq + r * ETX);
+                const float2 d = __ffma2_rn(r23, make_float2(pv.z, pv.w), __fmul2_rn(r01, make_float2(pv.x, pv.y)));
+                v0 += (double)__fadd_rn(d.x, d.y);
+              }
+              if (MODE == 2) {
+                const float2 d = __ffma2_rn(r23, r23, __fmul2_rn(r01, r01));
+                v1 += (double)__fadd_rn(d.x, d.y);
+              }
             }
           }
           o += nxy;
         }
       }
 #pragma unroll
-      for (int l = 0; l < AXV_ZW - AXV_B; ++l) win[l] = win[l + AXV_B];
+      for (int r = 0; r < AXV_NR; ++r) {
 #pragma unroll
-      for (int u = 0; u < AXV_B; ++u) win[AXV_ZW - AXV_B + u] = nw[u];
+        for (int l = 0; l < AXV_ZW - AXV_B; ++l) win[r][l] = win[r][l + AXV_B];
+#pragma unroll
+        for (int u = 0; u < AXV_B; ++u) win[r][AXV_ZW - AXV_B + u] = nw[r][u];
+      }
     }
     cp_wait<0>();
     if (MODE != 0) {
@@ -1435,9 +1492,10 @@ __global__ void __launch_bounds__(AXV_NT, 5) k_kr_ax32v(const KrylovJob<float>* 
 // ------------------------------------------------------------------------------------------
 // The FP64 operator (the Krylov list of an FP64 solve, and the outer residual of the mixed
 // solve) on grids with n1 divisible by 2: the collapsed 11-point product_div_grad with every
-// thread owning one 16-byte vector of 2 consecutive x points of one row.  The staging and z
-// window of k_kr_ax32v (16 x 8 threads per 32 x 8-column tile, 48 x 18 staged doubles per plane,
-// a ring of 2 groups of 4 planes, the window k-5 .. k+8 in registers); the weights are the per-row
+// thread owning one 16-byte vector of 2 consecutive x points of one row.  Staged like k_kr_ax32v,
+// with one row per thread and its own points in the staged plane (16 x 8 threads per 32 x 8-column
+// tile, 48 x 18 doubles per plane, a ring of 2 groups of 4 planes, the window k-5 .. k+8 in
+// registers; own points from the window: the same time, 286 us on 256 x 256 x 512); the weights are the per-row
 // weights of every axis (the FP64 operator defines the residual): x rows of the thread's two
 // columns and the y row of its row in registers, the z rows of the tile's planes in shared memory.
 //   MODE 0: rr = A phi;  1: Ap = A z1, partial rh.Ap;  2: Ar = A z2, partials Ar.rr, Ar.Ar;
@@ -3213,13 +3271,14 @@ inline int grid_multi(int ntiles) { return ntiles; }
 // default).  A tile is a serial chain of planes after a prologue of about 8 planes' time (the
 // job's scalars; in the operator the z window and the first staged group), so the depth minimises
 // waves of tiles over the kernel's resident blocks x (depth + 8), among kc, the multiples of 8
-// below it (the vector updates walk blocks of 8 planes) and 4.  Grids of many waves keep kc; on
+// below it (the vector updates walk blocks of 8 planes), 4 and, in the two-row
+// operator, 2 (its step).  Grids of many waves keep kc; on
 // 32 x 32 x 64 the 4 tiles of 64 planes become 64 of 4 (FP32 operator 26.6 -> 6.2 us, x update
 // 14.4 -> 4.3 us).  It depends on the grid alone, so a case's partial sums do not depend on its
 // batch.
 constexpr int kVecBlocksPerSm = 4;  // resident blocks of the vector updates
 template <typename TilesXY>
-inline int depth_for(TilesXY&& tiles, int n3, int kc, int slots) {
+inline int depth_for(TilesXY&& tiles, int n3, int kc, int slots, int least = 4) {
   int best = kc;
   long long cost = -1;
   auto consider = [&](int d) {
@@ -3231,11 +3290,12 @@ inline int depth_for(TilesXY&& tiles, int n3, int kc, int slots) {
   };
   consider(kc);
   for (int d = (kc - 1) / 8 * 8; d >= 8; d -= 8) consider(d);
-  if (kc > 4) consider(4);
+  for (int d = 4; d >= least; d /= 2)
+    if (kc > d) consider(d);
   return best;
 }
-inline int krylov_depth(const Geom& g, int kc, int slots) {
-  return depth_for([&](int d) { return (long long)tiles_of(g, d); }, g.n3, kc, slots);
+inline int krylov_depth(const Geom& g, int kc, int slots, int rows = ETY) {
+  return depth_for([&](int d) { return (long long)tiles_of(g, d, 1, rows); }, g.n3, kc, slots, rows > ETY ? 2 : 4);
 }
 // the depth of a list without partial sums: the same rule over all its grids together (the small
 // grids of a batch need no shallow tiles of their own to fill the GPU)
@@ -3443,21 +3503,22 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     // another order
     constexpr bool f32 = std::is_same<T, float>::value;
     const bool adapt = f32 || use_mg;
-    auto depths = [&](auto slots) {
+    auto depths = [&](auto slots, auto rows) {
       long long tiles = 0;
       for (int c = 0; c < n; ++c) {
-        kj[c].kc = adapt ? krylov_depth(kj[c].g, kc, slots(kj[c])) : kc;
-        kt[c] = tiles_of(kj[c].g, kj[c].kc);
+        kj[c].kc = adapt ? krylov_depth(kj[c].g, kc, slots(kj[c]), rows(kj[c])) : kc;
+        kt[c] = tiles_of(kj[c].g, kj[c].kc, 1, rows(kj[c]));
         tiles += kt[c];
       }
       return tiles;
     };
     const long long ta = depths([&](const KrylovJob<T>& J) {
       return std::min(J.vec ? (f32 ? g_axv_grid : g_axd_grid) : (f32 ? g_axs32_grid : g_axs64_grid),
-                      device_sms() * kVecBlocksPerSm);
-    });
+                      device_sms() * kVecBlocksPerSm );
+    }, [&](const KrylovJob<T>& J) { return f32 && J.vec ? AXV_Y : ETY; });
     kr_list_ = arena_.add(kj, kt);
-    const long long tv = depths([&](const KrylovJob<T>&) { return device_sms() * kVecBlocksPerSm; });
+    const long long tv = depths([&](const KrylovJob<T>&) { return device_sms() * kVecBlocksPerSm; },
+                                [](const KrylovJob<T>&) { return ETY; });
     kv_list_ = arena_.add(kj, kt);
     std::vector<Geom> gs;
     for (const auto& J : kj) gs.push_back(J.g);

@@ -27,8 +27,8 @@ constexpr int AXW = 11;     // product_div_grad collapsed to an 11-point stencil
 constexpr int KC_MAX = 64;  // largest tile depth
 
 inline int tiles_xy(const Geom& g) { return ((g.n1 + ETX - 1) / ETX) * ((g.n2 + ETY - 1) / ETY); }
-inline int tiles_of(const Geom& g, int kc, int vw = 1) {
-  return ((g.n1 + ETX * vw - 1) / (ETX * vw)) * ((g.n2 + ETY - 1) / ETY) * ((g.n3 + kc - 1) / kc);
+inline int tiles_of(const Geom& g, int kc, int vw = 1, int rows = ETY) {
+  return ((g.n1 + ETX * vw - 1) / (ETX * vw)) * ((g.n2 + rows - 1) / rows) * ((g.n3 + kc - 1) / kc);
 }
 // Tile geometry of the fused smoothing kernel k_lv_multi (MNT threads): a block's input region
 // is 16 V x (MNT / 16) columns (V = 16 bytes / element size consecutive columns per thread, one

@@ -47,3 +47,23 @@ def test_operator_matches_oracle(gi, op, tol):
     w = og.interior(want)
     assert np.abs(got - w).max() <= tol * np.abs(w).max()
     case.close()
+
+
+# the FP32 vector kernel's tiles of 32 x 16 columns: one row and one column over a tile, one short of
+# it, an odd last row pair, tiles of 2 planes and ragged last steps
+EDGES = [(32, 16, 8), (36, 17, 9), (28, 15, 34), (64, 31, 11), (8, 33, 131), (12, 47, 10)]
+
+
+@pytest.mark.parametrize("op,tol", [(0, 1e-12), (2, 1e-5)], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("n", EDGES, ids=lambda n: "%dx%dx%d" % n)
+def test_operator_at_tile_edges(n, op, tol):
+    N, L = tuple(k + 1 for k in n), tuple(k / 32.0 for k in n)
+    og, ig = O.Grid(N, L, (0, 0, 0)), I.Grid(N, L, (0, 0, 0))
+    case = I.Case(ig, precision=1 if op == 2 else 0)
+    x = og.random(18)
+    want = og.interior(og.product_div_grad(x.copy()))
+    case.upload("pre", x)
+    case.apply("pre", "res", op=op)
+    got = og.interior(case.download("res"))
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+    case.close()

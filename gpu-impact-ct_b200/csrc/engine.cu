@@ -1585,7 +1585,7 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
       }
       cp_commit();
     };
-    __syncthreads();  // the ring and the z weights of the previous tile are no longer read
+    __syncthreads();  // the ring of the previous tile is no longer read, and the weights are there
 #pragma unroll
     for (int gi = 0; gi < AXD_G - 1; ++gi) stage_group(gi);
     double2 win[AXD_ZW];
@@ -1709,6 +1709,8 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
           partial[(long long)b * 4 + 3] = s3;
         }
       }
+    } else {
+      __syncthreads();  // the z weights are rewritten by the next tile
     }
   }
 }

@@ -1492,68 +1492,92 @@ __global__ void __launch_bounds__(AXV_NT, 4) k_kr_ax32v(const KrylovJob<float>* 
 // ------------------------------------------------------------------------------------------
 // The FP64 operator (the Krylov list of an FP64 solve, and the outer residual of the mixed
 // solve) on grids with n1 divisible by 2: the collapsed 11-point product_div_grad with every
-// thread owning one 16-byte vector of 2 consecutive x points of one row.  Staged like k_kr_ax32v,
-// with one row per thread and its own points in the staged plane (16 x 8 threads per 32 x 8-column
-// tile, 48 x 18 doubles per plane, a ring of 2 groups of 4 planes, the window k-5 .. k+8 in
-// registers; own points from the window: the same time, 286 us on 256 x 256 x 512); the weights are the per-row
+// thread owning one 16-byte vector of 2 consecutive x points of NR rows, 16 x 8 threads per
+// 32 x 8 NR-column tile.  NR = 2 (the outer residual) is staged like k_kr_ax32v, with the y weights
+// in shared memory; NR = 1 stages the whole plane (48 x 18 doubles) in groups of 4, with the y weights
+// in registers.  Outer residual on 256 x 256 x 512 318 -> 309 us, 128 x 128 x 256 55 -> 52, a mixed
+// step at 384 x 384 x 768 154.1 -> 153.1 ms.  The Krylov lists keep one row: two take 267 instead of
+// 283 us on 256 x 256 x 512 and 8.3 instead of 6.8 on 32 x 32 x 64, and they sum the inner products
+// in another order, which the JOR solves' 100 iterations carry up to the solve's tolerance.  At one
+// row the own points from the window change nothing.  All bound by the shared-memory loads and the
+// latency of 8 warps per SM (255 registers); the weights are the per-row
 // weights of every axis (the FP64 operator defines the residual): x rows of the thread's two
 // columns and the y row of its row in registers, the z rows of the tile's planes in shared memory.
 //   MODE 0: rr = A phi;  1: Ap = A z1, partial rh.Ap;  2: Ar = A z2, partials Ar.rr, Ar.Ar;
 //   3: r32 = (float)(bb - A phi), partials max|r|, sum r^2, sum bb^2
 constexpr int AXD_TX = ETX / 2, AXD_NT = AXD_TX * ETY;   // 16 x 8 threads, 2 columns each
-constexpr int AXD_W = ETX + 16, AXD_H = ETY + 10;        // staged plane, doubles
+constexpr int AXD_W = ETX + 16;                          // staged row, doubles
 constexpr int AXD_CR = AXD_W / 2;                        // 16-byte chunks per row
-constexpr int AXD_NCH = AXD_CR * AXD_H;
-constexpr int AXD_PER = (AXD_NCH + AXD_NT - 1) / AXD_NT;
-constexpr int AXD_PLANE = AXD_W * AXD_H;
-constexpr int AXD_PP = ETX * ETY;
-constexpr int AXD_B = 4, AXD_G = 2, AXD_R = AXD_B * AXD_G, AXD_ZW = AXD_B + 10;
-constexpr size_t axd_smem_bytes() {
-  return sizeof(double) * ((size_t)AXD_R * (AXD_PLANE + AXD_PP) + (size_t)KC_MAX * AXW);
-}
+template <int NR>
+struct Axd {                                             // NR rows per thread
+  static constexpr int Y = NR * ETY, H = Y + 10;         // rows per tile, staged rows
+  static constexpr int NCH = AXD_CR * H, PER = (NCH + AXD_NT - 1) / AXD_NT;
+  static constexpr int PLANE = AXD_W * H, PP = ETX * Y;
+  static constexpr int B = NR == 1 ? 4 : 2, G = 2, R = B * G, ZW = B + 10;
+  static constexpr int WY = NR == 1 ? 0 : Y * 12;        // y weights in shared memory (NR > 1)
+  static constexpr size_t smem() { return sizeof(double) * ((size_t)R * (PLANE + PP) + WY + (size_t)KC_MAX * AXW); }
+};
 __device__ __forceinline__ double2 ldg2d(const double* p) { return __ldg(reinterpret_cast<const double2*>(p)); }
 __device__ __forceinline__ double2 lds2d(const double* p) { return *reinterpret_cast<const double2*>(p); }
 
-template <int MODE>
+constexpr int AXD_NR3 = 2;  // rows per thread of the outer residual (MODE 3)
+template <int MODE, int NR>
 __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>* __restrict__ jobs,
                                                         const int* __restrict__ ts, int nj, int ntiles,
                                                         double* __restrict__ partial) {
+  using AX = Axd<NR>;
+  constexpr int AXD_NCH = AX::NCH, AXD_PER = AX::PER, AXD_PLANE = AX::PLANE, AXD_PP = AX::PP;
+  constexpr int AXD_B = AX::B, AXD_G = AX::G, AXD_R = AX::R, AXD_ZW = AX::ZW;
   extern __shared__ __align__(16) unsigned char axd_smem[];
   double* ring = reinterpret_cast<double*>(axd_smem);
   double* pring = ring + (size_t)AXD_R * AXD_PLANE;
-  double(*wzs)[AXW] = reinterpret_cast<double(*)[AXW]>(pring + (size_t)AXD_R * AXD_PP);
+  double* wys = pring + (size_t)AXD_R * AXD_PP;
+  double(*wzs)[AXW] = reinterpret_cast<double(*)[AXW]>(wys + AX::WY);
   __shared__ double red[4][AXD_NT / 32];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = tx + AXD_TX * ty;
   const int cx = 8 + 2 * tx;          // the thread's first column in a staged row
-  const int pq = ty * ETX + 2 * tx;   // the thread's vector in a partner slot
+  const int pq = NR * ty * ETX + 2 * tx;   // the thread's vector in a partner slot
   for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
     const int q = find_job(ts, nj, b);
     const KrylovJob<double>& J = jobs[q];
     const SolverScalars* sc = J.sc;
     if (!J.vec || (MODE == 0 ? (sc->done != 0) : e_halted(sc))) continue;  // the others: k_kr_ax
     const Geom g = J.g;
-    const int ntx = (g.n1 + ETX - 1) / ETX, nty = (g.n2 + ETY - 1) / ETY;
+    const int ntx = (g.n1 + ETX - 1) / ETX, nty = (g.n2 + AX::Y - 1) / AX::Y;
     const int t0 = b - ts[q];
     const int ta = t0 % ntx, tr = t0 / ntx, tc = tr / nty;
-    const int i0 = ta * ETX + 1, j0 = (tr - tc * nty) * ETY + 1;
+    const int i0 = ta * ETX + 1, j0 = (tr - tc * nty) * AX::Y + 1;
     const int k0 = tc * J.kc + 1, k1 = min(g.n3, k0 + J.kc - 1);
     const int nk = k1 - k0 + 1;
-    const int i = i0 + 2 * tx, j = j0 + ty;
-    const bool act = i <= g.n1 && j <= g.n2;  // n1 % 2 == 0: both columns valid together
+    const int i = i0 + 2 * tx, j = j0 + NR * ty;
+    const bool in_x = i <= g.n1;  // n1 % 2 == 0: both columns valid together
+    bool act[NR];                 // (a second row past the last one holds its image, row 1, for the first)
+    int own[NR];                  // in-plane offsets of the thread's vectors
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      act[r] = in_x && j + r <= g.n2;
+      own[r] = (in_x ? i + 3 : 4) + g.nx * ((j + r <= g.n2 ? j + r : 1) + 3);
+    }
     const double* __restrict__ x = (MODE == 0 || MODE == 3) ? J.phi : (MODE == 1 ? J.z1 : J.z2);
     const double* __restrict__ d1 = MODE == 1 ? J.rh : (MODE == 3 ? J.bb : J.rr);
     const long long nxy = g.nxy;
-    const int ir = act ? i : 1, jr = j <= g.n2 ? j : 1;
-    double wx0[AXW], wx1[AXW], wy[AXW];
+    const int ir = in_x ? i : 1;
+    double wx0[AXW], wx1[AXW], wy1[AXW];
 #pragma unroll
     for (int l = 0; l < AXW; ++l) {
       wx0[l] = __ldg(J.W[0] + (size_t)(ir - 1) * AXW + l);
       wx1[l] = __ldg(J.W[0] + (size_t)ir * AXW + l);
-      wy[l] = __ldg(J.W[1] + (size_t)(jr - 1) * AXW + l);
+      if (NR == 1) wy1[l] = __ldg(J.W[1] + (size_t)((j <= g.n2 ? j : 1) - 1) * AXW + l);
     }
+    if (NR > 1)
+      for (int t = tid; t < AX::Y * AXW; t += AXD_NT) {
+        const int r = t / AXW, jr = j0 + r <= g.n2 ? j0 + r : 1;
+        wys[r * 12 + t % AXW] = __ldg(J.W[1] + (size_t)(jr - 1) * AXW + t % AXW);
+      }
+    auto wy = [&](int r, int l) { return NR == 1 ? wy1[l] : wys[(NR * ty + r) * 12 + l]; };
     for (int t = tid; t < nk * AXW; t += AXD_NT) wzs[t / AXW][t % AXW] = __ldg(J.W[2] + (size_t)(k0 - 1) * AXW + t);
-    const int ilast = min(i0 + ETX - 1, g.n1) + 5, jlast = min(j0 + ETY - 1, g.n2) + 5;
+    const int ilast = min(i0 + ETX - 1, g.n1) + 5, jlast = min(j0 + AX::Y - 1, g.n2) + 5;
     // a chunk starts at an odd column and n1 is even, so a chunk outside 1..n1 lies whole in one
     // periodic image (n1 >= 8): every chunk is one 16-byte copy from its image
     int cb[AXD_PER];
@@ -1562,10 +1586,11 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
       const int cq = tid + e * AXD_NT;
       const int r = cq / AXD_CR, c0 = (cq % AXD_CR) * 2;
       const int jj = j0 - 5 + r, ii = i0 - 8 + c0;
-      const bool need = cq < AXD_NCH && jj <= jlast && ii + 1 >= i0 - 5 && ii <= ilast;
+      // a chunk of the tile's own points comes from the z window
+      const bool mine = NR > 1 && c0 >= 8 && c0 < 8 + ETX && ii <= g.n1 && r >= 5 && r < 5 + AX::Y && jj <= g.n2;
+      const bool need = cq < AXD_NCH && jj <= jlast && ii + 1 >= i0 - 5 && ii <= ilast && !mine;
       cb[e] = need ? (wrapi(ii, g.n1) + 3) + g.nx * (wrapi(jj, g.n2) + 3) : -1;
     }
-    const int own = (act ? i + 3 : 4) + g.nx * (jr + 3);
     auto zoff = [&](int k) -> long long {
       return (long long)((k < 1 ? k + g.n3 : (k > g.n3 ? k - g.n3 : k)) + 3) * nxy;
     };
@@ -1580,7 +1605,9 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
 #pragma unroll
           for (int e = 0; e < AXD_PER; ++e)
             if (cb[e] >= 0) cp_async16(dst + e * AXD_NT * 2, src + cb[e]);
-          if (MODE != 0 && act) cp_async16(pring + (size_t)(t % AXD_R) * AXD_PP + pq, d1 + zo + own);
+#pragma unroll
+          for (int r = 0; r < NR; ++r)
+            if (MODE != 0 && act[r]) cp_async16(pring + (size_t)(t % AXD_R) * AXD_PP + pq + r * ETX, d1 + zo + own[r]);
         }
       }
       cp_commit();
@@ -1588,97 +1615,130 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
     __syncthreads();  // the ring of the previous tile is no longer read, and the weights are there
 #pragma unroll
     for (int gi = 0; gi < AXD_G - 1; ++gi) stage_group(gi);
-    double2 win[AXD_ZW];
+    double2 win[NR][AXD_ZW];
     const double2 zero2 = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int l = 0; l < AXD_ZW; ++l) win[l] = act ? ldg2d(x + zoff(k0 - 5 + l) + own) : zero2;
+    for (int l = 0; l < AXD_ZW; ++l)
+#pragma unroll
+      for (int r = 0; r < NR; ++r) win[r][l] = in_x ? ldg2d(x + zoff(k0 - 5 + l) + own[r]) : zero2;
+    // plane t of the thread's own points (window place l) into its slot
+    auto publish = [&](int t, int l) {
+      if (NR > 1 && t < nk)
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+          if (act[r])
+            *reinterpret_cast<double2*>(ring + (size_t)(t % AXD_R) * AXD_PLANE + (NR * ty + r + 5) * AXD_W + cx) = win[r][l];
+    };
+#pragma unroll
+    for (int u = 0; u < AXD_B; ++u) publish(u, 5 + u);
     double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-    const long long obase = (long long)(k0 + 3) * nxy + own;
+    const long long obase = (long long)(k0 + 3) * nxy;
     const int nsteps = (nk + AXD_B - 1) / AXD_B;
     for (int s = 0; s < nsteps; ++s) {
       const int tb = s * AXD_B;
       cp_wait<AXD_G - 2>();
       __syncthreads();  // everybody's copies of the step's group (and the z weights) are visible
       stage_group(s + AXD_G - 1);
-      double2 nw[AXD_B];
-      const bool more = act && tb + AXD_B < nk;
 #pragma unroll
-      for (int u = 0; u < AXD_B; ++u) nw[u] = more ? ldg2d(x + zoff(k0 + tb + AXD_B + 5 + u) + own) : zero2;
+      for (int u = 0; u < AXD_B; ++u) publish(tb + AXD_B + u, 5 + AXD_B + u);
+      double2 nw[NR][AXD_B];
+      const bool more = in_x && tb + AXD_B < nk;
+#pragma unroll
+      for (int u = 0; u < AXD_B; ++u)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) nw[r][u] = more ? ldg2d(x + zoff(k0 + tb + AXD_B + 5 + u) + own[r]) : zero2;
 #pragma unroll
       for (int u = 0; u < AXD_B; ++u) {
         const int t = tb + u;
         if (t < nk) {
           const double* sp = ring + (size_t)(t % AXD_R) * AXD_PLANE;
           const double* wz = wzs[t];
-          double xv[14];  // the thread's row, columns cx-6 .. cx+7 (own at 6, 7)
+          double a0[NR], a1[NR], y0[NR], y1[NR];
 #pragma unroll
-          for (int m = 0; m < 7; ++m) {
-            const double2 v = lds2d(sp + (ty + 5) * AXD_W + cx - 6 + 2 * m);
-            xv[2 * m] = v.x;
-            xv[2 * m + 1] = v.y;
-          }
-          const double wyz = __dadd_rn(wy[5], wz[5]);
-          const double2 cc = win[u + 5];
-          double r0 = mulT(__dadd_rn(wx0[5], wyz), cc.x), r1 = mulT(__dadd_rn(wx1[5], wyz), cc.y);
+          for (int r = 0; r < NR; ++r) {
+            double xv[14];  // the row, columns cx-6 .. cx+7 (own at 6, 7)
 #pragma unroll
-          for (int l = 0; l < AXW; ++l) {
-            if (l == 5) continue;
-            r0 = fmaT(wx0[l], xv[1 + l], r0);
-            r1 = fmaT(wx1[l], xv[2 + l], r1);
-          }
-          double y0 = 0.0, y1 = 0.0;
+            for (int m = 0; m < 7; ++m) {
+              const double2 v = m == 3 ? win[r][u + 5] : lds2d(sp + (NR * ty + r + 5) * AXD_W + cx - 6 + 2 * m);
+              xv[2 * m] = v.x;
+              xv[2 * m + 1] = v.y;
+            }
+            const double wyz = __dadd_rn(wy(r, 5), wz[5]);
+            a0[r] = mulT(__dadd_rn(wx0[5], wyz), xv[6]);
+            a1[r] = mulT(__dadd_rn(wx1[5], wyz), xv[7]);
 #pragma unroll
-          for (int l = 0; l < AXW; ++l) {
-            if (l == 5) continue;
-            const double2 v = lds2d(sp + (ty + l) * AXD_W + cx);
-            y0 = fmaT(wy[l], v.x, y0);
-            y1 = fmaT(wy[l], v.y, y1);
+            for (int l = 0; l < AXW; ++l) {
+              if (l == 5) continue;
+              a0[r] = fmaT(wx0[l], xv[1 + l], a0[r]);
+              a1[r] = fmaT(wx1[l], xv[2 + l], a1[r]);
+            }
+            y0[r] = y1[r] = 0.0;
           }
-          double z0 = 0.0, z1 = 0.0;
+          // y: each row of the thread's columns once for all its points
 #pragma unroll
-          for (int l = 0; l < AXW; ++l) {
-            if (l == 5) continue;
-            const double w = wz[l];
-            z0 = fmaT(w, win[u + l].x, z0);
-            z1 = fmaT(w, win[u + l].y, z1);
+          for (int m = 0; m < AXW + NR - 1; ++m) {
+            if (NR == 1 && m == 5) continue;
+            const double2 v = m >= 5 && m < 5 + NR ? win[m >= 5 && m < 5 + NR ? m - 5 : 0][u + 5]
+                                                   : lds2d(sp + (NR * ty + m) * AXD_W + cx);
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+              const int l = m - r;
+              if (l < 0 || l >= AXW || l == 5) continue;
+              const double w = wy(r, l);
+              y0[r] = fmaT(w, v.x, y0[r]);
+              y1[r] = fmaT(w, v.y, y1[r]);
+            }
           }
-          r0 = __dadd_rn(__dadd_rn(r0, y0), z0);
-          r1 = __dadd_rn(__dadd_rn(r1, y1), z1);
-          if (act) {
-            const long long o = obase + (long long)t * nxy;
-            if (MODE == 3) {
-              const double2 bv = lds2d(pring + (size_t)(t % AXD_R) * AXD_PP + pq);
-              const double e0 = bv.x - r0, e1 = bv.y - r1;
-              const float2 ef = make_float2((float)e0, (float)e1);
-              *reinterpret_cast<float2*>(J.r32 + o) = ef;
-              if (J.r32p) *reinterpret_cast<float2*>(J.r32p + o) = ef;
-              v3 += (double)ef.x * (double)ef.x;
-              v3 += (double)ef.y * (double)ef.y;
-              v0 = fmax(v0, fmax(fabs(e0), fabs(e1)));
-              v1 += e0 * e0;
-              v1 += e1 * e1;
-              v2 += bv.x * bv.x;
-              v2 += bv.y * bv.y;
-            } else {
-              double* out = MODE == 0 ? J.rr : (MODE == 1 ? J.Ap : J.Ar);
-              *reinterpret_cast<double2*>(out + o) = make_double2(r0, r1);
-              if (MODE != 0) {
-                const double2 pv = lds2d(pring + (size_t)(t % AXD_R) * AXD_PP + pq);
-                v0 += r0 * pv.x;
-                v0 += r1 * pv.y;
-              }
-              if (MODE == 2) {
-                v1 += r0 * r0;
-                v1 += r1 * r1;
+#pragma unroll
+          for (int r = 0; r < NR; ++r) {
+            double z0 = 0.0, z1 = 0.0;
+#pragma unroll
+            for (int l = 0; l < AXW; ++l) {
+              if (l == 5) continue;
+              const double w = wz[l];
+              z0 = fmaT(w, win[r][u + l].x, z0);
+              z1 = fmaT(w, win[r][u + l].y, z1);
+            }
+            const double r0 = __dadd_rn(__dadd_rn(a0[r], y0[r]), z0), r1 = __dadd_rn(__dadd_rn(a1[r], y1[r]), z1);
+            if (act[r]) {
+              const long long o = obase + own[r] + (long long)t * nxy;
+              if (MODE == 3) {
+                const double2 bv = lds2d(pring + (size_t)(t % AXD_R) * AXD_PP + pq + r * ETX);
+                const double e0 = bv.x - r0, e1 = bv.y - r1;
+                const float2 ef = make_float2((float)e0, (float)e1);
+                *reinterpret_cast<float2*>(J.r32 + o) = ef;
+                if (J.r32p) *reinterpret_cast<float2*>(J.r32p + o) = ef;
+                v3 += (double)ef.x * (double)ef.x;
+                v3 += (double)ef.y * (double)ef.y;
+                v0 = fmax(v0, fmax(fabs(e0), fabs(e1)));
+                v1 += e0 * e0;
+                v1 += e1 * e1;
+                v2 += bv.x * bv.x;
+                v2 += bv.y * bv.y;
+              } else {
+                double* out = MODE == 0 ? J.rr : (MODE == 1 ? J.Ap : J.Ar);
+                *reinterpret_cast<double2*>(out + o) = make_double2(r0, r1);
+                if (MODE != 0) {
+                  const double2 pv = lds2d(pring + (size_t)(t % AXD_R) * AXD_PP + pq + r * ETX);
+                  v0 += r0 * pv.x;
+                  v0 += r1 * pv.y;
+                }
+                if (MODE == 2) {
+                  v1 += r0 * r0;
+                  v1 += r1 * r1;
+                }
               }
             }
           }
         }
       }
 #pragma unroll
-      for (int l = 0; l < AXD_ZW - AXD_B; ++l) win[l] = win[l + AXD_B];
+      for (int r = 0; r < NR; ++r) {
 #pragma unroll
-      for (int u = 0; u < AXD_B; ++u) win[AXD_ZW - AXD_B + u] = nw[u];
+        for (int l = 0; l < AXD_ZW - AXD_B; ++l) win[r][l] = win[r][l + AXD_B];
+#pragma unroll
+        for (int u = 0; u < AXD_B; ++u) win[r][AXD_ZW - AXD_B + u] = nw[r][u];
+      }
     }
     cp_wait<0>();
     if (MODE != 0) {
@@ -3169,7 +3229,7 @@ __global__ void __launch_bounds__(ENT) k_mx_apply(const MixJob* __restrict__ job
 
 // grids of the vector operator kernels: the blocks resident at once on the device (a grid-stride
 // kernel given more would leave its last blocks to run after the others, one tile step behind)
-int g_axv_grid = 0, g_axd_grid = 0;
+int g_axv_grid = 0, g_axd_grid = 0, g_axd3_grid = 0;
 int g_axs32_grid = 0, g_axs64_grid = 0;  // the same of the staged operator kernels
 // the operator kernels use more than 48 KB of dynamic shared memory: opt in once per process
 // and device
@@ -3185,10 +3245,10 @@ void ax_attributes() {
   cudaFuncSetAttribute(k_kr_ax32<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axa_smem_bytes());
   cudaFuncSetAttribute(k_kr_ax32<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axa_smem_bytes());
   cudaFuncSetAttribute(k_kr_ax32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axa_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax64v<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axd_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax64v<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axd_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax64v<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axd_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax64v<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axd_smem_bytes());
+  cudaFuncSetAttribute(k_kr_ax64v<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<3, AXD_NR3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<AXD_NR3>::smem());
   cudaFuncSetAttribute(k_kr_ax32v<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axv_smem_bytes());
   cudaFuncSetAttribute(k_kr_ax32v<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axv_smem_bytes());
   cudaFuncSetAttribute(k_kr_ax32v<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axv_smem_bytes());
@@ -3202,8 +3262,9 @@ void ax_attributes() {
   if (nsm <= 0) nsm = 148;
   g_axv_grid = nsm * std::min({occ(k_kr_ax32v<0>, AXV_NT, axv_smem_bytes()), occ(k_kr_ax32v<1>, AXV_NT, axv_smem_bytes()),
                                occ(k_kr_ax32v<2>, AXV_NT, axv_smem_bytes())});
-  g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<1>, AXD_NT, axd_smem_bytes()),
-                               occ(k_kr_ax64v<2>, AXD_NT, axd_smem_bytes()), occ(k_kr_ax64v<3>, AXD_NT, axd_smem_bytes())});
+  g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0, 1>, AXD_NT, Axd<1>::smem()), occ(k_kr_ax64v<1, 1>, AXD_NT, Axd<1>::smem()),
+                               occ(k_kr_ax64v<2, 1>, AXD_NT, Axd<1>::smem())});
+  g_axd3_grid = nsm * occ(k_kr_ax64v<3, AXD_NR3>, AXD_NT, Axd<AXD_NR3>::smem());
   g_axs32_grid = nsm * occ(k_kr_ax32<1>, AXNT, axa_smem_bytes());
   g_axs64_grid = nsm * occ(k_kr_ax<double, 1>, AXNT, ax_smem_bytes<double>());
   cudaFuncSetAttribute(k_lv_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
@@ -3260,8 +3321,10 @@ void launch_ax(int grid, const KrylovJob<T>* J, const int* ts, int n, int ntiles
     if (vec != 1) k_kr_ax32<MODE><<<grid, kAxBlock, axa_smem_bytes(), s>>>(J, ts, n, ntiles, partial);
     if (vec == 2) prof::count(1);  // two launches where the callers count one
   } else {
-    const int gv = g_axd_grid > 0 ? std::min(g_axd_grid, ntiles) : grid;
-    if (vec != 0) k_kr_ax64v<MODE><<<gv, dim3(AXD_TX, ETY), axd_smem_bytes(), s>>>(J, ts, n, ntiles, partial);
+    constexpr int NR = MODE == 3 ? AXD_NR3 : 1;
+    const int slots = MODE == 3 ? g_axd3_grid : g_axd_grid;
+    const int gv = slots > 0 ? std::min(slots, ntiles) : grid;
+    if (vec != 0) k_kr_ax64v<MODE, NR><<<gv, dim3(AXD_TX, ETY), Axd<NR>::smem(), s>>>(J, ts, n, ntiles, partial);
     if (vec != 1) k_kr_ax<T, MODE><<<grid, kAxBlock, ax_smem_bytes<T>(), s>>>(J, ts, n, ntiles, partial);
     if (vec == 2) prof::count(1);
   }
@@ -4321,8 +4384,9 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
     M.e32 = C.e32;
     M.q = q_ + 4 * c;
     M.isc = inner_.scal_dev() + c;
-    A.kc = krylov_depth(C.g, kc, A.vec ? g_axd_grid : g_axs64_grid);
-    t[c] = tiles_of(C.g, A.kc);
+    const int rows = A.vec ? Axd<AXD_NR3>::Y : ETY;
+    A.kc = krylov_depth(C.g, kc, A.vec ? g_axd3_grid : g_axs64_grid, rows);
+    t[c] = tiles_of(C.g, A.kc, 1, rows);
     tiles += t[c];
     M.kc = dl;
     M.vecu = C.g.n1 % 4 == 0 && (reinterpret_cast<uintptr_t>(C.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(C.e32) & 15) == 0;

@@ -67,3 +67,22 @@ def test_operator_at_tile_edges(n, op, tol):
     got = og.interior(case.download("res"))
     assert np.abs(got - want).max() <= tol * np.abs(want).max()
     case.close()
+
+
+@pytest.mark.parametrize("n", EDGES + [(22, 19, 12), (30, 33, 21)], ids=lambda n: "%dx%dx%d" % n)
+def test_mixed_solve_residual_at_tile_edges(n):
+    """The outer residual of the mixed solve (FP64, tiles of 32 x 16 columns, two rows per thread)
+    decides when it stops: the solution's residual under the oracle's operator must be the 1e-8 that
+    was asked for (twice that for the last correction's rounding; a wrong row is of order one)."""
+    N, L = tuple(k + 1 for k in n), tuple(k / 32.0 for k in n)
+    og, ig = O.Grid(N, L, (0, 0, 0)), I.Grid(N, L, (0, 0, 0))
+    case = I.Case(ig, precision=1)
+    b = og.product_div_grad(og.random(19).copy())
+    case.upload("res", b)
+    r = case.poisson("res", "pre", I.solver_params(precond=0, n_sweeps=4, tol_rel=1e-8, max_it=40, inner_tol_rel=1e-3,
+                                                   inner_max_it=4000))
+    assert r.status == 0
+    ax = og.product_div_grad(case.download("pre").copy())
+    d = og.interior(b) - og.interior(ax)
+    assert np.linalg.norm(d) <= 2e-8 * np.linalg.norm(og.interior(b))
+    case.close()

@@ -521,9 +521,9 @@ __global__ void __launch_bounds__(ENT, sizeof(T) == 4 ? 3 : 2) k_kr_x(const Kryl
     if (e_halted(sc)) continue;
     const Geom g = J.g;
     double v[3] = {0.0, 0.0, 0.0};
-    // FP32 only: the order of the partial sums differs, and the last bits of an FP64 solve's sums
-    // travel far over its iterations
-    if (sizeof(T) == 4 && J.vecu) {
+    // vecx: FP32 with the V-cycle only: the order of the partial sums differs, and the last bits of
+    // an FP64 solve's sums, or of any over the many iterations of a JOR solve, travel far
+    if (sizeof(T) == 4 && J.vecx) {
       const VTile<T> V(g, J.kc, b - ts[q]);
       if (V.act) {
         constexpr int W = VTile<T>::W, PH = VTile<T>::PH, U = 1;
@@ -1200,7 +1200,9 @@ __global__ void __launch_bounds__(AXNT, 3) k_kr_ax32(const KrylovJob<float>* __r
 // The FP32 operator on lists whose grids have n1 divisible by 4 and uniform x and z spacing
 // (every row of W[0] and of W[2] the same): the same collapsed 11-point product_div_grad as
 // k_kr_ax32, with the center weights of the three axes combined into one and every thread
-// owning one 16-byte vector of 4 consecutive x points of two neighbouring rows.
+// owning one 16-byte vector of 4 consecutive x points of NR neighbouring rows: two, and one (tiles
+// of 32 x 8 columns, groups of 4 planes) in solves with JOR sweeps, whose partial sums keep their
+// order.  The following is for two.
 //
 // A block of 8 x 8 threads owns one 32 x 16-column tile over kc planes.  The 5-wide halo of each
 // plane of the tile is staged by 16-byte cp.async into a ring of AXV_R slots (48 x 26 floats:
@@ -1226,29 +1228,30 @@ __global__ void __launch_bounds__(AXNT, 3) k_kr_ax32(const KrylovJob<float>* __r
 constexpr int AXV_TX = ETX / 4, AXV_NT = AXV_TX * ETY;   // 8 x 8 threads, 4 columns each
 constexpr int AXV_HX = 8;                                // staged columns left of the tile
 constexpr int AXV_W = ETX + 16;                          // staged row: 8 + 32 + 8 (5 needed each side)
-constexpr int AXV_NR = 2;                                // rows per thread
-constexpr int AXV_Y = AXV_NR * ETY;                      // rows per tile
-constexpr int AXV_H = AXV_Y + 10;                        // staged rows
 constexpr int AXV_CR = AXV_W / 4;                        // 16-byte chunks per row
-constexpr int AXV_NCH = AXV_CR * AXV_H;                  // chunks per plane
-constexpr int AXV_PER = (AXV_NCH + AXV_NT - 1) / AXV_NT; // chunks per thread and plane
-constexpr int AXV_PLANE = AXV_W * AXV_H;                 // floats per slot
-constexpr int AXV_PP = ETX * AXV_Y;                      // partner floats per slot
-constexpr int AXV_B = 2;                                 // planes per step
-constexpr int AXV_G = 2;                                 // groups of AXV_B planes in the ring
-constexpr int AXV_R = AXV_B * AXV_G;                     // ring slots
-constexpr int AXV_ZW = AXV_B + 10;                       // z window (planes t-5 .. t+AXV_B+4)
-static_assert((AXV_PLANE * 4) % 16 == 0 && (AXV_PP * 4) % 16 == 0, "slots must keep 16-byte alignment");
-constexpr size_t axv_smem_bytes() { return sizeof(float) * (size_t)AXV_R * (AXV_PLANE + AXV_PP); }
+template <int NR>
+struct Axv {                                             // NR rows per thread
+  static constexpr int Y = NR * ETY, H = Y + 10;         // rows per tile, staged rows
+  static constexpr int NCH = AXV_CR * H;                 // chunks per plane
+  static constexpr int PER = (NCH + AXV_NT - 1) / AXV_NT; // chunks per thread and plane
+  static constexpr int PLANE = AXV_W * H, PP = ETX * Y;  // floats and partner floats per slot
+  static constexpr int B = NR == 1 ? 4 : 2, G = 2, R = B * G; // planes per step, groups in the ring, slots
+  static constexpr int ZW = B + 10;                      // z window (planes t-5 .. t+B+4)
+  static constexpr size_t smem() { return sizeof(float) * (size_t)R * (PLANE + PP); }
+  static_assert((PLANE * 4) % 16 == 0 && (PP * 4) % 16 == 0, "slots must keep 16-byte alignment");
+};
 
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-template <int MODE>
-__global__ void __launch_bounds__(AXV_NT, 4) k_kr_ax32v(const KrylovJob<float>* __restrict__ jobs,
+template <int MODE, int AXV_NR>
+__global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const KrylovJob<float>* __restrict__ jobs,
                                                         const int* __restrict__ ts, int nj, int ntiles,
                                                         double* __restrict__ partial) {
   static_assert(MODE >= 0 && MODE <= 2, "FP32 operator modes: 0 residual, 1 alpha, 2 omega");
+  using AX = Axv<AXV_NR>;
+  constexpr int AXV_Y = AX::Y, AXV_NCH = AX::NCH, AXV_PER = AX::PER, AXV_PLANE = AX::PLANE, AXV_PP = AX::PP;
+  constexpr int AXV_B = AX::B, AXV_G = AX::G, AXV_R = AX::R, AXV_ZW = AX::ZW;
   extern __shared__ __align__(16) unsigned char axv_smem[];
   float* ring = reinterpret_cast<float*>(axv_smem);
   float* pring = ring + (size_t)AXV_R * AXV_PLANE;
@@ -3229,7 +3232,7 @@ __global__ void __launch_bounds__(ENT) k_mx_apply(const MixJob* __restrict__ job
 
 // grids of the vector operator kernels: the blocks resident at once on the device (a grid-stride
 // kernel given more would leave its last blocks to run after the others, one tile step behind)
-int g_axv_grid = 0, g_axd_grid = 0, g_axd3_grid = 0;
+int g_axv_grid[2] = {0, 0}, g_axd_grid = 0, g_axd3_grid = 0;
 int g_axs32_grid = 0, g_axs64_grid = 0;  // the same of the staged operator kernels
 // the operator kernels use more than 48 KB of dynamic shared memory: opt in once per process
 // and device
@@ -3249,9 +3252,12 @@ void ax_attributes() {
   cudaFuncSetAttribute(k_kr_ax64v<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
   cudaFuncSetAttribute(k_kr_ax64v<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
   cudaFuncSetAttribute(k_kr_ax64v<3, AXD_NR3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<AXD_NR3>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axv_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax32v<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axv_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax32v<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axv_smem_bytes());
+  cudaFuncSetAttribute(k_kr_ax32v<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
   auto occ = [](auto kernel, int threads, size_t smem) {
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) != cudaSuccess || nb < 1) nb = 1;
@@ -3260,8 +3266,10 @@ void ax_attributes() {
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (nsm <= 0) nsm = 148;
-  g_axv_grid = nsm * std::min({occ(k_kr_ax32v<0>, AXV_NT, axv_smem_bytes()), occ(k_kr_ax32v<1>, AXV_NT, axv_smem_bytes()),
-                               occ(k_kr_ax32v<2>, AXV_NT, axv_smem_bytes())});
+  g_axv_grid[0] = nsm * std::min({occ(k_kr_ax32v<0, 1>, AXV_NT, Axv<1>::smem()), occ(k_kr_ax32v<1, 1>, AXV_NT, Axv<1>::smem()),
+                                  occ(k_kr_ax32v<2, 1>, AXV_NT, Axv<1>::smem())});
+  g_axv_grid[1] = nsm * std::min({occ(k_kr_ax32v<0, 2>, AXV_NT, Axv<2>::smem()), occ(k_kr_ax32v<1, 2>, AXV_NT, Axv<2>::smem()),
+                                  occ(k_kr_ax32v<2, 2>, AXV_NT, Axv<2>::smem())});
   g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0, 1>, AXD_NT, Axd<1>::smem()), occ(k_kr_ax64v<1, 1>, AXD_NT, Axd<1>::smem()),
                                occ(k_kr_ax64v<2, 1>, AXD_NT, Axd<1>::smem())});
   g_axd3_grid = nsm * occ(k_kr_ax64v<3, AXD_NR3>, AXD_NT, Axd<AXD_NR3>::smem());
@@ -3314,10 +3322,13 @@ const dim3 kAxBlock(ETX, AXTY);  // k_kr_ax: two rows per thread
 // 1 all, 2 some), by the 16-byte staged, stepped kernel for the others; FP64 alike
 template <typename T, int MODE>
 void launch_ax(int grid, const KrylovJob<T>* J, const int* ts, int n, int ntiles, double* partial, cudaStream_t s,
-               int vec) {
+               int vec, int rows = 1) {
   if constexpr (std::is_same<T, float>::value && MODE <= 2) {
-    const int gv = g_axv_grid > 0 ? std::min(g_axv_grid, ntiles) : grid;
-    if (vec != 0) k_kr_ax32v<MODE><<<gv, dim3(AXV_TX, ETY), axv_smem_bytes(), s>>>(J, ts, n, ntiles, partial);
+    const int slots = g_axv_grid[rows - 1], gv = slots > 0 ? std::min(slots, ntiles) : grid;
+    if (vec != 0 && rows == 2)
+      k_kr_ax32v<MODE, 2><<<gv, dim3(AXV_TX, ETY), Axv<2>::smem(), s>>>(J, ts, n, ntiles, partial);
+    else if (vec != 0)
+      k_kr_ax32v<MODE, 1><<<gv, dim3(AXV_TX, ETY), Axv<1>::smem(), s>>>(J, ts, n, ntiles, partial);
     if (vec != 1) k_kr_ax32<MODE><<<grid, kAxBlock, axa_smem_bytes(), s>>>(J, ts, n, ntiles, partial);
     if (vec == 2) prof::count(1);  // two launches where the callers count one
   } else {
@@ -3560,14 +3571,17 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       bool ual = J.g.n1 % VecT<T>::W == 0;
       for (const void* q : uf) ual = ual && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
       J.vecu = ual ? 1 : 0;
+      J.vecx = ual && std::is_same<T, float>::value && use_mg;
       nv += J.vec;
     }
     kr_vec_ = nv == 0 ? 0 : (nv == n ? 1 : 2);
-    // FP64 with JOR sweeps (about 100 iterations) keeps kc: so many iterations carry the last bits
-    // of the inner products up to the solve's tolerance, and another depth would sum them in
-    // another order
+    // Solves with JOR sweeps (some 100 iterations) keep kc, one row per thread in the operator and the
+    // x update's point order: their inner products cancel by many digits, and so many iterations
+    // carry the last bits of the sums up to the solve's tolerance (FP32 on 59 x 47 x 83: with shallow
+    // tiles one solve in some 60 ended 4e-7 of max|p| from the deep tiles' result).
     constexpr bool f32 = std::is_same<T, float>::value;
-    const bool adapt = f32 || use_mg;
+    const bool adapt = use_mg;
+    kr_rows_ = f32 && use_mg ? 2 : 1;
     auto depths = [&](auto slots, auto rows) {
       long long tiles = 0;
       for (int c = 0; c < n; ++c) {
@@ -3578,9 +3592,9 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       return tiles;
     };
     const long long ta = depths([&](const KrylovJob<T>& J) {
-      return std::min(J.vec ? (f32 ? g_axv_grid : g_axd_grid) : (f32 ? g_axs32_grid : g_axs64_grid),
+      return std::min(J.vec ? (f32 ? g_axv_grid[kr_rows_ - 1] : g_axd_grid) : (f32 ? g_axs32_grid : g_axs64_grid),
                       device_sms() * kVecBlocksPerSm );
-    }, [&](const KrylovJob<T>& J) { return f32 && J.vec ? AXV_Y : ETY; });
+    }, [&](const KrylovJob<T>& J) { return f32 && J.vec ? kr_rows_ * ETY : ETY; });
     kr_list_ = arena_.add(kj, kt);
     const long long tv = depths([&](const KrylovJob<T>&) { return device_sms() * kVecBlocksPerSm; },
                                 [](const KrylovJob<T>&) { return ETY; });
@@ -4044,11 +4058,11 @@ void Engine<T>::enqueue_iteration() {
   const double fb = sizeof(T) * cells_[kr_list_];
   IMPACT_PROF(prof::K_P_UPDATE, 4 * fb, s, (k_kr_p<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(0);
-  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_)));
+  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_, kr_rows_)));
   k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 1, 0, EFIN_ALPHA, scal_, nullptr);
   IMPACT_PROF(prof::K_R_UPDATE, 3 * fb, s, (k_kr_r<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(1);
-  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_)));
+  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_, kr_rows_)));
   k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 2, 0, EFIN_OMEGA, scal_, nullptr);
   IMPACT_PROF(prof::K_X_UPDATE, 8 * fb, s, (k_kr_x<T><<<gw, kBlock, 0, s>>>(JW, W.ts, n, W.ntiles, partial_)));
   k_efin<<<n, 256, 0, s>>>(W.ts, partial_, 3, 1, EFIN_NORMS, scal_, nullptr);
@@ -4098,7 +4112,7 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
     prof::count(1);
   } else {
     if (!zero_phi) {
-      launch_ax<T, 0>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_);
+      launch_ax<T, 0>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_);
       prof::count(1);
     }
     IMPACT_PROF(prof::K_KR_INIT, 4.0 * sizeof(T) * cells_[kr_list_], s_,
@@ -4194,7 +4208,7 @@ int Engine<T>::apply_operator() {
   if (e != cudaSuccess) return impact_set_error(e, "engine scalars", __FILE__, __LINE__);
   const DevList& K = arena_.lists[kr_list_];
   const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
-  launch_ax<T, 0>(grid_for(K.ntiles), J, K.ts, n, K.ntiles, partial_, s_, kr_vec_);
+  launch_ax<T, 0>(grid_for(K.ntiles), J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_);
   prof::count(1);
   e = cudaStreamSynchronize(s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine operator", __FILE__, __LINE__);
@@ -4247,11 +4261,11 @@ int Engine<T>::bench(int kind, int iters, double* ms, double* bytes) {
     }
     case 5:
       by = 3 * sz * fc;
-      f = [&]() { launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_); };
+      f = [&]() { launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_); };
       break;
     case 6:
       by = 3 * sz * fc;
-      f = [&]() { launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_); };
+      f = [&]() { launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_); };
       break;
     case 7:
       by = 8 * sz * fc;

@@ -76,6 +76,7 @@ struct KrylovJob {
   int xuni;       // 1: every x row of W[0] is the same (uniform x spacing)
   int vec;        // the operator of this job runs in the vector kernel
   int vecu;       // the vector updates move 16 bytes per thread (n1 a multiple of the vector, aligned fields)
+  int vecx;       // so does the x update (its partial sums in another order)
   const T* bb;
   T* phi;
   T *rr, *rh, *pp, *Ap, *Ar, *z1, *z2;
@@ -224,6 +225,7 @@ class Engine {
   std::vector<double> cells_, cells_f_, cells_c_;
   std::vector<char> fast_;  // per list: every job vectorised with uniform z (k_lv_fast)
   int tail_blocks_ = 1;     // blocks per coarse tail: 1, or a cluster cut into z slabs
+  int kr_rows_ = 1;         // rows per thread of the FP32 vector operator
   int kr_vec_ = 0;          // FP32 Krylov list: jobs in the vector kernel -- 0 none, 1 all, 2 some
 };
 

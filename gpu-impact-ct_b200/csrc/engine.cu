@@ -2465,8 +2465,8 @@ __global__ void __launch_bounds__(ENT, sizeof(T) == 4 ? 3 : 2) k_lv_prolong(cons
 // Every point is evaluated with the operations of the one-sweep kernels (jres / jsweep / jinit
 // / jresid), so the fused phase gives the same iterate bit for bit.
 // Outputs: PRE (INIT, RES): B = x_NSW and C = residual; POST and the JOR preconditioner (INIT): B =
-// x_NSW.  The JOR preconditioner's 4 sweeps as one launch instead of 4 (a mixed step on
-// 59 x 47 x 83 29.9 -> 23.7 ms, an FP64 step on 64 x 64 x 128 35.6 -> 28.7 ms).
+// x_NSW.  The JOR preconditioner's 4 sweeps as one launch instead of 4 (an FP64 step
+// on 64 x 64 x 128 35.6 -> 28.7 ms).
 constexpr int MPF = 2;  // planes staged ahead of the newest one in use
 const dim3 kMBlock(32, MNT / 32);
 static_assert(MNT / 32 <= 16, "one named barrier per pair of neighbouring warps (ids 1..15)");
@@ -3578,7 +3578,7 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     // Solves with JOR sweeps (some 100 iterations) keep kc, one row per thread in the operator and the
     // x update's point order: their inner products cancel by many digits, and so many iterations
     // carry the last bits of the sums up to the solve's tolerance (FP32 on 59 x 47 x 83: with shallow
-    // tiles one solve in some 60 ended 4e-7 of max|p| from the deep tiles' result).
+    // tiles one step in some 30 ended 4e-7 of max|p| from the deep tiles' result).
     constexpr bool f32 = std::is_same<T, float>::value;
     const bool adapt = use_mg;
     kr_rows_ = f32 && use_mg ? 2 : 1;

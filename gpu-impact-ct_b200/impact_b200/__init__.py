@@ -241,7 +241,7 @@ def solver_params(tol_rel=1e-8, tol_abs_inf=0.0, max_it=2000, n_sweeps=4, omega=
     tile_kc: most z-planes per tile of the solver kernels (0: library default; small grids take fewer).  smooth_unfused: 1 runs
     every sweep (V-cycle, JOR preconditioner) as its own launch instead of one fused kernel per phase.
     bottom_cheb: d > 0 replaces the coarsest level's Jacobi sweeps by d Chebyshev steps (fused
-    schedule, coarsest level within the one-block tail)."""
+    schedule, coarsest level within the fused tail)."""
     return SolverParams(tol_rel, tol_abs_inf, max_it, n_sweeps, omega, init_yes, check_every,
                         inner_tol_rel, inner_max_it, precond, mg_down, mg_up, mg_bottom, tile_kc, smooth_unfused,
                         bottom_cheb)

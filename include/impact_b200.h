@@ -287,7 +287,7 @@ typedef struct {
                           sweeps, then mg_bottom more (relax_bottom, mod_solvers.f90:420-450);
                           d > 0: d steps of the Chebyshev semi-iteration of the Jacobi-scaled
                           coarsest operator from x = 0 instead (a fixed polynomial in A, so the
-                          preconditioner stays linear), in the one-block coarse tail, on cases whose
+                          preconditioner stays linear), in the fused coarse tail, on cases whose
                           coarsest level fits there.  For hierarchies that stop at a large coarsest
                           level (n = 8 x odd); no counterpart in the reference */
 } impact_b200_solver_params;

@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "kernels.cuh"
 #include "prof.cuh"
 
 namespace impact {
@@ -3302,16 +3303,6 @@ void ax_attributes() {
   done[dev] = true;
 }
 
-int g_sms = 0;
-inline int device_sms() {
-  if (g_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_sms <= 0) g_sms = 148;
-  }
-  return g_sms;
-}
 inline int grid_for(int ntiles) {
   const int cap = device_sms() * 8;
   return ntiles < cap ? ntiles : cap;

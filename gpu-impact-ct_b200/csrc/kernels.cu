@@ -11,7 +11,20 @@
 #include "stencil25d.cuh"
 #include "stencil3.cuh"
 
+#include <atomic>
+
 namespace impact {
+
+int device_sms() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  n = known[dev].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
 
 constexpr int BX = 32, BY = 8;
 

@@ -4,6 +4,9 @@
 
 namespace impact {
 
+// SMs of the current device (asked for once per device)
+int device_sms();
+
 // ---- one-axis stencils as streaming passes (march.cu): out (=, += for OP 1) the CNT-point
 // stencil from LO along axis a (0 x, 1 y, 2 z) of f; OP 2 the upwind term (cA where pp >= 0,
 // else cB; overwrite when first).

@@ -12,18 +12,19 @@
 //   a = x:      marches z with the coefficient rows of its points loaded once; each plane takes the
 //               aligned vectors of the row that its points' stencils span (V = 1: its taps).
 // Threads are numbered along the vectors of a row and then along the rows, so that narrow grids
-// fill their warps, and a segment is as short as 4 steps where a small grid would otherwise leave
-// SMs idle.  Periodic wrapping is applied to the coordinate along a only; each point sums its
-// terms in table order with fused multiply-adds.
+// fill their warps, and a segment is as short as one step where a small grid would otherwise leave
+// SMs idle (march_seg, shape.h).  Periodic wrapping is applied to the coordinate along a only; each
+// point sums its terms in table order with fused multiply-adds.
 //
 // Bound by DRAM on large grids and by latency on small ones.  256 x 256 x 512 FP64 (270 MB a
-// field, 6.5 TB/s copy bandwidth): the y and z interpolations 96 us (5.6 TB/s; 118 - 125 us with one
-// step's loads at a time and segments of 64), along x 127 us, the upwind terms 244 / 196 us (234 /
-// 252), axpby 126 us (146).  Segments beyond 16 steps lost 8 % on every pass there.  187 x 131 x 157
-// FP32, rows of odd length: 12.6 us (one point per thread with its taps wrapped one by one: 25), the
-// upwind terms 19 - 21 us (29).  64 x 64 x 128 FP64: JOR sweep 6.4 us (10.8), interpolations 5.2 us
-// (8.4).
+// field, 6.5 TB/s copy bandwidth): the y and z interpolations 90 and 87 us (6.0 and 6.2 TB/s; 95 and 94
+// with blocks of 256 threads, 118 - 125 with one step's loads at a time and segments of 64), along x
+// 113 us (125 with spilled planes), the upwind terms 234 / 198 us, axpby 123 us.  187 x 131 x 157
+// FP32, rows of odd length: 12.4 us (one point per thread with its taps wrapped one by one: 25), the
+// upwind terms 16.5 - 18.6 us (29 - 31).  64 x 64 x 128 FP64: JOR sweep 6.3 us (10.7), interpolations
+// 4.7 us (8.3).
 #include "kernels.cuh"
+#include "shape.h"
 
 namespace impact {
 namespace {
@@ -98,7 +99,7 @@ __device__ __forceinline__ T point_value(const T* __restrict__ ca, const T* __re
   return s;
 }
 
-constexpr int MT = 256;  // threads per block
+constexpr int MT = 128;  // threads per block
 
 template <typename T, int V>
 __device__ __forceinline__ void ldv(const T* p, T (&o)[V]) {
@@ -126,7 +127,9 @@ template <typename T, int V, int LO, int CNT, int OP>
 __global__ void __launch_bounds__(MT) k_march_yz(int a, Geom g, const T* __restrict__ cA, const T* __restrict__ cB,
                                                  const T* __restrict__ f, const T* __restrict__ pp,
                                                  T* __restrict__ out, int first, int seg) {
-  constexpr int U = 4, NW = CNT - 1 + U;
+  // steps at a time: 4, or 2 where the operands of 4 take the registers of too many warps
+  constexpr bool wide = OP == 1 ? V == 2 : (OP == 2 && (V == 4 || (V == 1 && sizeof(T) == 8)));
+  constexpr int U = wide ? 2 : 4, NW = CNT - 1 + U;
   const int nvx = g.n1 / V;
   const unsigned idx = blockIdx.x * MT + threadIdx.x;
   const int o = (int)(idx / (unsigned)nvx) + 1;
@@ -175,12 +178,22 @@ __global__ void __launch_bounds__(MT) k_march_yz(int a, Geom g, const T* __restr
   }
 }
 
+// Resident blocks of k_march_x, which set its registers: as many as hold the coefficient rows and the
+// planes in flight without spills (vectors one plane at a time: 64 registers.  With 2 or 4 planes in those
+// 64 a thread spilled 24 to 268 bytes: 128^3 FP64 20.5 us, now 8.3; 192^3 FP32 22.6, now 12.5)
+template <typename T, int V, int OP>
+constexpr int march_x_blocks() {
+  if (V > 1) return OP == 2 ? 4 : 8;
+  return OP != 2 ? 4 : (sizeof(T) == 8 ? 6 : 8);
+}
 // a = 0 (x): thread (vector, row j) marches z
 template <typename T, int V, int LO, int CNT, int OP>
-__global__ void __launch_bounds__(MT, V == 1 ? (OP == 2 ? 4 : 2) : (OP == 2 ? 2 : 4)) k_march_x(Geom g, const T* __restrict__ cA, const T* __restrict__ cB,
-                                                const T* __restrict__ f, const T* __restrict__ pp,
-                                                T* __restrict__ out, int first, int seg) {
-  constexpr int U = OP == 2 ? 1 : (sizeof(T) == 8 && V > 1 ? 2 : 4);
+__global__ void __launch_bounds__(MT, march_x_blocks<T, V, OP>()) k_march_x(Geom g, const T* __restrict__ cA,
+                                                                            const T* __restrict__ cB,
+                                                                            const T* __restrict__ f,
+                                                                            const T* __restrict__ pp,
+                                                                            T* __restrict__ out, int first, int seg) {
+  constexpr int U = OP == 2 || V > 1 ? 1 : 4;
   constexpr int FV = (LO - (V - 1)) / V;          // floor(LO / V) for LO < 0
   constexpr int LV = (V - 1 + LO + CNT - 1) / V;  // floor of the last position / V (>= 0)
   constexpr int NV = LV - FV + 1;
@@ -243,7 +256,7 @@ __global__ void __launch_bounds__(MT, V == 1 ? (OP == 2 ? 4 : 2) : (OP == 2 ? 2 
 // out = omega (bb - sum of the six off-diagonal terms of cdg) / diag + (1 - omega) rel.  Thread
 // (vector, row j) marches z with the column's rel at k-1..k+1 in registers.
 template <typename T, int V>
-__global__ void __launch_bounds__(MT) k_jacobi_march(Geom g, const T* __restrict__ c1, const T* __restrict__ c2,
+__global__ void __launch_bounds__(MT, 5) k_jacobi_march(Geom g, const T* __restrict__ c1, const T* __restrict__ c2,
                                                      const T* __restrict__ c3, T omega, const T* __restrict__ bb,
                                                      const T* __restrict__ rel, T* __restrict__ out, int seg) {
   constexpr int U = 2;
@@ -336,22 +349,21 @@ __global__ void __launch_bounds__(MT) k_axpby(Geom g, T a, T b, const T* __restr
   }
 }
 
+template <typename T>
+__global__ void __launch_bounds__(256) k_axpby_points(Geom g, T a, T b, const T* __restrict__ x,
+                                                      const T* __restrict__ y, T* __restrict__ z) {
+  const int i = blockIdx.x * 32 + threadIdx.x + 1, j = blockIdx.y * 8 + threadIdx.y + 1;
+  if (i > g.n1 || j > g.n2) return;
+  const long long p = off(g, i, j, blockIdx.z + 1);
+  z[p] = fmaT(a, x[p], mulT(b, y[p]));
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// steps per marching thread, 4 .. 16 in whole blocks of 4: as many as leave about `per_sm` threads
-// per SM (a segment re-reads the CNT - 1 values before it, mostly from L2, and pays its set-up
-// once).  Along x the set-up loads the coefficient rows of the thread's points, strided over the
-// warp, which for whole vectors costs as much as some ten planes: at least 8 steps there (16 with
-// the upwind term's two tables in FP32), and half the threads.
-inline int march_seg(long long threads, int na, int per_sm, int least) {
-  long long seg = threads * na / (148LL * per_sm) / 4 * 4;
-  seg = seg < least ? least : (seg > 16 ? 16 : seg);
-  return (int)std::min<long long>(seg, na);
-}
-// grid of a pass: threads (vectors of one row x no rows), na steps
-inline dim3 march_grid(const Geom& g, int V, int no, int na, int& seg, int per_sm = 1024, int least = 4) {
+// grid of a pass: threads (vectors of one row x no rows), na steps, segments by march_seg
+inline dim3 march_grid(const Geom& g, int V, int no, int na, int& seg, int per_sm = 320, int most = 8) {
   const long long threads = (long long)(g.n1 / V) * no;
-  seg = march_seg(threads, na, per_sm, least);
+  seg = march_seg(threads, na, device_sms(), per_sm, most);
   return dim3((unsigned)((threads + MT - 1) / MT), (na + seg - 1) / seg);
 }
 
@@ -360,7 +372,7 @@ void march1(int a, const Geom& g, const T* cA, const T* cB, const T* f, const T*
             cudaStream_t s) {
   int seg = 0;
   if (a == 0) {
-    const dim3 grid = V > 1 ? march_grid(g, V, g.n2, g.n3, seg, 512, OP == 2 && V == 4 ? 16 : 8) : march_grid(g, V, g.n2, g.n3, seg);
+    const dim3 grid = march_grid(g, V, g.n2, g.n3, seg, 256, 16);
     k_march_x<T, V, LO, CNT, OP><<<grid, MT, 0, s>>>(g, cA, cB, f, pp, out, first, seg);
   } else {
     const dim3 grid = march_grid(g, V, a == 2 ? g.n2 : g.n3, a == 2 ? g.n3 : g.n2, seg);
@@ -397,11 +409,16 @@ template <typename T>
 void launch_axpby(const Geom& g, T a, T b, const T* x, const T* y, T* z, cudaStream_t s) {
   constexpr int W = V16<T>::W;
   int seg = 0;
-  if (g.n1 % W == 0 && aligned16(x) && aligned16(y) && aligned16(z)) {
-    const dim3 grid = march_grid(g, W, g.n2, g.n3, seg);
+  // fewer vectors than 320 threads per SM (46 points a side in FP64, 57 in FP32): all latency, one point
+  // per thread without a march (32 x 32 x 64: 3.1 us against 3.6 to 4.1)
+  if ((long long)g.n1 * g.n2 * g.n3 < 320LL * W * device_sms()) {
+    const dim3 grid((g.n1 + 31) / 32, (g.n2 + 7) / 8, g.n3);
+    k_axpby_points<T><<<grid, dim3(32, 8), 0, s>>>(g, a, b, x, y, z);
+  } else if (g.n1 % W == 0 && aligned16(x) && aligned16(y) && aligned16(z)) {
+    const dim3 grid = march_grid(g, W, g.n2, g.n3, seg, 640);
     k_axpby<T, W><<<grid, MT, 0, s>>>(g, a, b, x, y, z, seg);
   } else {
-    const dim3 grid = march_grid(g, 1, g.n2, g.n3, seg);
+    const dim3 grid = march_grid(g, 1, g.n2, g.n3, seg, 640);
     k_axpby<T, 1><<<grid, MT, 0, s>>>(g, a, b, x, y, z, seg);
   }
 }

@@ -1,0 +1,46 @@
+"""Launch shapes of the streaming passes (csrc/shape.h, compiled here for the host) and the registers
+of their kernels: a small grid may not be left to a few long threads, and no kernel of the one-axis
+passes may spill."""
+import ctypes as C
+import os
+import re
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "gpu-impact-ct_b200", "csrc")
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def shape(tmp_path_factory):
+    out = tmp_path_factory.mktemp("shape") / "libshape_host.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", CSRC, os.path.join(ROOT, "tests", "shape_host.cpp"),
+                    "-o", str(out)], check=True)
+    lib = C.CDLL(str(out))
+    lib.host_march_seg.restype, lib.host_march_seg.argtypes = C.c_int, [C.c_longlong] + [C.c_int] * 4
+    return lib
+
+
+@pytest.mark.parametrize("per_sm,most", [(320, 8), (256, 16)], ids=["y-z", "x"])
+@pytest.mark.parametrize("vector", [1, 2, 4])
+@pytest.mark.parametrize("n", [8, 9, 16, 24, 33, 48, 56, 57, 64, 81, 128, 256])
+def test_a_marching_pass_fills_the_device_before_it_lengthens_its_segments(shape, n, vector, per_sm, most):
+    threads, na = -(-n // vector) * n, n
+    seg = shape.host_march_seg(threads, na, SMS, per_sm, most)
+    assert 1 <= seg <= min(most, na)
+    launched = threads * -(-na // seg)
+    assert seg == 1 or launched >= SMS * per_sm
+    assert seg == most or 2 * seg > na or threads * na < SMS * per_sm * 2 * seg
+
+
+@pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc")
+def test_one_axis_kernels_do_not_spill(tmp_path):
+    r = subprocess.run(["nvcc", "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, "-I", os.path.join(ROOT, "include"),
+                        "-gencode", "arch=compute_100a,code=sm_100a", "-Xptxas", "-v", "-cubin", "-o", str(tmp_path / "march.cubin"),
+                        os.path.join(CSRC, "march.cu")], capture_output=True, text=True, check=True)
+    kernels = re.findall(r"Compiling entry function '(\S*k_march_\S*)'.*?(\d+) bytes spill stores, (\d+) bytes spill loads", r.stderr, re.S)
+    assert len(kernels) == 32  # 4 operators, 2 orientations, vectors and points, 2 types
+    assert [k for k in kernels if k[1:] != ("0", "0")] == []

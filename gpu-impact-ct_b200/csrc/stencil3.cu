@@ -12,14 +12,16 @@
 // The passes these replace gave every thread one point: 18 scalar loads per point and, for the
 // x stencil, one strided table load per tap, which cost more of the L1 data path than the fields
 // themselves.  Now bound by that path still (65 % of its cycles; 12 vector loads per 2 points) and by
-// the latency of 16 warps per SM.  256 x 256 x 512 FP64: Helmholtz 250 us (295), divergence2 257 us
-// (389); 128 x 128 x 224 FP32: 17 us (19), 15 us (41); 187 x 131 x 157 FP32: 31 us (50), 27 us (43).
+// the latency of 16 warps per SM.  256 x 256 x 512 FP64: Helmholtz 253 us (294), divergence2 263 us
+// (390); 128 x 128 x 224 FP32: 16.5 us (19), 16 us (40); 187 x 131 x 157 FP32: 31 us (51), 27 us (43).
 // 384 x 384 x 768 FP64, in the time step: interpolate_vel 1.09 ms (1.44; with get_dtime's bound
 // in the same pass, which took another 1.94), divergence2 0.82 ms (1.33), projection 1.35 (1.44).
 // The same with the tiles staged in shared memory by cp.async, four planes in a ring: 255 and
 // 262 us, and slower on small grids.
 #include <algorithm>
 
+#include "kernels.cuh"
+#include "shape.h"
 #include "stencil3.cuh"
 
 namespace impact {
@@ -346,29 +348,15 @@ bool tri_vectorable(const Geom& g, int elt, const void* const* fields, int n) {
   return ok;
 }
 
-// The depth minimises waves of blocks over the resident ones (about 3 per SM) x (planes + the 6
-// planes' time of a block's set-up): deep blocks on large grids (fewer window loads), blocks of
-// 4 planes where a small grid would leave SMs idle.
 TriGrid tri_grid(const Geom& g, int elt, bool vec, long long total_points) {
   TriGrid t;
   t.vec = vec ? 1 : 0;
   const int nx = vec ? 16 * (16 / elt) : 32, ny = vec ? 16 : 8;
   t.gx = (g.n1 + nx - 1) / nx;
   t.gy = (g.n2 + ny - 1) / ny;
-  const double cells = (double)g.n1 * g.n2 * g.n3;
-  const double share = total_points > 0 ? cells / (double)total_points : 1.0;
-  const double slots = std::max(1.0, 148.0 * (vec ? 3 : 6) * share);
-  double best = -1.0;
-  t.kz = 64;
-  for (int kz : {64, 48, 32, 24, 16, 12, 8, 4, 2, 1}) {
-    const double blocks = (double)t.gx * t.gy * ((g.n3 + kz - 1) / kz);
-    const double waves = blocks / slots <= 1.0 ? 1.0 : (blocks / slots <= 4.0 ? (double)(long long)(blocks / slots + 0.999999) : blocks / slots);
-    const double cost = waves * (std::min(kz, g.n3) + 6);
-    if (best < 0.0 || cost < best) {
-      best = cost;
-      t.kz = kz;
-    }
-  }
+  // a grid of a batch: its share of the SMs, by its points
+  const double share = total_points > 0 ? (double)g.n1 * g.n2 * g.n3 / (double)total_points : 1.0;
+  t.kz = tri_depth((double)t.gx * t.gy, g.n3, device_sms() * share, vec);
   t.gz = (g.n3 + t.kz - 1) / t.kz;
   return t;
 }

@@ -1,4 +1,4 @@
-// stencil3.cuh -- the passes whose stencils run along all three axes, as staged z-marching passes
+// stencil3.cuh -- the passes whose stencils run along all three axes, as z-marching passes
 // (stencil3.cu; internal):
 //
 //   divergence2        D1 u + D2 v + D3 w                                  (mod_diff.f90:130-215)
@@ -47,7 +47,8 @@ struct TriGrid {
 bool tri_vectorable(const Geom& g, int elt, const void* const* fields, int n);
 // the pass's fields exceed what the L2 keeps between its planes
 bool tri_ahead(const Geom& g, int elt);
-// total: grids advanced by the same launch share the GPU (0: this grid alone)
+// depth by tri_depth (shape.h).  total_points: grids advanced by the same launch share the GPU (0: this
+// grid alone)
 TriGrid tri_grid(const Geom& g, int elt, bool vec, long long total_points = 0);
 
 template <int KIND, typename T, typename TO>

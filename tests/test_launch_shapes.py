@@ -1,6 +1,6 @@
 """Launch shapes of the streaming passes (csrc/shape.h, compiled here for the host) and the registers
-of their kernels: a small grid may not be left to a few long threads, and no kernel of the one-axis
-passes may spill."""
+of their kernels: a small grid may not be left to a few long threads or blocks, a large one not to a
+nearly empty last round, and no kernel of the one-axis passes may spill."""
 import ctypes as C
 import os
 import re
@@ -21,6 +21,7 @@ def shape(tmp_path_factory):
                     "-o", str(out)], check=True)
     lib = C.CDLL(str(out))
     lib.host_march_seg.restype, lib.host_march_seg.argtypes = C.c_int, [C.c_longlong] + [C.c_int] * 4
+    lib.host_tri_depth.restype, lib.host_tri_depth.argtypes = C.c_int, [C.c_double, C.c_int, C.c_double, C.c_int]
     return lib
 
 
@@ -34,6 +35,27 @@ def test_a_marching_pass_fills_the_device_before_it_lengthens_its_segments(shape
     launched = threads * -(-na // seg)
     assert seg == 1 or launched >= SMS * per_sm
     assert seg == most or 2 * seg > na or threads * na < SMS * per_sm * 2 * seg
+
+
+def test_a_three_axis_pass_prefers_one_full_round(shape):
+    # tiles of 32 x 16 points of two doubles: one round of two blocks per SM
+    for n, kz in ((112, 12), (128, 16), (160, 32), (192, 48)):
+        gxy = -(-n // 32) * -(-n // 16)
+        assert shape.host_tri_depth(gxy, n, SMS, 1) == kz
+        assert SMS < gxy * -(-n // kz) <= 2 * SMS
+
+
+@pytest.mark.parametrize("vec", [0, 1])
+@pytest.mark.parametrize("n", [8, 16, 24, 48, 64])
+def test_a_three_axis_pass_on_a_small_grid_takes_shallow_blocks(shape, n, vec):
+    gxy = -(-n // 32) * -(-n // (16 if vec else 8))
+    kz = shape.host_tri_depth(gxy, n, SMS, vec)
+    assert gxy * -(-n // kz) >= min(SMS / 2, gxy * n)
+
+
+@pytest.mark.parametrize("share", [1.0, 0.25, 0.001])
+def test_depths_of_a_batch_grow_as_its_share_shrinks(shape, share):
+    assert shape.host_tri_depth(8, 64, SMS * share, 1) >= shape.host_tri_depth(8, 64, SMS, 1)
 
 
 @pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc")

@@ -22,6 +22,7 @@
 #include "engine.cuh"
 #include "kernels.cuh"
 #include "prof.cuh"
+#include "shape.h"
 
 namespace impact {
 
@@ -886,15 +887,16 @@ __global__ void __launch_bounds__(AXNT, 2) k_kr_ax(const KrylovJob<T>* __restric
     else
       walk(std::false_type{});
     cp_wait<0>();
+    double* const pt = partial + (long long)(J.us + t0) * 4;
     if (MODE == 1) {
       double v[1] = {v0};
-      tile_partials<1, 0, AXNT>(v, partial + (long long)b * 4);
+      tile_partials<1, 0, AXNT>(v, pt);
     } else if (MODE == 2) {
       double v[2] = {v0, v1};
-      tile_partials<2, 0, AXNT>(v, partial + (long long)b * 4);
+      tile_partials<2, 0, AXNT>(v, pt);
     } else if (MODE == 3) {
       double v[4] = {v0, v1, v2, v3};
-      tile_partials<4, 1, AXNT>(v, partial + (long long)b * 4);
+      tile_partials<4, 1, AXNT>(v, pt);
     } else {
       __syncthreads();  // the ring and the weights are rewritten by the next tile
     }
@@ -1185,12 +1187,13 @@ __global__ void __launch_bounds__(AXNT, 3) k_kr_ax32(const KrylovJob<float>* __r
     else
       walk(std::false_type{});
     cp_wait<0>();
+    double* const pt = partial + (long long)(J.us + t0) * 4;
     if (MODE == 1) {
       double v[1] = {v0};
-      tile_partials<1, 0, AXNT>(v, partial + (long long)b * 4);
+      tile_partials<1, 0, AXNT>(v, pt);
     } else if (MODE == 2) {
       double v[2] = {v0, v1};
-      tile_partials<2, 0, AXNT>(v, partial + (long long)b * 4);
+      tile_partials<2, 0, AXNT>(v, pt);
     } else {
       __syncthreads();  // the ring and the weights are rewritten by the next tile
     }
@@ -1362,6 +1365,32 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
     double v0 = 0.0, v1 = 0.0;
     float* o = out + (long long)(k0 + 3) * nxy;
     const int nsteps = (nk + AXV_B - 1) / AXV_B;
+    // block-wide sums of the planes since the last ones, after every ks planes and at the end of the tile
+    const int unit_steps = (J.ks + AXV_B - 1) / AXV_B;
+    int left = unit_steps;
+    double* pt = partial + 4 * (J.us + (long long)(t0 % (ntx * nty)) + (long long)ntx * nty * ((k0 - 1) / J.ks));
+    auto sums = [&]() {
+      v0 = e_wsum(v0);
+      v1 = e_wsum(v1);
+      if ((tid & 31) == 0) {
+        red[0][tid >> 5] = v0;
+        red[1][tid >> 5] = v1;
+      }
+      __syncthreads();  // (before `red` is written again every warp has passed a step's barrier)
+      if (tid == 0) {
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int w = 0; w < AXV_NT / 32; ++w) {
+          s0 += red[0][w];
+          s1 += red[1][w];
+        }
+        pt[0] = s0;
+        if (MODE == 2) pt[1] = s1;
+      }
+      pt += 4LL * ntx * nty;
+      v0 = v1 = 0.0;
+      left = unit_steps;
+    };
     for (int s = 0; s < nsteps; ++s) {
       const int tb = s * AXV_B;
       cp_wait<AXV_G - 2>();  // this thread's copies of the step's group have landed
@@ -1468,27 +1497,9 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
 #pragma unroll
         for (int u = 0; u < AXV_B; ++u) win[r][AXV_ZW - AXV_B + u] = nw[r][u];
       }
+      if (MODE != 0 && (--left == 0 || s + 1 == nsteps)) sums();
     }
     cp_wait<0>();
-    if (MODE != 0) {
-      v0 = e_wsum(v0);
-      v1 = e_wsum(v1);
-      if ((tid & 31) == 0) {
-        red[0][tid >> 5] = v0;
-        red[1][tid >> 5] = v1;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-        for (int w = 0; w < AXV_NT / 32; ++w) {
-          s0 += red[0][w];
-          s1 += red[1][w];
-        }
-        partial[(long long)b * 4] = s0;
-        if (MODE == 2) partial[(long long)b * 4 + 1] = s1;
-      }
-    }
     // the ring and red are rewritten by the next tile only after its first barrier
   }
 }
@@ -1638,6 +1649,42 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
     double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
     const long long obase = (long long)(k0 + 3) * nxy;
     const int nsteps = (nk + AXD_B - 1) / AXD_B;
+    // block-wide sums of the planes since the last ones, after every ks planes and at the end of the tile
+    const int unit_steps = (J.ks + AXD_B - 1) / AXD_B;
+    int left = unit_steps;
+    double* pt = partial + 4 * (J.us + (long long)(t0 % (ntx * nty)) + (long long)ntx * nty * ((k0 - 1) / J.ks));
+    auto sums = [&]() {
+      v0 = MODE == 3 ? e_wmax(v0) : e_wsum(v0);
+      v1 = e_wsum(v1);
+      v2 = e_wsum(v2);
+      v3 = e_wsum(v3);
+      if ((tid & 31) == 0) {
+        red[0][tid >> 5] = v0;
+        red[1][tid >> 5] = v1;
+        red[2][tid >> 5] = v2;
+        red[3][tid >> 5] = v3;
+      }
+      __syncthreads();  // (before `red` is written again every warp has passed a step's barrier)
+      if (tid == 0) {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+        for (int w = 0; w < AXD_NT / 32; ++w) {
+          s0 = MODE == 3 ? fmax(s0, red[0][w]) : s0 + red[0][w];
+          s1 += red[1][w];
+          s2 += red[2][w];
+          s3 += red[3][w];
+        }
+        pt[0] = s0;
+        if (MODE >= 2) pt[1] = s1;
+        if (MODE == 3) {
+          pt[2] = s2;
+          pt[3] = s3;
+        }
+      }
+      pt += 4LL * ntx * nty;
+      v0 = v1 = v2 = v3 = 0.0;
+      left = unit_steps;
+    };
     for (int s = 0; s < nsteps; ++s) {
       const int tb = s * AXD_B;
       cp_wait<AXD_G - 2>();
@@ -1743,39 +1790,10 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
 #pragma unroll
         for (int u = 0; u < AXD_B; ++u) win[r][AXD_ZW - AXD_B + u] = nw[r][u];
       }
+      if (MODE != 0 && (--left == 0 || s + 1 == nsteps)) sums();
     }
     cp_wait<0>();
-    if (MODE != 0) {
-      v0 = MODE == 3 ? e_wmax(v0) : e_wsum(v0);
-      v1 = e_wsum(v1);
-      v2 = e_wsum(v2);
-      v3 = e_wsum(v3);
-      if ((tid & 31) == 0) {
-        red[0][tid >> 5] = v0;
-        red[1][tid >> 5] = v1;
-        red[2][tid >> 5] = v2;
-        red[3][tid >> 5] = v3;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-#pragma unroll
-        for (int w = 0; w < AXD_NT / 32; ++w) {
-          s0 = MODE == 3 ? fmax(s0, red[0][w]) : s0 + red[0][w];
-          s1 += red[1][w];
-          s2 += red[2][w];
-          s3 += red[3][w];
-        }
-        partial[(long long)b * 4] = s0;
-        if (MODE >= 2) partial[(long long)b * 4 + 1] = s1;
-        if (MODE == 3) {
-          partial[(long long)b * 4 + 2] = s2;
-          partial[(long long)b * 4 + 3] = s3;
-        }
-      }
-    } else {
-      __syncthreads();  // the z weights are rewritten by the next tile
-    }
+    if (MODE == 0) __syncthreads();  // the z weights are rewritten by the next tile (after the sums' barrier)
   }
 }
 
@@ -3334,48 +3352,10 @@ void launch_ax(int grid, const KrylovJob<T>* J, const int* ts, int n, int ntiles
 // the fused smoothing kernel runs one block per tile (one block per SM at a time)
 inline int grid_multi(int ntiles) { return ntiles; }
 
-// Tile depth of one grid in a Krylov list, at most kc (the solver parameter tile_kc or its
-// default).  A tile is a serial chain of planes after a prologue of about 8 planes' time (the
-// job's scalars; in the operator the z window and the first staged group), so the depth minimises
-// waves of tiles over the kernel's resident blocks x (depth + 8), among kc, the multiples of 8
-// below it (the vector updates walk blocks of 8 planes), 4 and, in the two-row
-// operator, 2 (its step).  Grids of many waves keep kc; on
-// 32 x 32 x 64 the 4 tiles of 64 planes become 64 of 4 (FP32 operator 26.6 -> 6.2 us, x update
-// 14.4 -> 4.3 us).  It depends on the grid alone, so a case's partial sums do not depend on its
-// batch.
 constexpr int kVecBlocksPerSm = 4;  // resident blocks of the vector updates
-template <typename TilesXY>
-inline int depth_for(TilesXY&& tiles, int n3, int kc, int slots, int least = 4) {
-  int best = kc;
-  long long cost = -1;
-  auto consider = [&](int d) {
-    const long long c = (tiles(d) + slots - 1) / slots * (std::min(d, n3) + 8);
-    if (cost < 0 || c < cost) {
-      cost = c;
-      best = d;
-    }
-  };
-  consider(kc);
-  for (int d = (kc - 1) / 8 * 8; d >= 8; d -= 8) consider(d);
-  for (int d = 4; d >= least; d /= 2)
-    if (kc > d) consider(d);
-  return best;
-}
-inline int krylov_depth(const Geom& g, int kc, int slots, int rows = ETY) {
-  return depth_for([&](int d) { return (long long)tiles_of(g, d, 1, rows); }, g.n3, kc, slots, rows > ETY ? 2 : 4);
-}
-// the depth of a list without partial sums: the same rule over all its grids together (the small
-// grids of a batch need no shallow tiles of their own to fill the GPU)
-inline int list_depth(const std::vector<Geom>& gs, int kc, int slots) {
-  int n3 = 0;
-  for (const Geom& g : gs) n3 = std::max(n3, g.n3);
-  return depth_for(
-      [&](int d) {
-        long long t = 0;
-        for (const Geom& g : gs) t += tiles_of(g, d);
-        return t;
-      },
-      n3, kc, slots);
+// a grid's tiles of 32 x `rows` columns, for the depth rules of shape.h
+inline TileGrid tile_grid(const Geom& g, int rows = ETY, bool stack = false) {
+  return TileGrid{ETX, rows, g.n1, g.n2, g.n3, stack, 0, 0};
 }
 
 }  // namespace
@@ -3400,24 +3380,29 @@ void collapse_divgrad(int M, const double* cG, const double* cD, std::vector<dou
 }
 
 template <typename J>
-int ListArena::add(const std::vector<J>& jobs, const std::vector<int>& tiles) {
+int ListArena::add(const std::vector<J>& jobs, const std::vector<int>& tiles, const std::vector<int>* units) {
   auto align = [this](size_t a) {
     while (host.size() % a) host.push_back(0);
   };
   DevList L;
   L.njobs = (int)jobs.size();
-  align(16);
-  ts_off.push_back(host.size());
-  int acc = 0;
-  std::vector<int> ts(jobs.size() + 1);
-  for (size_t q = 0; q < jobs.size(); ++q) {
-    ts[q] = acc;
-    acc += tiles[q];
-  }
-  ts[jobs.size()] = acc;
-  L.ntiles = acc;
-  const unsigned char* tb = reinterpret_cast<const unsigned char*>(ts.data());
-  host.insert(host.end(), tb, tb + ts.size() * sizeof(int));
+  auto prefix = [&](const std::vector<int>& n) {  // its place in the arena
+    align(16);
+    const size_t at = host.size();
+    int acc = 0;
+    std::vector<int> ps(jobs.size() + 1);
+    for (size_t q = 0; q < jobs.size(); ++q) {
+      ps[q] = acc;
+      acc += n[q];
+    }
+    ps[jobs.size()] = acc;
+    const unsigned char* b = reinterpret_cast<const unsigned char*>(ps.data());
+    host.insert(host.end(), b, b + ps.size() * sizeof(int));
+    return at;
+  };
+  for (int n : tiles) L.ntiles += n;
+  ts_off.push_back(prefix(tiles));
+  us_off.push_back(units ? prefix(*units) : ts_off.back());
   align(16);
   job_off.push_back(host.size());
   const unsigned char* jb = reinterpret_cast<const unsigned char*>(jobs.data());
@@ -3439,6 +3424,7 @@ int ListArena::upload(cudaStream_t s) {
   if (e != cudaSuccess) return impact_set_error(e, "job list upload", __FILE__, __LINE__);
   for (size_t q = 0; q < lists.size(); ++q) {
     lists[q].ts = reinterpret_cast<const int*>(dev + ts_off[q]);
+    lists[q].us = reinterpret_cast<const int*>(dev + us_off[q]);
     lists[q].jobs = dev + job_off[q];
   }
   return 0;
@@ -3450,6 +3436,7 @@ void ListArena::release() {
   host.clear();
   lists.clear();
   ts_off.clear();
+  us_off.clear();
   job_off.clear();
 }
 
@@ -3573,28 +3560,42 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     constexpr bool f32 = std::is_same<T, float>::value;
     const bool adapt = use_mg;
     kr_rows_ = f32 && use_mg ? 2 : 1;
-    auto depths = [&](auto slots, auto rows) {
-      long long tiles = 0;
-      for (int c = 0; c < n; ++c) {
-        kj[c].kc = adapt ? krylov_depth(kj[c].g, kc, slots(kj[c]), rows(kj[c])) : kc;
-        kt[c] = tiles_of(kj[c].g, kj[c].kc, 1, rows(kj[c]));
-        tiles += kt[c];
-      }
-      return tiles;
-    };
-    const long long ta = depths([&](const KrylovJob<T>& J) {
+    auto slots_of = [&](const KrylovJob<T>& J) {
       return std::min(J.vec ? (f32 ? g_axv_grid[kr_rows_ - 1] : g_axd_grid) : (f32 ? g_axs32_grid : g_axs64_grid),
-                      device_sms() * kVecBlocksPerSm );
-    }, [&](const KrylovJob<T>& J) { return f32 && J.vec ? kr_rows_ * ETY : ETY; });
-    kr_list_ = arena_.add(kj, kt);
-    const long long tv = depths([&](const KrylovJob<T>&) { return device_sms() * kVecBlocksPerSm; },
-                                [](const KrylovJob<T>&) { return ETY; });
+                      device_sms() * kVecBlocksPerSm);
+    };
+    auto rows_of = [&](const KrylovJob<T>& J) { return f32 && J.vec ? kr_rows_ * ETY : ETY; };
+    std::vector<TileGrid> tg(n);
+    int slots = 1;
+    for (int c = 0; c < n; ++c) {
+      tg[c] = tile_grid(kj[c].g, rows_of(kj[c]), kj[c].vec != 0);
+      tg[c].kc = tg[c].ks = adapt ? grid_depth(tg[c], kc, slots_of(kj[c])) : kc;
+      slots = std::max(slots, slots_of(kj[c]));
+    }
+    if (adapt) stack_units(tg, kc, slots, f32 ? Axv<2>::B : Axd<1>::B);  // (adapt: two rows in FP32)
+    std::vector<int> ku(n);
+    long long ta = 0, tv = 0;
+    for (int c = 0; c < n; ++c) {
+      kj[c].kc = tg[c].kc;
+      kj[c].ks = tg[c].ks;
+      kt[c] = tiles_of(kj[c].g, kj[c].kc, 1, rows_of(kj[c]));
+      ku[c] = tiles_of(kj[c].g, kj[c].ks, 1, rows_of(kj[c]));
+      kj[c].us = (int)ta;
+      ta += ku[c];
+    }
+    kr_list_ = arena_.add(kj, kt, &ku);
+    for (int c = 0; c < n; ++c) {
+      kj[c].kc = kj[c].ks = adapt ? grid_depth(tile_grid(kj[c].g), kc, device_sms() * kVecBlocksPerSm) : kc;
+      kt[c] = tiles_of(kj[c].g, kj[c].kc);
+      kj[c].us = (int)tv;
+      tv += kt[c];
+    }
     kv_list_ = arena_.add(kj, kt);
-    std::vector<Geom> gs;
-    for (const auto& J : kj) gs.push_back(J.g);
+    std::vector<TileGrid> gs;
+    for (const auto& J : kj) gs.push_back(tile_grid(J.g));
     const int dl = list_depth(gs, kc, device_sms() * kVecBlocksPerSm);
     for (int c = 0; c < n; ++c) {
-      kj[c].kc = dl;
+      kj[c].kc = kj[c].ks = dl;
       kt[c] = tiles_of(kj[c].g, dl);
     }
     ku_list_ = arena_.add(kj, kt);
@@ -4050,11 +4051,11 @@ void Engine<T>::enqueue_iteration() {
   IMPACT_PROF(prof::K_P_UPDATE, 4 * fb, s, (k_kr_p<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(0);
   IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_, kr_rows_)));
-  k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 1, 0, EFIN_ALPHA, scal_, nullptr);
+  k_efin<<<n, 256, 0, s>>>(K.us, partial_, 1, 0, EFIN_ALPHA, scal_, nullptr);
   IMPACT_PROF(prof::K_R_UPDATE, 3 * fb, s, (k_kr_r<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(1);
   IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_, kr_rows_)));
-  k_efin<<<n, 256, 0, s>>>(K.ts, partial_, 2, 0, EFIN_OMEGA, scal_, nullptr);
+  k_efin<<<n, 256, 0, s>>>(K.us, partial_, 2, 0, EFIN_OMEGA, scal_, nullptr);
   IMPACT_PROF(prof::K_X_UPDATE, 8 * fb, s, (k_kr_x<T><<<gw, kBlock, 0, s>>>(JW, W.ts, n, W.ntiles, partial_)));
   k_efin<<<n, 256, 0, s>>>(W.ts, partial_, 3, 1, EFIN_NORMS, scal_, nullptr);
   prof::count(3);
@@ -4357,10 +4358,10 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
   cudaMemsetAsync(oscal_, 0, (size_t)n * sizeof(SolverScalars), s);
   std::vector<KrylovJob<double>> aj(n);
   std::vector<MixJob> mj(n);
-  std::vector<int> t(n), tm(n);
-  long long tiles = 0;
-  std::vector<Geom> gs;
-  for (const Case& c : cs) gs.push_back(c.g);
+  std::vector<int> t(n), tu(n), tm(n);
+  long long units = 0;
+  std::vector<TileGrid> gs, tg(n);
+  for (const Case& c : cs) gs.push_back(tile_grid(c.g));
   const int dl = list_depth(gs, kc, device_sms() * kVecBlocksPerSm);
   for (int c = 0; c < n; ++c) {
     const Case& C = cs[c];
@@ -4389,15 +4390,22 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
     M.e32 = C.e32;
     M.q = q_ + 4 * c;
     M.isc = inner_.scal_dev() + c;
-    const int rows = A.vec ? Axd<AXD_NR3>::Y : ETY;
-    A.kc = krylov_depth(C.g, kc, A.vec ? g_axd3_grid : g_axs64_grid, rows);
-    t[c] = tiles_of(C.g, A.kc, 1, rows);
-    tiles += t[c];
+    tg[c] = tile_grid(C.g, A.vec ? Axd<AXD_NR3>::Y : ETY, A.vec != 0);
+    tg[c].kc = tg[c].ks = grid_depth(tg[c], kc, A.vec ? g_axd3_grid : g_axs64_grid);
+    A.ks = tg[c].ks;
+    A.us = (int)units;
+    tu[c] = tiles_of(C.g, A.ks, 1, tg[c].rows);
+    units += tu[c];
     M.kc = dl;
     M.vecu = C.g.n1 % 4 == 0 && (reinterpret_cast<uintptr_t>(C.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(C.e32) & 15) == 0;
     tm[c] = tiles_of(C.g, dl);
   }
-  e = cudaMalloc((void**)&partial_, (size_t)(tiles * 4 + 64) * sizeof(double));
+  stack_units(tg, kc, g_axd3_grid, Axd<AXD_NR3>::B);
+  for (int c = 0; c < n; ++c) {
+    aj[c].kc = tg[c].kc;
+    t[c] = tiles_of(aj[c].g, aj[c].kc, 1, tg[c].rows);
+  }
+  e = cudaMalloc((void**)&partial_, (size_t)(units * 4 + 64) * sizeof(double));
   if (e != cudaSuccess) {
     release();
     return impact_set_error(e, "mixed engine allocation", __FILE__, __LINE__);
@@ -4407,7 +4415,7 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
     for (const auto& A : aj) nv += A.vec;
     ax_vec_ = nv == 0 ? 0 : (nv == n ? 1 : 2);
   }
-  ax_list_ = arena_.add(aj, t);
+  ax_list_ = arena_.add(aj, t, &tu);
   mix_list_ = arena_.add(mj, tm);
   rc = arena_.upload(s);
   if (rc) {
@@ -4471,7 +4479,7 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
     // r = b - A x in FP64 (the reference operator), stored as the FP32 right-hand side of the
     // inner solve, with its norms
     IMPACT_PROF(prof::K_MX_RESID, 20.0 * cells, s_, (launch_ax<double, 3>(grid, AJ, AL.ts, n, AL.ntiles, partial_, s_, ax_vec_)));
-    k_efin<<<n, 256, 0, s_>>>(AL.ts, partial_, 3, 1, EFIN_RAW, nullptr, q_);
+    k_efin<<<n, 256, 0, s_>>>(AL.us, partial_, 3, 1, EFIN_RAW, nullptr, q_);
     prof::count(1);
     cudaError_t e = cudaMemcpyAsync(q_host_, q_, (size_t)n * 4 * sizeof(double), cudaMemcpyDeviceToHost, s_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
@@ -4525,7 +4533,7 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
     }
     if (!any) break;
     // e from 0, not written before the first x update; rr and the norms from the residual kernel
-    rc = inner_.solve(init, 2, ir, AL.ts, partial_);
+    rc = inner_.solve(init, 2, ir, AL.us, partial_);
     if (rc) return rc;
     for (int c = 0; c < n; ++c) {
       if (init[c].done) continue;

@@ -71,6 +71,9 @@ template <typename T>
 struct KrylovJob {
   Geom g;
   int kc;
+  // the operator's partial sums: one per column of tiles and `ks` planes (kc, or a divisor of it: the
+  // FP64 vector kernel's tiles may hold several), from row `us` of the list's partials on
+  int ks, us;
   const T* W[3];  // collapsed product_div_grad weights, row (i-1) holds offsets -5..5
   int zuni;       // 1: every z row of W[2] is the same (uniform z spacing)
   int xuni;       // 1: every x row of W[0] is the same (uniform x spacing)
@@ -102,6 +105,7 @@ struct MixJob {
 struct DevList {
   int njobs = 0, ntiles = 0;
   const int* ts = nullptr;    // tile prefix sums (njobs + 1)
+  const int* us = nullptr;    // prefix sums of the partials that its kernels write (ts: one per tile)
   const void* jobs = nullptr;
 };
 
@@ -152,10 +156,11 @@ enum { PH_INIT = 0, PH_SWEEP, PH_COPY, PH_RESID, PH_RESTRICT, PH_PROLONG, PH_PRE
 struct ListArena {
   std::vector<unsigned char> host;
   std::vector<DevList> lists;
-  std::vector<size_t> ts_off, job_off;
+  std::vector<size_t> ts_off, us_off, job_off;
   unsigned char* dev = nullptr;
+  // units: partials per job, where a tile writes several (null: one per tile)
   template <typename J>
-  int add(const std::vector<J>& jobs, const std::vector<int>& tiles);
+  int add(const std::vector<J>& jobs, const std::vector<int>& tiles, const std::vector<int>* units = nullptr);
   int upload(cudaStream_t s);
   void release();
 };

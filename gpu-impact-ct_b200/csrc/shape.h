@@ -1,7 +1,8 @@
-// shape.h -- launch shapes of the streaming passes (march.cu, stencil3.cu) as functions of the grid
-// and of the device's SM count (host code, no CUDA: tests/test_launch_shapes.py runs it).
+// shape.h -- launch shapes of the streaming passes (march.cu, stencil3.cu) and of the Krylov kernels
+// (engine.cu) as functions of the grids and of the device's SM count (host code, no CUDA: tests/test_launch_shapes.py runs it).
 #pragma once
 #include <algorithm>
+#include <vector>
 
 namespace impact {
 
@@ -46,6 +47,96 @@ inline int tri_depth(double gxy, int n3, double sms, bool vec) {
     }
   }
   return depth;
+}
+
+// A grid cut into tiles of tx x rows columns and kc planes for a Krylov kernel.  ks: the planes of one unit of
+// summation (one partial sum each); stack: a tile may hold several units.
+struct TileGrid {
+  int tx, rows, n1, n2, n3;
+  bool stack;
+  int ks, kc;
+};
+inline long long tiles_at(const TileGrid& g, int kc) {
+  return (long long)((g.n1 + g.tx - 1) / g.tx) * ((g.n2 + g.rows - 1) / g.rows) * ((g.n3 + kc - 1) / kc);
+}
+
+// Tile depth, at most kc (the solver parameter tile_kc or its default), for `tiles(depth)` tiles over
+// grids of up to n3 planes.  A tile is a serial chain of planes after a prologue of about 8 planes' time
+// (the job's scalars; in the operator the z window and the first staged group), so the depth minimises
+// waves of tiles over the kernel's `slots` resident blocks x (depth + 8), among kc, the multiples of 8
+// below it (the vector updates walk blocks of 8 planes) and 4, or as far down as `least`.
+template <typename Tiles>
+inline int depth_for(Tiles&& tiles, int n3, int kc, int slots, int least = 4) {
+  int best = kc;
+  long long cost = -1;
+  auto consider = [&](int d) {
+    const long long c = (tiles(d) + slots - 1) / slots * (std::min(d, n3) + 8);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = d;
+    }
+  };
+  consider(kc);
+  for (int d = (kc - 1) / 8 * 8; d >= 8; d -= 8) consider(d);
+  for (int d = 4; d >= least; d /= 2)
+    if (kc > d) consider(d);
+  return best;
+}
+
+// The depth of one grid, from the grid alone: the unit of its partial sums, so that a case's sums do not
+// depend on its batch.  Grids of many waves keep kc; on 32 x 32 x 64 the 4 tiles of 64 planes become 64 of 4
+// (FP32 operator 26.6 -> 6.2 us, x update 14.4 -> 4.3 us); kernels of two rows per thread (tiles of more than
+// 8 rows) step by 2 planes and may take as few.
+inline int grid_depth(const TileGrid& g, int kc, int slots) {
+  return depth_for([&](int d) { return tiles_at(g, d); }, g.n3, kc, slots, g.rows > 8 ? 2 : 4);
+}
+
+// the depth of a list without partial sums: the same rule over all its grids together (the small
+// grids of a batch need no shallow tiles of their own to fill the GPU)
+inline int list_depth(const std::vector<TileGrid>& gs, int kc, int slots) {
+  int n3 = 0;
+  for (const TileGrid& g : gs) n3 = std::max(n3, g.n3);
+  auto tiles = [&](int d) {
+    long long t = 0;
+    for (const TileGrid& g : gs) t += tiles_at(g, d);
+    return t;
+  };
+  return depth_for(tiles, n3, kc, slots);
+}
+
+// Tile depths of an operator list of several grids whose units ks are chosen.  A grid whose tiles of ks planes
+// would fill the GPU alone shares it here, where each tile's prologue is paid for nothing: a tile holds
+// as many whole units as the list's common depth allows, and its kernel sums each unit by itself.  The
+// depth minimises the list's planes and prologues per resident block + the longest tile.  step: the
+// planes per step of the kernel, of which a unit must be a multiple.  48 cases of 32 to 152 cells a
+// side: FP64 operator 32.0 ms a step with tiles of one unit, 30.0 with several (29.2 with 64 planes in every tile
+// and unit), FP32 operator 14.4 and 13.5.
+inline void stack_units(std::vector<TileGrid>& gs, int kc, int slots, int step) {
+  auto depth = [&](const TileGrid& g, int d) { return g.stack && g.ks % step == 0 ? g.ks * std::max(1, d / g.ks) : g.ks; };
+  int best = 1;
+  double least = -1.0;
+  auto consider = [&](int d) {
+    double work = 0.0;
+    int longest = 0;
+    for (const TileGrid& g : gs) {
+      const int e = depth(g, d);
+      const double columns = (double)tiles_at(g, g.n3);
+      work += columns * (g.n3 + 8.0 * ((g.n3 + e - 1) / e));
+      longest = std::max(longest, std::min(e, g.n3) + 8);
+    }
+    const double cost = work / slots + longest;
+    if (least < 0.0 || cost < least) {
+      least = cost;
+      best = d;
+    }
+  };
+  if (gs.size() > 1) {
+    consider(kc);
+    for (int d = (kc - 1) / 8 * 8; d >= 8; d -= 8) consider(d);
+    for (int d : {4, 1})
+      if (kc > d) consider(d);
+  }
+  for (TileGrid& g : gs) g.kc = depth(g, best);
 }
 
 }  // namespace impact

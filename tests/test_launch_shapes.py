@@ -22,6 +22,7 @@ def shape(tmp_path_factory):
     lib = C.CDLL(str(out))
     lib.host_march_seg.restype, lib.host_march_seg.argtypes = C.c_int, [C.c_longlong] + [C.c_int] * 4
     lib.host_tri_depth.restype, lib.host_tri_depth.argtypes = C.c_int, [C.c_double, C.c_int, C.c_double, C.c_int]
+    lib.host_stack.restype, lib.host_stack.argtypes = None, [C.POINTER(C.c_int)] + [C.c_int] * 5 + [C.POINTER(C.c_int)] * 2
     return lib
 
 
@@ -56,6 +57,48 @@ def test_a_three_axis_pass_on_a_small_grid_takes_shallow_blocks(shape, n, vec):
 @pytest.mark.parametrize("share", [1.0, 0.25, 0.001])
 def test_depths_of_a_batch_grow_as_its_share_shrinks(shape, share):
     assert shape.host_tri_depth(8, 64, SMS * share, 1) >= shape.host_tri_depth(8, 64, SMS, 1)
+
+
+def _stacked(shape, sizes, rows, kc, slots, step):
+    arr = C.c_int * len(sizes)
+    ks, depth = arr(), arr()
+    shape.host_stack(arr(*sizes), len(sizes), rows, kc, slots, step, ks, depth)
+    return list(ks), list(depth)
+
+
+def _planes(sizes, depths, rows):
+    """Planes marched by a list's tiles, with the 8 planes' time of each tile's prologue."""
+    return sum(-(-n // 32) * -(-n // rows) * sum(min(d, 2 * n - k) + 8 for k in range(0, 2 * n, d)) for n, d in zip(sizes, depths))
+
+
+UNEVEN = [32, 40, 40, 48, 56, 64, 64, 72, 80, 88, 96, 96, 104, 112, 120, 136, 144, 152]
+KERNELS = [(8, 296, 4), (16, 296, 2), (16, 592, 2)]  # FP64 operator, FP64 outer residual, FP32 operator
+
+
+@pytest.mark.parametrize("rows,slots,step", KERNELS, ids=["fp64", "residual", "fp32"])
+def test_a_batch_does_not_pay_for_the_shallow_tiles_of_its_cases_alone(shape, rows, slots, step):
+    sizes = 3 * UNEVEN
+    ks, depth = _stacked(shape, sizes, rows, 64, slots, step)
+    assert _planes(sizes, depth, rows) <= 1.03 * _planes(sizes, [64] * len(sizes), rows) < _planes(sizes, ks, rows)
+    for n, u, d in zip(sizes, ks, depth):
+        assert d % u == 0 and d <= 64
+        assert u == _stacked(shape, [n], rows, 64, slots, step)[0][0]  # the unit is the grid's own
+
+
+@pytest.mark.parametrize("rows,slots,step", KERNELS, ids=["fp64", "residual", "fp32"])
+@pytest.mark.parametrize("kc", [1, 5, 8, 12, 30, 64])
+@pytest.mark.parametrize("n", [8, 33, 64, 160])
+def test_a_case_alone_keeps_one_unit_per_tile(shape, n, kc, rows, slots, step):
+    ks, depth = _stacked(shape, [n], rows, kc, slots, step)
+    assert depth == ks and 1 <= ks[0] <= kc
+
+
+@pytest.mark.parametrize("kc", [1, 5, 8, 12, 30, 64])
+def test_tiles_of_several_units_hold_whole_steps(shape, kc):
+    for rows, slots, step in KERNELS:
+        ks, depth = _stacked(shape, UNEVEN, rows, kc, slots, step)
+        for u, d in zip(ks, depth):
+            assert d == u or (u % step == 0 and d % u == 0 and d <= kc)
 
 
 @pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc")

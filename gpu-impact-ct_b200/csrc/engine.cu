@@ -3249,6 +3249,24 @@ __global__ void __launch_bounds__(ENT) k_mx_apply(const MixJob* __restrict__ job
   }
 }
 
+// launch of k_lv_tail: `tails` clusters of `blocks` blocks
+struct TailLaunch {
+  cudaLaunchAttribute at[1] = {};
+  cudaLaunchConfig_t cfg = {};
+  TailLaunch(int blocks, int tails, cudaStream_t s) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(tails * blocks);
+    cfg.blockDim = dim3(TNT);
+    cfg.dynamicSmemBytes = TAIL_BYTES + TAIL_TAB_BYTES;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = blocks > 1;
+  }
+  TailLaunch(const TailLaunch&) = delete;
+};
+
 // grids of the vector operator kernels: the blocks resident at once on the device (a grid-stride
 // kernel given more would leave its last blocks to run after the others, one tile step behind)
 int g_axv_grid[2] = {0, 0}, g_axd_grid = 0, g_axd3_grid = 0;
@@ -3809,11 +3827,21 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       ++ntails;
       want |= gl.n1 * gl.n2 * gl.n3 >= TAIL_SPLIT;
     }
-    for (int cb = TAIL_CLUSTER; want && cb > 1 && tail_blocks_ == 1; cb /= 2) {
-      bool ok = ntails * cb <= device_sms();
-      for (int c = 0; ok && c < n; ++c) ok = lt[c] < 0 || tail_job(c, lt[c], nlev[c], 0, cb).nl > 0;
-      if (ok) tail_blocks_ = cb;
-    }
+    auto fits = [&](int cb) {
+      for (int c = 0; c < n; ++c)
+        if (lt[c] >= 0 && tail_job(c, lt[c], nlev[c], 0, cb).nl == 0) return false;
+      return true;
+    };
+    auto held = [&](int cb) {
+      int clusters = 0;
+      const TailLaunch L(cb, 1, s);
+      if (cudaOccupancyMaxActiveClusters(&clusters, k_lv_tail<T, true>, &L.cfg) != cudaSuccess) {
+        cudaGetLastError();  // no such cluster here: not an error of the solve
+        return 0;
+      }
+      return clusters;
+    };
+    if (want) tail_blocks_ = tail_cluster(ntails, TAIL_CLUSTER, fits, held);
   }
   auto in_lists = [&](int c, int g) { return lt[c] < 0 || g < lt[c]; };
   if (use_mg) {
@@ -3963,20 +3991,10 @@ void launch_multi_post(int sweeps, bool fast, const LevelJob<T>* J, const DevLis
 }
 
 template <typename T>
-void launch_tail(int blocks, const DevList& L, T om, int n_down, int n_up, int n_bottom, cudaStream_t s) {
-  cudaLaunchAttribute at[1] = {};
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = blocks;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(L.ntiles * blocks);
-  cfg.blockDim = dim3(TNT);
-  cfg.dynamicSmemBytes = TAIL_BYTES + TAIL_TAB_BYTES;
-  cfg.stream = s;
-  cfg.attrs = at;
-  cfg.numAttrs = blocks > 1;
-  cudaLaunchKernelEx(&cfg, blocks > 1 ? k_lv_tail<T, true> : k_lv_tail<T, false>, static_cast<const TailJob<T>*>(L.jobs),
-                     L.ts, L.njobs, L.ntiles, om, n_down, n_up, n_bottom);
+cudaError_t launch_tail(int blocks, const DevList& L, T om, int n_down, int n_up, int n_bottom, cudaStream_t s) {
+  const TailLaunch l(blocks, L.ntiles, s);
+  return cudaLaunchKernelEx(&l.cfg, blocks > 1 ? k_lv_tail<T, true> : k_lv_tail<T, false>,
+                            static_cast<const TailJob<T>*>(L.jobs), L.ts, L.njobs, L.ntiles, om, n_down, n_up, n_bottom);
 }
 
 template <typename T>
@@ -4023,8 +4041,10 @@ void Engine<T>::enqueue_phase(const Phase& ph) {
       IMPACT_PROF(prof::K_MG_SWEEP, 2 * sz * c, s, launch_multi_jor<T>(p_.n_sweeps, fast_[ph.list] != 0, J, L, om, s));
       break;
     case PH_TAIL:  // one block or cluster per case; bytes: read the first level's right-hand side, write its iterate
-      IMPACT_PROF(prof::K_MG_TAIL, 2 * sz * c, s,
-                  launch_tail<T>(tail_blocks_, L, om, p_.mg_down, p_.mg_up, p_.mg_bottom, s));
+      IMPACT_PROF(prof::K_MG_TAIL, 2 * sz * c, s, {
+        const cudaError_t e = launch_tail<T>(tail_blocks_, L, om, p_.mg_down, p_.mg_up, p_.mg_bottom, s);
+        if (e != cudaSuccess) tail_err_ = e;
+      });
       break;
     default:
       break;
@@ -4074,6 +4094,14 @@ int Engine<T>::poll(bool& all_done) {
     if (!(h.done || (h.status != 0 && h.status != 4))) all_done = false;
   }
   return 0;
+}
+
+template <typename T>
+int Engine<T>::tail_failed() {
+  const cudaError_t e = tail_err_;
+  tail_err_ = cudaSuccess;
+  cudaGetLastError();  // reported here
+  return impact_set_error(e, "launch of the coarse tail", __FILE__, __LINE__);
 }
 
 template <typename T>
@@ -4128,6 +4156,12 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
       if (profiling) gpairs_ = prof::capture_end();
       e = cudaStreamEndCapture(s_, &gr);
     }
+    if (e == cudaSuccess && tail_err_ != cudaSuccess) {  // without its tail the graph would use stale iterates
+      cudaGraphDestroy(gr);
+      prof::graph_release(gpairs_);
+      return tail_failed();
+    }
+    tail_err_ = cudaSuccess;  // (a capture that failed: the launches below tell)
     if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_, gr, 0);
     if (gr) cudaGraphDestroy(gr);
     if (e != cudaSuccess) {  // capture unavailable on this stream: launch directly from now on
@@ -4147,6 +4181,7 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
       prof::count((long long)chunk * launches_iter_);
     } else {
       for (int t = 0; t < chunk; ++t) enqueue_iteration();
+      if (tail_err_ != cudaSuccess) return tail_failed();
     }
     launched += chunk;
     bool all_done = false;
@@ -4186,6 +4221,7 @@ int Engine<T>::apply_precond() {
   cudaError_t e = cudaMemcpyAsync(scal_, scal_host_, n * sizeof(SolverScalars), cudaMemcpyHostToDevice, s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine scalars", __FILE__, __LINE__);
   enqueue_precond(0);
+  if (tail_err_ != cudaSuccess) return tail_failed();
   e = cudaStreamSynchronize(s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine precond", __FILE__, __LINE__);
   return 0;

@@ -206,6 +206,7 @@ class Engine {
   void enqueue_phase(const Phase& ph);
   void smooth(std::vector<Phase>& out, int list, int init, int sweeps);
   int poll(bool& all_done);
+  int tail_failed();  // reports tail_err_
 
   std::vector<EngineCase<T>> cs_;
   EngineParams p_{};
@@ -230,6 +231,7 @@ class Engine {
   std::vector<double> cells_, cells_f_, cells_c_;
   std::vector<char> fast_;  // per list: every job vectorised with uniform z (k_lv_fast)
   int tail_blocks_ = 1;     // blocks per coarse tail: 1, or a cluster cut into z slabs
+  cudaError_t tail_err_ = cudaSuccess;  // a refused launch of the tail
   int kr_rows_ = 1;         // rows per thread of the FP32 vector operator
   int kr_vec_ = 0;          // FP32 Krylov list: jobs in the vector kernel -- 0 none, 1 all, 2 some
 };

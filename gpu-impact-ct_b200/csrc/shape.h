@@ -139,4 +139,15 @@ inline void stack_units(std::vector<TileGrid>& gs, int kc, int slots, int step) 
   for (TileGrid& g : gs) g.kc = depth(g, best);
 }
 
+// Blocks per coarse tail of a list of `ntails`: the largest power of two up to `most` whose cut into slabs fits
+// (fits(blocks)) and of which the device can hold a cluster for every tail at once (held(blocks): clusters;
+// 15 of 8, 33 of 4 and 74 of 2 on a whole B200, whose SMs stand in groups; a part of one may hold none);
+// else one.
+template <typename Fits, typename Held>
+inline int tail_cluster(int ntails, int most, Fits&& fits, Held&& held) {
+  for (int cb = most; cb > 1; cb /= 2)
+    if (fits(cb) && held(cb) >= ntails) return cb;
+  return 1;
+}
+
 }  // namespace impact

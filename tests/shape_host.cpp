@@ -19,3 +19,8 @@ extern "C" void host_stack(const int* n, int count, int rows, int kc, int slots,
     depth[q] = g[q].kc;
   }
 }
+// held: clusters of 2, 4 and 8 blocks that the device holds; fitted: most blocks that the slabs of every case fit
+extern "C" int host_tail_cluster(int ntails, const int* held, int fitted) {
+  return impact::tail_cluster(ntails, 8, [&](int cb) { return cb <= fitted; },
+                              [&](int cb) { return held[cb == 2 ? 0 : (cb == 4 ? 1 : 2)]; });
+}

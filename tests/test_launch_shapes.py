@@ -101,6 +101,15 @@ def test_tiles_of_several_units_hold_whole_steps(shape, kc):
             assert d == u or (u % step == 0 and d % u == 0 and d <= kc)
 
 
+def test_a_coarse_tail_takes_no_cluster_that_the_device_cannot_hold(shape):
+    def f(ntails, held, fitted=8):
+        return shape.host_tail_cluster(ntails, (C.c_int * 3)(*held), fitted)
+    whole = (74, 33, 15)
+    assert [f(n, whole) for n in (1, 15, 16, 33, 34, 74, 75)] == [8, 8, 4, 4, 2, 2, 1]
+    assert [f(1, whole, fitted) for fitted in (8, 4, 2, 1)] == [8, 4, 2, 1]
+    assert [f(1, part) for part in ((4, 2, 0), (4, 0, 0), (0, 0, 0))] == [4, 2, 1]
+
+
 @pytest.mark.skipif(shutil.which("nvcc") is None, reason="needs nvcc")
 def test_one_axis_kernels_do_not_spill(tmp_path):
     r = subprocess.run(["nvcc", "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, "-I", os.path.join(ROOT, "include"),

@@ -1248,7 +1248,8 @@ struct Axv {                                             // NR rows per thread
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-template <int MODE, int AXV_NR>
+// STACK: tiles of several units of summation (batches)
+template <int MODE, int AXV_NR, bool STACK>
 __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const KrylovJob<float>* __restrict__ jobs,
                                                         const int* __restrict__ ts, int nj, int ntiles,
                                                         double* __restrict__ partial) {
@@ -1366,9 +1367,10 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
     float* o = out + (long long)(k0 + 3) * nxy;
     const int nsteps = (nk + AXV_B - 1) / AXV_B;
     // block-wide sums of the planes since the last ones, after every ks planes and at the end of the tile
-    const int unit_steps = (J.ks + AXV_B - 1) / AXV_B;
+    const int unit_steps = STACK ? (J.ks + AXV_B - 1) / AXV_B : 0;
     int left = unit_steps;
-    double* pt = partial + 4 * (J.us + (long long)(t0 % (ntx * nty)) + (long long)ntx * nty * ((k0 - 1) / J.ks));
+    double* pt = nullptr;  // the unit's row of partials; without several to a tile the tile's own
+    if (STACK) pt = partial + 4 * (J.us + t0 + (long long)ntx * nty * tc * (J.nu - 1));
     auto sums = [&]() {
       v0 = e_wsum(v0);
       v1 = e_wsum(v1);
@@ -1384,12 +1386,15 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
           s0 += red[0][w];
           s1 += red[1][w];
         }
-        pt[0] = s0;
-        if (MODE == 2) pt[1] = s1;
+        double* const o = STACK ? pt : partial + 4LL * b;
+        o[0] = s0;
+        if (MODE == 2) o[1] = s1;
       }
-      pt += 4LL * ntx * nty;
-      v0 = v1 = 0.0;
-      left = unit_steps;
+      if (STACK) {
+        pt += 4LL * ntx * nty;
+        v0 = v1 = 0.0;
+        left = unit_steps;
+      }
     };
     for (int s = 0; s < nsteps; ++s) {
       const int tb = s * AXV_B;
@@ -1497,9 +1502,10 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
 #pragma unroll
         for (int u = 0; u < AXV_B; ++u) win[r][AXV_ZW - AXV_B + u] = nw[r][u];
       }
-      if (MODE != 0 && (--left == 0 || s + 1 == nsteps)) sums();
+      if (STACK && MODE != 0 && --left == 0) sums();
     }
     cp_wait<0>();
+    if (MODE != 0 && (!STACK || left != unit_steps)) sums();
     // the ring and red are rewritten by the next tile only after its first barrier
   }
 }
@@ -1536,7 +1542,7 @@ __device__ __forceinline__ double2 ldg2d(const double* p) { return __ldg(reinter
 __device__ __forceinline__ double2 lds2d(const double* p) { return *reinterpret_cast<const double2*>(p); }
 
 constexpr int AXD_NR3 = 2;  // rows per thread of the outer residual (MODE 3)
-template <int MODE, int NR>
+template <int MODE, int NR, bool STACK>
 __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>* __restrict__ jobs,
                                                         const int* __restrict__ ts, int nj, int ntiles,
                                                         double* __restrict__ partial) {
@@ -1650,9 +1656,10 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
     const long long obase = (long long)(k0 + 3) * nxy;
     const int nsteps = (nk + AXD_B - 1) / AXD_B;
     // block-wide sums of the planes since the last ones, after every ks planes and at the end of the tile
-    const int unit_steps = (J.ks + AXD_B - 1) / AXD_B;
+    const int unit_steps = STACK ? (J.ks + AXD_B - 1) / AXD_B : 0;
     int left = unit_steps;
-    double* pt = partial + 4 * (J.us + (long long)(t0 % (ntx * nty)) + (long long)ntx * nty * ((k0 - 1) / J.ks));
+    double* pt = nullptr;  // the unit's row of partials; without several to a tile the tile's own
+    if (STACK) pt = partial + 4 * (J.us + t0 + (long long)ntx * nty * tc * (J.nu - 1));
     auto sums = [&]() {
       v0 = MODE == 3 ? e_wmax(v0) : e_wsum(v0);
       v1 = e_wsum(v1);
@@ -1674,16 +1681,19 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
           s2 += red[2][w];
           s3 += red[3][w];
         }
-        pt[0] = s0;
-        if (MODE >= 2) pt[1] = s1;
+        double* const o = STACK ? pt : partial + 4LL * b;
+        o[0] = s0;
+        if (MODE >= 2) o[1] = s1;
         if (MODE == 3) {
-          pt[2] = s2;
-          pt[3] = s3;
+          o[2] = s2;
+          o[3] = s3;
         }
       }
-      pt += 4LL * ntx * nty;
-      v0 = v1 = v2 = v3 = 0.0;
-      left = unit_steps;
+      if (STACK) {
+        pt += 4LL * ntx * nty;
+        v0 = v1 = v2 = v3 = 0.0;
+        left = unit_steps;
+      }
     };
     for (int s = 0; s < nsteps; ++s) {
       const int tb = s * AXD_B;
@@ -1790,9 +1800,10 @@ __global__ void __launch_bounds__(AXD_NT, 2) k_kr_ax64v(const KrylovJob<double>*
 #pragma unroll
         for (int u = 0; u < AXD_B; ++u) win[r][AXD_ZW - AXD_B + u] = nw[r][u];
       }
-      if (MODE != 0 && (--left == 0 || s + 1 == nsteps)) sums();
+      if (STACK && MODE != 0 && --left == 0) sums();
     }
     cp_wait<0>();
+    if (MODE != 0 && (!STACK || left != unit_steps)) sums();
     if (MODE == 0) __syncthreads();  // the z weights are rewritten by the next tile (after the sums' barrier)
   }
 }
@@ -3285,16 +3296,21 @@ void ax_attributes() {
   cudaFuncSetAttribute(k_kr_ax32<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axa_smem_bytes());
   cudaFuncSetAttribute(k_kr_ax32<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axa_smem_bytes());
   cudaFuncSetAttribute(k_kr_ax32<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)axa_smem_bytes());
-  cudaFuncSetAttribute(k_kr_ax64v<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
-  cudaFuncSetAttribute(k_kr_ax64v<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
-  cudaFuncSetAttribute(k_kr_ax64v<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
-  cudaFuncSetAttribute(k_kr_ax64v<3, AXD_NR3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<AXD_NR3>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
-  cudaFuncSetAttribute(k_kr_ax32v<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<0, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<3, AXD_NR3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<AXD_NR3>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<0, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<0, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<1, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<1, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<1, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<2, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<1>::smem());
+  cudaFuncSetAttribute(k_kr_ax64v<3, AXD_NR3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axd<AXD_NR3>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<1, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
+  cudaFuncSetAttribute(k_kr_ax32v<2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Axv<2>::smem());
   auto occ = [](auto kernel, int threads, size_t smem) {
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) != cudaSuccess || nb < 1) nb = 1;
@@ -3303,13 +3319,13 @@ void ax_attributes() {
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (nsm <= 0) nsm = 148;
-  g_axv_grid[0] = nsm * std::min({occ(k_kr_ax32v<0, 1>, AXV_NT, Axv<1>::smem()), occ(k_kr_ax32v<1, 1>, AXV_NT, Axv<1>::smem()),
-                                  occ(k_kr_ax32v<2, 1>, AXV_NT, Axv<1>::smem())});
-  g_axv_grid[1] = nsm * std::min({occ(k_kr_ax32v<0, 2>, AXV_NT, Axv<2>::smem()), occ(k_kr_ax32v<1, 2>, AXV_NT, Axv<2>::smem()),
-                                  occ(k_kr_ax32v<2, 2>, AXV_NT, Axv<2>::smem())});
-  g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0, 1>, AXD_NT, Axd<1>::smem()), occ(k_kr_ax64v<1, 1>, AXD_NT, Axd<1>::smem()),
-                               occ(k_kr_ax64v<2, 1>, AXD_NT, Axd<1>::smem())});
-  g_axd3_grid = nsm * occ(k_kr_ax64v<3, AXD_NR3>, AXD_NT, Axd<AXD_NR3>::smem());
+  g_axv_grid[0] = nsm * std::min({occ(k_kr_ax32v<0, 1, false>, AXV_NT, Axv<1>::smem()), occ(k_kr_ax32v<1, 1, false>, AXV_NT, Axv<1>::smem()),
+                                  occ(k_kr_ax32v<2, 1, false>, AXV_NT, Axv<1>::smem())});
+  g_axv_grid[1] = nsm * std::min({occ(k_kr_ax32v<0, 2, false>, AXV_NT, Axv<2>::smem()), occ(k_kr_ax32v<1, 2, false>, AXV_NT, Axv<2>::smem()),
+                                  occ(k_kr_ax32v<2, 2, false>, AXV_NT, Axv<2>::smem())});
+  g_axd_grid = nsm * std::min({occ(k_kr_ax64v<0, 1, false>, AXD_NT, Axd<1>::smem()), occ(k_kr_ax64v<1, 1, false>, AXD_NT, Axd<1>::smem()),
+                               occ(k_kr_ax64v<2, 1, false>, AXD_NT, Axd<1>::smem())});
+  g_axd3_grid = nsm * occ(k_kr_ax64v<3, AXD_NR3, false>, AXD_NT, Axd<AXD_NR3>::smem());
   g_axs32_grid = nsm * occ(k_kr_ax32<1>, AXNT, axa_smem_bytes());
   g_axs64_grid = nsm * occ(k_kr_ax<double, 1>, AXNT, ax_smem_bytes<double>());
   cudaFuncSetAttribute(k_lv_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(TAIL_BYTES + TAIL_TAB_BYTES));
@@ -3348,21 +3364,28 @@ const dim3 kAxBlock(ETX, AXTY);  // k_kr_ax: two rows per thread
 // the operator over a Krylov list: FP32 by the vector kernel for the jobs that qualify (vec:
 // 1 all, 2 some), by the 16-byte staged, stepped kernel for the others; FP64 alike
 template <typename T, int MODE>
-void launch_ax(int grid, const KrylovJob<T>* J, const int* ts, int n, int ntiles, double* partial, cudaStream_t s,
-               int vec, int rows = 1) {
+void launch_ax(int grid, const DevList& L, double* partial, cudaStream_t s, int vec, int rows = 1) {
+  const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(L.jobs);
+  const int *ts = L.ts, n = L.njobs, ntiles = L.ntiles;
+  constexpr bool UNITS = MODE != 0;  // (no sums in mode 0: one instance)
   if constexpr (std::is_same<T, float>::value && MODE <= 2) {
     const int slots = g_axv_grid[rows - 1], gv = slots > 0 ? std::min(slots, ntiles) : grid;
-    if (vec != 0 && rows == 2)
-      k_kr_ax32v<MODE, 2><<<gv, dim3(AXV_TX, ETY), Axv<2>::smem(), s>>>(J, ts, n, ntiles, partial);
+    if (vec != 0 && rows == 2 && UNITS && L.stacked)
+      k_kr_ax32v<MODE, 2, UNITS><<<gv, dim3(AXV_TX, ETY), Axv<2>::smem(), s>>>(J, ts, n, ntiles, partial);
+    else if (vec != 0 && rows == 2)
+      k_kr_ax32v<MODE, 2, false><<<gv, dim3(AXV_TX, ETY), Axv<2>::smem(), s>>>(J, ts, n, ntiles, partial);
     else if (vec != 0)
-      k_kr_ax32v<MODE, 1><<<gv, dim3(AXV_TX, ETY), Axv<1>::smem(), s>>>(J, ts, n, ntiles, partial);
+      k_kr_ax32v<MODE, 1, false><<<gv, dim3(AXV_TX, ETY), Axv<1>::smem(), s>>>(J, ts, n, ntiles, partial);
     if (vec != 1) k_kr_ax32<MODE><<<grid, kAxBlock, axa_smem_bytes(), s>>>(J, ts, n, ntiles, partial);
     if (vec == 2) prof::count(1);  // two launches where the callers count one
   } else {
     constexpr int NR = MODE == 3 ? AXD_NR3 : 1;
     const int slots = MODE == 3 ? g_axd3_grid : g_axd_grid;
     const int gv = slots > 0 ? std::min(slots, ntiles) : grid;
-    if (vec != 0) k_kr_ax64v<MODE, NR><<<gv, dim3(AXD_TX, ETY), Axd<NR>::smem(), s>>>(J, ts, n, ntiles, partial);
+    if (vec != 0 && UNITS && L.stacked)
+      k_kr_ax64v<MODE, NR, UNITS><<<gv, dim3(AXD_TX, ETY), Axd<NR>::smem(), s>>>(J, ts, n, ntiles, partial);
+    else if (vec != 0)
+      k_kr_ax64v<MODE, NR, false><<<gv, dim3(AXD_TX, ETY), Axd<NR>::smem(), s>>>(J, ts, n, ntiles, partial);
     if (vec != 1) k_kr_ax<T, MODE><<<grid, kAxBlock, ax_smem_bytes<T>(), s>>>(J, ts, n, ntiles, partial);
     if (vec == 2) prof::count(1);
   }
@@ -3420,7 +3443,8 @@ int ListArena::add(const std::vector<J>& jobs, const std::vector<int>& tiles, co
   };
   for (int n : tiles) L.ntiles += n;
   ts_off.push_back(prefix(tiles));
-  us_off.push_back(units ? prefix(*units) : ts_off.back());
+  L.stacked = units && *units != tiles;
+  us_off.push_back(L.stacked ? prefix(*units) : ts_off.back());
   align(16);
   job_off.push_back(host.size());
   const unsigned char* jb = reinterpret_cast<const unsigned char*>(jobs.data());
@@ -3596,6 +3620,7 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     for (int c = 0; c < n; ++c) {
       kj[c].kc = tg[c].kc;
       kj[c].ks = tg[c].ks;
+      kj[c].nu = tg[c].kc / tg[c].ks;
       kt[c] = tiles_of(kj[c].g, kj[c].kc, 1, rows_of(kj[c]));
       ku[c] = tiles_of(kj[c].g, kj[c].ks, 1, rows_of(kj[c]));
       kj[c].us = (int)ta;
@@ -4061,7 +4086,6 @@ void Engine<T>::enqueue_iteration() {
   const DevList& K = arena_.lists[kr_list_];
   const DevList& W = arena_.lists[kv_list_];
   const DevList& U = arena_.lists[ku_list_];
-  const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
   const KrylovJob<T>* JW = static_cast<const KrylovJob<T>*>(W.jobs);
   const KrylovJob<T>* JU = static_cast<const KrylovJob<T>*>(U.jobs);
   const int n = K.njobs;
@@ -4070,11 +4094,11 @@ void Engine<T>::enqueue_iteration() {
   const double fb = sizeof(T) * cells_[kr_list_];
   IMPACT_PROF(prof::K_P_UPDATE, 4 * fb, s, (k_kr_p<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(0);
-  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_, kr_rows_)));
+  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 1>(grid, K, partial_, s, kr_vec_, kr_rows_)));
   k_efin<<<n, 256, 0, s>>>(K.us, partial_, 1, 0, EFIN_ALPHA, scal_, nullptr);
   IMPACT_PROF(prof::K_R_UPDATE, 3 * fb, s, (k_kr_r<T><<<gu, kBlock, 0, s>>>(JU, U.ts, n, U.ntiles)));
   enqueue_precond(1);
-  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s, kr_vec_, kr_rows_)));
+  IMPACT_PROF(prof::K_DIVGRAD, 3 * fb, s, (launch_ax<T, 2>(grid, K, partial_, s, kr_vec_, kr_rows_)));
   k_efin<<<n, 256, 0, s>>>(K.us, partial_, 2, 0, EFIN_OMEGA, scal_, nullptr);
   IMPACT_PROF(prof::K_X_UPDATE, 8 * fb, s, (k_kr_x<T><<<gw, kBlock, 0, s>>>(JW, W.ts, n, W.ntiles, partial_)));
   k_efin<<<n, 256, 0, s>>>(W.ts, partial_, 3, 1, EFIN_NORMS, scal_, nullptr);
@@ -4122,7 +4146,6 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
   cudaError_t e = cudaMemcpyAsync(scal_, scal_host_, n * sizeof(SolverScalars), cudaMemcpyHostToDevice, s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine scalars", __FILE__, __LINE__);
   const DevList& K = arena_.lists[kr_list_];
-  const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
   const int grid = grid_for(K.ntiles);
   const DevList& W = arena_.lists[kv_list_];
   const KrylovJob<T>* JW = static_cast<const KrylovJob<T>*>(W.jobs);
@@ -4132,7 +4155,7 @@ int Engine<T>::solve(const std::vector<SolverScalars>& init, int zero_phi, std::
     prof::count(1);
   } else {
     if (!zero_phi) {
-      launch_ax<T, 0>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_);
+      launch_ax<T, 0>(grid, K, partial_, s_, kr_vec_, kr_rows_);
       prof::count(1);
     }
     IMPACT_PROF(prof::K_KR_INIT, 4.0 * sizeof(T) * cells_[kr_list_], s_,
@@ -4235,8 +4258,7 @@ int Engine<T>::apply_operator() {
   cudaError_t e = cudaMemcpyAsync(scal_, scal_host_, n * sizeof(SolverScalars), cudaMemcpyHostToDevice, s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine scalars", __FILE__, __LINE__);
   const DevList& K = arena_.lists[kr_list_];
-  const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
-  launch_ax<T, 0>(grid_for(K.ntiles), J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_);
+  launch_ax<T, 0>(grid_for(K.ntiles), K, partial_, s_, kr_vec_, kr_rows_);
   prof::count(1);
   e = cudaStreamSynchronize(s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine operator", __FILE__, __LINE__);
@@ -4255,7 +4277,6 @@ int Engine<T>::bench(int kind, int iters, double* ms, double* bytes) {
   cudaError_t e = cudaMemcpyAsync(scal_, scal_host_, n * sizeof(SolverScalars), cudaMemcpyHostToDevice, s_);
   if (e != cudaSuccess) return impact_set_error(e, "engine scalars", __FILE__, __LINE__);
   const DevList& K = arena_.lists[kr_list_];
-  const KrylovJob<T>* J = static_cast<const KrylovJob<T>*>(K.jobs);
   const int grid = grid_for(K.ntiles);
   const DevList& W = arena_.lists[kv_list_];
   const KrylovJob<T>* JW = static_cast<const KrylovJob<T>*>(W.jobs);
@@ -4289,11 +4310,11 @@ int Engine<T>::bench(int kind, int iters, double* ms, double* bytes) {
     }
     case 5:
       by = 3 * sz * fc;
-      f = [&]() { launch_ax<T, 1>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_); };
+      f = [&]() { launch_ax<T, 1>(grid, K, partial_, s_, kr_vec_, kr_rows_); };
       break;
     case 6:
       by = 3 * sz * fc;
-      f = [&]() { launch_ax<T, 2>(grid, J, K.ts, n, K.ntiles, partial_, s_, kr_vec_, kr_rows_); };
+      f = [&]() { launch_ax<T, 2>(grid, K, partial_, s_, kr_vec_, kr_rows_); };
       break;
     case 7:
       by = 8 * sz * fc;
@@ -4439,6 +4460,7 @@ int MixedEngine::build(const std::vector<Case>& cs, const EngineParams& p, cudaS
   stack_units(tg, kc, g_axd3_grid, Axd<AXD_NR3>::B);
   for (int c = 0; c < n; ++c) {
     aj[c].kc = tg[c].kc;
+    aj[c].nu = tg[c].kc / tg[c].ks;
     t[c] = tiles_of(aj[c].g, aj[c].kc, 1, tg[c].rows);
   }
   e = cudaMalloc((void**)&partial_, (size_t)(units * 4 + 64) * sizeof(double));
@@ -4483,7 +4505,6 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
   const DevList& ML = arena_.lists[mix_list_];
   double cells = 0.0;  // algorithmic bytes of both kernels: 20 per cell (x, b or e, r32 or x)
   for (const auto& c : cs_) cells += (double)c.g.n1 * c.g.n2 * c.g.n3;
-  const KrylovJob<double>* AJ = static_cast<const KrylovJob<double>*>(AL.jobs);
   const MixJob* MJ = static_cast<const MixJob*>(ML.jobs);
   const int grid = grid_for(AL.ntiles), gm = grid_for(ML.ntiles);
   // the cases' done flags on the device, sent when they changed.  The copies read pinned memory and
@@ -4514,7 +4535,7 @@ int MixedEngine::solve(const std::vector<SolverScalars>& outer, double inner_tol
     if (rc) return rc;
     // r = b - A x in FP64 (the reference operator), stored as the FP32 right-hand side of the
     // inner solve, with its norms
-    IMPACT_PROF(prof::K_MX_RESID, 20.0 * cells, s_, (launch_ax<double, 3>(grid, AJ, AL.ts, n, AL.ntiles, partial_, s_, ax_vec_)));
+    IMPACT_PROF(prof::K_MX_RESID, 20.0 * cells, s_, (launch_ax<double, 3>(grid, AL, partial_, s_, ax_vec_)));
     k_efin<<<n, 256, 0, s_>>>(AL.us, partial_, 3, 1, EFIN_RAW, nullptr, q_);
     prof::count(1);
     cudaError_t e = cudaMemcpyAsync(q_host_, q_, (size_t)n * 4 * sizeof(double), cudaMemcpyDeviceToHost, s_);

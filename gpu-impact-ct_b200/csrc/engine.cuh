@@ -71,9 +71,9 @@ template <typename T>
 struct KrylovJob {
   Geom g;
   int kc;
-  // the operator's partial sums: one per column of tiles and `ks` planes (kc, or a divisor of it: the
-  // FP64 vector kernel's tiles may hold several), from row `us` of the list's partials on
-  int ks, us;
+  // the operator's partial sums: one per column of tiles and `ks` planes, from row `us` of the list's
+  // partials on; a tile of the vector kernels may hold several, kc / ks = nu
+  int ks, nu, us;
   const T* W[3];  // collapsed product_div_grad weights, row (i-1) holds offsets -5..5
   int zuni;       // 1: every z row of W[2] is the same (uniform z spacing)
   int xuni;       // 1: every x row of W[0] is the same (uniform x spacing)
@@ -106,6 +106,7 @@ struct DevList {
   int njobs = 0, ntiles = 0;
   const int* ts = nullptr;    // tile prefix sums (njobs + 1)
   const int* us = nullptr;    // prefix sums of the partials that its kernels write (ts: one per tile)
+  bool stacked = false;       // tiles of several partials
   const void* jobs = nullptr;
 };
 

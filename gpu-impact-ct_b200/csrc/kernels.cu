@@ -16,13 +16,14 @@
 namespace impact {
 
 int device_sms() {
-  static std::atomic<int> known[64];
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  n = known[dev].load(std::memory_order_relaxed);
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
   if (n > 0) return n;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  known[dev].store(n, std::memory_order_relaxed);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+    n = 148;
+  known.store(n, std::memory_order_relaxed);
   return n;
 }
 

@@ -4,7 +4,7 @@
 
 namespace impact {
 
-// SMs of the current device (asked for once per device)
+// SMs of the device, asked for once (a node's GPUs are alike; only launch shapes depend on it)
 int device_sms();
 
 // ---- one-axis stencils as streaming passes (march.cu): out (=, += for OP 1) the CNT-point

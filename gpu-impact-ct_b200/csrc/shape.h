@@ -107,30 +107,42 @@ inline int list_depth(const std::vector<TileGrid>& gs, int kc, int slots) {
 // Tile depths of an operator list of several grids whose units ks are chosen.  A grid whose tiles of ks planes
 // would fill the GPU alone shares it here, where each tile's prologue is paid for nothing: a tile holds
 // as many whole units as the list's common depth allows, and its kernel sums each unit by itself.  The
-// depth minimises the list's planes and prologues per resident block + the longest tile.  step: the
+// depth minimises the planes and prologues of the most loaded of `slots` blocks, which take the list's tiles
+// in turn, + those of the average one (a block that is done leaves its SM to another).  step: the
 // planes per step of the kernel, of which a unit must be a multiple.  48 cases of 32 to 152 cells a
-// side: FP64 operator 32.0 ms a step with tiles of one unit, 30.0 with several (29.2 with 64 planes in every tile
-// and unit), FP32 operator 14.4 and 13.5.
+// side: FP64 operator 32.0 ms a step with tiles of one unit, 29.4 with several (29.2 with 64 planes in every
+// tile and unit), FP32 operator 14.4 and 13.4.  Lists of fewer than 3 waves of one-unit tiles keep those: the
+// prologues hide behind the other blocks' planes, and fewer tiles leave SMs idle (FP64 cases of 72 and 64
+// cells a side, step 9.22 ms; with tiles of 32 planes 9.54).
 inline void stack_units(std::vector<TileGrid>& gs, int kc, int slots, int step) {
   auto depth = [&](const TileGrid& g, int d) { return g.stack && g.ks % step == 0 ? g.ks * std::max(1, d / g.ks) : g.ks; };
   int best = 1;
   double least = -1.0;
+  std::vector<long long> change(slots + 1);
   auto consider = [&](int d) {
-    double work = 0.0;
-    int longest = 0;
+    std::fill(change.begin(), change.end(), 0);  // of the load from one block to the next
+    long long first = 0, work = 0;
     for (const TileGrid& g : gs) {
-      const int e = depth(g, d);
-      const double columns = (double)tiles_at(g, g.n3);
-      work += columns * (g.n3 + 8.0 * ((g.n3 + e - 1) / e));
-      longest = std::max(longest, std::min(e, g.n3) + 8);
+      const int e = depth(g, d), len = std::min(e, g.n3) + 8;
+      const long long tiles = tiles_at(g, e), part = tiles % slots, at = first % slots;
+      change[0] += tiles / slots * len;
+      change[at] += len;
+      change[(at + part) % slots] -= len;  // (at slots: past the last block, undone by the next line)
+      if (at + part >= slots) change[0] += len;
+      first += tiles;
+      work += tiles * len;
     }
-    const double cost = work / slots + longest;
+    long long load = 0, longest = 0;
+    for (int b = 0; b < slots; ++b) longest = std::max(longest, load += change[b]);
+    const double cost = (double)longest + (double)work / slots;
     if (least < 0.0 || cost < least) {
       least = cost;
       best = d;
     }
   };
-  if (gs.size() > 1) {
+  long long alone = 0;
+  for (const TileGrid& g : gs) alone += tiles_at(g, g.ks);
+  if (gs.size() > 1 && alone >= 3LL * slots) {
     consider(kc);
     for (int d = (kc - 1) / 8 * 8; d >= 8; d -= 8) consider(d);
     for (int d : {4, 1})

@@ -79,7 +79,9 @@ KERNELS = [(8, 296, 4), (16, 296, 2), (16, 592, 2)]  # FP64 operator, FP64 outer
 def test_a_batch_does_not_pay_for_the_shallow_tiles_of_its_cases_alone(shape, rows, slots, step):
     sizes = 3 * UNEVEN
     ks, depth = _stacked(shape, sizes, rows, 64, slots, step)
-    assert _planes(sizes, depth, rows) <= 1.03 * _planes(sizes, [64] * len(sizes), rows) < _planes(sizes, ks, rows)
+    deep, alone = _planes(sizes, [64] * len(sizes), rows), _planes(sizes, ks, rows)
+    assert alone > 1.1 * deep
+    assert _planes(sizes, depth, rows) - deep <= 0.25 * (alone - deep)  # (the rest: units that do not divide 64, the last round)
     for n, u, d in zip(sizes, ks, depth):
         assert d % u == 0 and d <= 64
         assert u == _stacked(shape, [n], rows, 64, slots, step)[0][0]  # the unit is the grid's own

@@ -2834,14 +2834,19 @@ __global__ void __launch_bounds__(MNT, 1) k_lv_multi(const LevelJob<T>* __restri
 // with a ghost plane at either end that the neighbours write into each other's shared memory in
 // every pass, and a pass ends with the cluster's barrier.  That barrier takes longer than the
 // warps' own, so the cut pays where many passes run on a level large enough for one SM's
-// instructions to bound it: the Chebyshev steps of a coarsest level of at least TAIL_SPLIT cells.  104x104x208, 32 steps on 13x13x26: V-cycle FP32 189 -> 160 us, FP64 255 -> 207.  With
-// Jacobi bottoms (levels halved down to a few cells) the cut is slower at every size measured:
-// 128x128x256 FP32 192 -> 199 us, FP64 290 -> 297.
+// instructions to bound it: the Chebyshev steps of a coarsest level of at least TAIL_SPLIT cells
+// (TAIL_SPLIT_ANY where one is to pay for a list's small levels too: 1458 and 16 cells together, FP64
+// cases of 72x72x144 and 64x64x128, a step 9.25 -> 9.45 ms).
+// V-cycle in us with 32 steps, one block -> cluster, by the coarsest level's cells: 343 FP32 89 -> 93,
+// FP64 99 -> 101; 686 105.5 -> 105.5 (16 steps: 97 -> 94), 125.5 -> 121; 729 116 -> 101, 136 -> 114; 1458
+// 142 -> 118, 162 -> 148; 4394 189 -> 158, 253 -> 202.  With Jacobi bottoms (levels halved down to a few
+// cells) the cut is slower at every size measured: 128x128x256 FP32 192 -> 199 us, FP64 290 -> 297.
 constexpr int TNT = 512;
 constexpr size_t TAIL_BYTES = 200 * 1024;     // the levels' fields
 constexpr size_t TAIL_TAB_BYTES = 22 * 1024;  // their tables (longer ones are read from global memory)
 constexpr int TAIL_CLUSTER = 8;               // most blocks per case with Chebyshev steps
-constexpr int TAIL_SPLIT = 1536;              // cells of a coarsest level from which they are used
+constexpr int TAIL_SPLIT = 512;               // cells of every tail's coarsest level from which they are used
+constexpr int TAIL_SPLIT_ANY = 1536;          // ... or of one of the tails
 
 // one level inside the tail: extents, thread mapping, shared-memory offsets (elements)
 struct TailLevel {
@@ -3845,12 +3850,14 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
   tail_blocks_ = 1;
   if (p_.bottom_cheb > 0) {
     int ntails = 0;
-    bool want = false;
+    bool large = false, all = true;
     for (int c = 0; c < n; ++c) {
       if (lt[c] < 0) continue;
       const Geom& gl = cs[c].mg->lv[nlev[c] - 1].g;
+      const int cells = gl.n1 * gl.n2 * gl.n3;
       ++ntails;
-      want |= gl.n1 * gl.n2 * gl.n3 >= TAIL_SPLIT;
+      large |= cells >= TAIL_SPLIT_ANY;
+      all = all && cells >= TAIL_SPLIT;
     }
     auto fits = [&](int cb) {
       for (int c = 0; c < n; ++c)
@@ -3866,7 +3873,7 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
       }
       return clusters;
     };
-    if (want) tail_blocks_ = tail_cluster(ntails, TAIL_CLUSTER, fits, held);
+    if (large || all) tail_blocks_ = tail_cluster(ntails, TAIL_CLUSTER, fits, held);
   }
   auto in_lists = [&](int c, int g) { return lt[c] < 0 || g < lt[c]; };
   if (use_mg) {

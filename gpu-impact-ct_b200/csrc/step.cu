@@ -1043,6 +1043,8 @@ extern "C" int impact_b200_case_apply(impact_b200_case* c, int op, int field_in,
   EngineParams ep = engine_params(s, &p);
   ep.use_graph = 0;
   if (op == 2) {  // field_out = A field_in in FP32 (the operator of the mixed solve's inner solve)
+    // the kernel and the tile depth of the case's multigrid solves; without a hierarchy, of its JOR solves
+    ep.precond = s.mg_levels ? 1 : 0;
     const long long nf = s.g.nfield;
     float* buf = nullptr;  // input, output, unused Krylov slots
     IMPACT_CUDA_CHECK(cudaMalloc((void**)&buf, 3 * nf * sizeof(float)));
@@ -1057,7 +1059,7 @@ extern "C" int impact_b200_case_apply(impact_b200_case* c, int op, int field_in,
     ef.zuni = s.zuni;
     ef.xuni = s.xuni;
     ef.cdg_zuni = s.cdg_zuni;
-    ef.mg = nullptr;
+    ef.mg = s.mg_levels ? &s.mg32 : nullptr;
     ef.bb = ef.phi = buf;
     ef.rr = buf + nf;
     ef.rh = ef.pp = ef.Ap = ef.Ar = ef.z1 = ef.z2 = ef.comp = buf + 2 * nf;

@@ -1219,7 +1219,7 @@ __global__ void __launch_bounds__(AXNT, 3) k_kr_ax32(const KrylovJob<float>* __r
 // neighbours from 10 other rows (one vector each, shared by the two rows).  The arithmetic runs on
 // packed FP32 pairs (fma.rn.f32x2: two IEEE fmas per instruction), the per-plane inner-product
 // terms are summed in FP32 and added in FP64.  The ring holds two groups of AXV_B planes: a step
-// computes on one while the next is in flight (42 KB of shared memory and 242 registers: 4 blocks
+// computes on one while the next is in flight (28 KB of shared memory and 242 registers: 4 blocks
 // per SM).
 //
 // What bounds it: reads from L2 (1.4 of halo, 1 of window and 1 of partners per point, 1 written)
@@ -1305,7 +1305,7 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
     }
     // this thread's chunks of a staged plane: chunk cq = tid + e*AXV_NT holds columns
     // i0-8+4(cq%12) .. +3 of row j0-5+cq/12.  The points of the tile read columns
-    // i0-5 .. min(i0+31, n1)+5 and rows j0-5 .. min(j0+7, n2)+5; cb[e] is the chunk's in-plane
+    // i0-5 .. min(i0+31, n1)+5 and rows j0-5 .. min(j0+AXV_Y-1, n2)+5; cb[e] is the chunk's in-plane
     // offset, -1 for a chunk nothing needs.  A chunk starts at a column = 1 (mod 4) and n1 % 4 == 0,
     // so a chunk outside 1..n1 lies whole in one periodic image (n1 >= 8): every chunk, at the box
     // ends too, is one 16-byte copy from its image.
@@ -1518,8 +1518,8 @@ __global__ void __launch_bounds__(AXV_NT, AXV_NR == 1 ? 5 : 4) k_kr_ax32v(const 
 // in shared memory; NR = 1 stages the whole plane (48 x 18 doubles) in groups of 4, with the y weights
 // in registers.  Outer residual on 256 x 256 x 512 318 -> 309 us, 128 x 128 x 256 55 -> 52, a mixed
 // step at 384 x 384 x 768 154.1 -> 153.1 ms.  The Krylov lists keep one row: two take 267 instead of
-// 283 us on 256 x 256 x 512 and 8.3 instead of 6.8 on 32 x 32 x 64, and they sum the inner products
-// in another order, which the JOR solves' 100 iterations carry up to the solve's tolerance.  At one
+// 283 us on 256 x 256 x 512 but 8.3 instead of 6.8 on 32 x 32 x 64, and in JOR solves another order of the
+// inner products' terms travels, over 100 iterations, up to the solve's tolerance.  At one
 // row the own points from the window change nothing.  All bound by the shared-memory loads and the
 // latency of 8 warps per SM (255 registers); the weights are the per-row
 // weights of every axis (the FP64 operator defines the residual): x rows of the thread's two
@@ -3398,7 +3398,12 @@ void launch_ax(int grid, const DevList& L, double* partial, cudaStream_t s, int 
 // the fused smoothing kernel runs one block per tile (one block per SM at a time)
 inline int grid_multi(int ntiles) { return ntiles; }
 
-constexpr int kVecBlocksPerSm = 4;  // resident blocks of the vector updates
+// Slots per SM in the depth rule of the vector updates (k_kr_x holds 2 blocks per SM in FP64 and 3 in FP32, the p
+// and r updates 3).  2, 3, 4, 6, 8, x update in us: FP32 96x96x192 10.3, 10.3, 10.3, 12.3, 12.3 and 128x128x256 22.6,
+// 22.1, 25.9, 23.2, 26.3; FP64 96x96x192 16.4, 20.6, 20.7, 20.5, 20.5 and 128x128x256 52.9, 65.1, 53.4, 57.3, 55.3; below
+// 80 cells a side and from 192 on the same, the p and r updates within 10 %.  The depth is the x update's unit
+// of summation, so another value is another order of its sums.
+constexpr int kVecBlocksPerSm = 4;
 // a grid's tiles of 32 x `rows` columns, for the depth rules of shape.h
 inline TileGrid tile_grid(const Geom& g, int rows = ETY, bool stack = false) {
   return TileGrid{ETX, rows, g.n1, g.n2, g.n3, stack, 0, 0};
@@ -3603,7 +3608,9 @@ int Engine<T>::build(const std::vector<EngineCase<T>>& cs, const EngineParams& p
     // Solves with JOR sweeps (some 100 iterations) keep kc, one row per thread in the operator and the
     // x update's point order: their inner products cancel by many digits, and so many iterations
     // carry the last bits of the sums up to the solve's tolerance (FP32 on 59 x 47 x 83: with shallow
-    // tiles one step in some 30 ended 4e-7 of max|p| from the deep tiles' result).
+    // tiles one step in some 30 ended 4e-7 of max|p| from the deep tiles' result).  Excepted is a mixed
+    // solve's first r.r, which comes from the outer residual's own tiles: 80 of 80 steps on 59 x 47 x 83
+    // and 40 x 34 x 56 gave the bits of the deep tiles' sum.
     constexpr bool f32 = std::is_same<T, float>::value;
     const bool adapt = use_mg;
     kr_rows_ = f32 && use_mg ? 2 : 1;

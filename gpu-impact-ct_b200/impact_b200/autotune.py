@@ -1,9 +1,11 @@
 """Autotuner of the pressure solve: tile depth of the solver kernels, multigrid sweep schedule and,
 for mixed precision, the tolerance of each FP32 inner solve.
 
-The kernels of the Poisson engine cut every grid into tiles of 32 x 8 columns and `tile_kc`
-z-planes; deeper tiles stream longer columns (fewer tile start-ups), shallower ones give more
-tiles to fill the 148 SMs on small grids and coarse levels.  The V-cycle's sweep counts trade
+The kernels of the Poisson engine cut every grid into tiles of 32 x 8 or 32 x 16 columns and at most
+`tile_kc` z-planes; deeper tiles stream longer columns (fewer tile start-ups), shallower ones give more
+tiles to fill the SMs on small grids and coarse levels.  With the V-cycle the Krylov kernels take
+fewer planes by themselves where a grid is small, so there several candidates can be the same
+engine; the reported time (rounded to 1 us) then keeps the first.  The V-cycle's sweep counts trade
 the cost of one preconditioner application against the number of BiCGstab iterations.  Both are
 chosen here by timing complete Poisson solves of the case's own current right-hand side to the
 requested tolerance, one per candidate, on the device, and keeping the fastest candidate that

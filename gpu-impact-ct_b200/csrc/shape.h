@@ -6,6 +6,8 @@
 
 namespace impact {
 
+constexpr int MAX_GRID_YZ = 65535;  // blocks of a launch along y or z
+
 // Steps of a thread that marches along an axis of na steps, `threads` threads side by side: the
 // largest power of two up to `most` that leaves `per_sm` threads per SM.  A longer segment re-reads
 // fewer of the CNT - 1 values before it and pays its set-up once; a thread too few costs a small grid
@@ -16,6 +18,7 @@ namespace impact {
 inline int march_seg(long long threads, int na, int sms, int per_sm, int most) {
   int seg = 1;
   while (2 * seg <= most && 2 * seg <= na && threads * na >= (long long)sms * per_sm * 2 * seg) seg *= 2;
+  while ((na - 1) / seg + 1 > MAX_GRID_YZ) seg *= 2;
   return seg;
 }
 
@@ -46,6 +49,7 @@ inline int tri_depth(double gxy, int n3, double sms, bool vec) {
       depth = kz;
     }
   }
+  while ((n3 - 1) / depth + 1 > MAX_GRID_YZ) depth *= 2;
   return depth;
 }
 

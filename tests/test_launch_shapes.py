@@ -54,6 +54,14 @@ def test_a_three_axis_pass_on_a_small_grid_takes_shallow_blocks(shape, n, vec):
     assert gxy * -(-n // kz) >= min(SMS / 2, gxy * n)
 
 
+def test_long_axes_stay_within_the_launch_limit(shape):
+    for n in (65535, 65536, 600_000, 3_000_000, 20_000_000):
+        for threads in (16, 32, 64):
+            assert -(-n // shape.host_march_seg(threads, n, SMS, 320, 8)) <= 65535
+        for vec in (0, 1):
+            assert -(-n // shape.host_tri_depth(1, n, SMS, vec)) <= 65535
+
+
 @pytest.mark.parametrize("share", [1.0, 0.25, 0.001])
 def test_depths_of_a_batch_grow_as_its_share_shrinks(shape, share):
     assert shape.host_tri_depth(8, 64, SMS * share, 1) >= shape.host_tri_depth(8, 64, SMS, 1)

@@ -1,6 +1,6 @@
 """Launch shapes of the streaming passes (csrc/shape.h, compiled here for the host) and the registers
 of their kernels: a small grid may not be left to a few long threads or blocks, a large one not to a
-nearly empty last round, and no kernel of the one-axis passes may spill."""
+nearly empty last wave, and no kernel of the one-axis passes may spill."""
 import ctypes as C
 import os
 import re
@@ -38,8 +38,8 @@ def test_a_marching_pass_fills_the_device_before_it_lengthens_its_segments(shape
     assert seg == most or 2 * seg > na or threads * na < SMS * per_sm * 2 * seg
 
 
-def test_a_three_axis_pass_prefers_one_full_round(shape):
-    # tiles of 32 x 16 points of two doubles: one round of two blocks per SM
+def test_a_three_axis_pass_prefers_one_full_wave(shape):
+    # tiles of 32 x 16 points of two doubles: one wave of two blocks per SM
     for n, kz in ((112, 12), (128, 16), (160, 32), (192, 48)):
         gxy = -(-n // 32) * -(-n // 16)
         assert shape.host_tri_depth(gxy, n, SMS, 1) == kz
@@ -89,7 +89,7 @@ def test_a_batch_does_not_pay_for_the_shallow_tiles_of_its_cases_alone(shape, ro
     ks, depth = _stacked(shape, sizes, rows, 64, slots, step)
     deep, alone = _planes(sizes, [64] * len(sizes), rows), _planes(sizes, ks, rows)
     assert alone > 1.1 * deep
-    assert _planes(sizes, depth, rows) - deep <= 0.25 * (alone - deep)  # (the rest: units that do not divide 64, the last round)
+    assert _planes(sizes, depth, rows) - deep <= 0.25 * (alone - deep)  # (the rest: units that do not divide 64, the last wave)
     for n, u, d in zip(sizes, ks, depth):
         assert d % u == 0 and d <= 64
         assert u == _stacked(shape, [n], rows, 64, slots, step)[0][0]  # the unit is the grid's own
